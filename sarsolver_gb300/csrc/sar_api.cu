@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/sargpu.h"
+#include "sar_fir.cuh"
 #include "sar_host_prep.h"
 #include "sar_kernels.cuh"
 #include "sar_fft_cb.h"
@@ -125,12 +126,21 @@ struct sar_plan {
     float2* d_wadj = nullptr;
     float2* d_wfwd = nullptr;
     void* d_spec = nullptr;        // FFT rows: float2, or double2 when fft_double
-    // fused up/downsampling (N = 1024, 2048, 4096; M a multiple of N): twiddle tables e^{2 pi i q / N}, e^{2 pi i q / M}
+    // fused up/downsampling (N = 512 ... 8192; M a multiple of N): twiddle tables e^{2 pi i q / N} and, without
+    // the base grid, e^{2 pi i q / M}
     bool fused_up = false;
     bool fused_down = false;   // fused forward downsampling (those N, M a multiple of N, Lg <= M)
     float2* d_tw_n = nullptr;
     float2* d_tw_m = nullptr;
+    // base-grid transforms (sar_fir.cu): even upsampling factors from 4, any N
+    bool fir = false;
+    FirLayout fir_layout;
+    float2* d_fir_wave = nullptr;   // waveform / c(k)
+    float2* d_half = nullptr;       // e^{2 pi i k / (2 N)} (fused kernels)
+    float* d_taps = nullptr;
+    float* d_pair_taps = nullptr;
     bool fft_double = false;
+    long fft_len = 0;               // length of the cuFFT rows: M, or 2 N with fir
     float4* d_prof = nullptr;   // [S][Lg] pairs (adjoint) / float2 accumulator (forward)
     int* d_strip = nullptr;
     unsigned* d_flags = nullptr;
@@ -190,6 +200,10 @@ struct sar_plan {
         cudaFree(d_spec);
         cudaFree(d_tw_n);
         cudaFree(d_tw_m);
+        cudaFree(d_fir_wave);
+        cudaFree(d_half);
+        cudaFree(d_taps);
+        cudaFree(d_pair_taps);
         cudaFree(d_prof);
         cudaFree(d_strip);
         cudaFree(d_flags);
@@ -253,7 +267,7 @@ int run_fft(sar_plan* p, void* data, int rows, int direction, cudaStream_t st) {
         for (auto& e : p->fft_other)
             if (e.first == rows) h = e.second;
         if (!h) {
-            int rc = make_fft(&h, (long)p->M, rows, p->fft_double);
+            int rc = make_fft(&h, p->fft_len, rows, p->fft_double);
             if (rc) return rc;
             p->fft_other.emplace_back(rows, h);
         }
@@ -777,29 +791,65 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
     // of one block, [block][Lg] float2, fits in half of one slot)
     if ((rc = p->alloc(&p->d_prof, (size_t)(p->block ? 2 * p->block : S) * p->Lg, "range profiles"))) return rc;
 
-    // ---- FFT work rows
-    p->fft_double = !smooth_length(M);
+    // ---- range-profile transforms.  Even upsampling factors from 4 go through the base grid (2 N points
+    // and a short filter, sar_fir.cu); the rest through U transforms of N points in one kernel where N
+    // allows it, or cuFFT of length M.  The callback transforms (opt-in, below) are of length M.
+    const char* cb_env = getenv("SAR_FFT_CALLBACKS");
+    const bool want_cb = !p->block && cb_env && cb_env[0] == '1' && smooth_length(M);
+    p->fir = !want_cb && fir_plan((long)N, (long)M, p->Lg, p->bg0, &p->fir_layout);
+    p->fft_len = p->fir ? 2 * (long)N : (long)M;
+    p->fft_double = !smooth_length((size_t)p->fft_len);
     const size_t elem = p->fft_double ? sizeof(double2) : sizeof(float2);
-    p->chunk = (int)std::min<size_t>(p->block ? p->block : S, std::max<size_t>(1, kSpecBudget / (M * elem)));
-    {
+    p->chunk = (int)std::min<size_t>(p->block ? p->block : S, std::max<size_t>(1, kSpecBudget / (p->fft_len * elem)));
+    if (p->fir) {
+        std::vector<float> taps, pair_taps;
+        std::vector<double> inv_c;
+        fir_tables(p->fir_layout, &taps, &pair_taps, &inv_c);
+        std::vector<float2> fw(N), half(N);
+        for (size_t f = 0; f < N; ++f) {
+            const double wr = g->waveform_fft ? g->waveform_fft[2 * f] : 1.0, wi = g->waveform_fft ? g->waveform_fft[2 * f + 1] : 0.0;
+            fw[f] = make_float2((float)(wr * inv_c[f]), (float)(wi * inv_c[f]));
+            const double k = f < N - N / 2 ? (double)f : (double)f - (double)N, angle = 3.14159265358979323846 * k / (double)N;
+            half[f] = make_float2((float)std::cos(angle), (float)std::sin(angle));
+        }
+        if ((rc = p->alloc(&p->d_fir_wave, N, "waveform"))) return rc;
+        if ((rc = p->alloc(&p->d_half, N, "twiddles"))) return rc;
+        if ((rc = p->alloc(&p->d_taps, taps.size(), "filter taps"))) return rc;
+        if ((rc = p->alloc(&p->d_pair_taps, pair_taps.size(), "filter taps"))) return rc;
+        SAR_CUDA(cudaMemcpy(p->d_fir_wave, fw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice), "waveform");
+        SAR_CUDA(cudaMemcpy(p->d_half, half.data(), sizeof(float2) * N, cudaMemcpyHostToDevice), "twiddles");
+        SAR_CUDA(cudaMemcpy(p->d_taps, taps.data(), sizeof(float) * taps.size(), cudaMemcpyHostToDevice), "filter taps");
+        SAR_CUDA(cudaMemcpy(p->d_pair_taps, pair_taps.data(), sizeof(float) * pair_taps.size(), cudaMemcpyHostToDevice),
+                 "filter taps");
+    }
+    if (!p->fir || !p->fir_layout.fused) {
         double2* spec = nullptr;
-        if ((rc = p->alloc(&spec, ((size_t)p->chunk * M * elem + sizeof(double2) - 1) / sizeof(double2), "FFT rows")))
+        if ((rc = p->alloc(&spec, ((size_t)p->chunk * p->fft_len * elem + sizeof(double2) - 1) / sizeof(double2), "FFT rows")))
             return rc;
         p->d_spec = spec;
+        if ((rc = make_fft(&p->fft_full, p->fft_len, p->chunk, p->fft_double))) return rc;
+        p->have_full = true;
+        const int tail = (int)(S % (size_t)p->chunk);
+        if (tail) {
+            if ((rc = make_fft(&p->fft_tail, p->fft_len, tail, p->fft_double))) return rc;
+            p->have_tail = true;
+            p->tail_rows = tail;
+        }
     }
-    if ((rc = make_fft(&p->fft_full, (long)M, p->chunk, p->fft_double))) return rc;
-    p->have_full = true;
-    const int tail = (int)(S % (size_t)p->chunk);
-    if (tail) {
-        if ((rc = make_fft(&p->fft_tail, (long)M, tail, p->fft_double))) return rc;
-        p->have_tail = true;
-        p->tail_rows = tail;
-    }
-    // Fused adjoint upsampling: for N = 512, 1024, 2048, 4096 or 8192 and M a multiple of N the backprojection's range
-    // profiles come from one kernel (U-way split of the length-M transform into N-point ones,
+    // Without the base grid: for N = 512, 1024, 2048, 4096 or 8192 and M a multiple of N the backprojection's
+    // range profiles come from one kernel (U-way split of the length-M transform into N-point ones,
     // stored span only) instead of pack + inverse FFT + unpack; twiddles computed in FP64.
-    const bool up_ok = upsample_fused_supported((int)N, (long)M, p->Lg);
-    const bool down_ok = downsample_fused_supported((int)N, (long)M, p->Lg);
+    const bool up_ok = !p->fir && upsample_fused_supported((int)N, (long)M, p->Lg);
+    const bool down_ok = !p->fir && downsample_fused_supported((int)N, (long)M, p->Lg);
+    p->fused_up = p->fused_down = p->fir && p->fir_layout.fused;
+    if (p->fused_up) {
+        std::vector<float2> tn(N);
+        const double two_pi = 6.283185307179586476925286766559;
+        for (size_t q = 0; q < N; ++q)
+            tn[q] = make_float2((float)std::cos(two_pi * (double)q / (double)N), (float)std::sin(two_pi * (double)q / (double)N));
+        if ((rc = p->alloc(&p->d_tw_n, N, "twiddles"))) return rc;
+        SAR_CUDA(cudaMemcpy(p->d_tw_n, tn.data(), sizeof(float2) * N, cudaMemcpyHostToDevice), "twiddles");
+    }
     if (up_ok || down_ok) {
         // tw_m: e^{2 pi i q / M} for q < M, then for each residue r < 2U the 16 thread-independent
         // factors e^{2 pi i (T e - N [e >= 8]) r / M} (T = N / 16) of the fused kernels' twiddles
@@ -830,9 +880,8 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
     // cufftMakePlanMany for LTO-IR of compute_90 .. compute_103a alike), so the packing kernels are
     // the default; when forced on, a plan that cannot link the callbacks reports why.
     {
-        const char* env = getenv("SAR_FFT_CALLBACKS");
-        const bool want = !p->fft_double && !p->block && env && env[0] == '1';
-        if (want) {
+        const char* env = cb_env;
+        if (want_cb) {
             p->Lc = (int)std::min<size_t>((size_t)p->Lg + 1, M);
             cufftHandle h = 0;
             int crc = p->alloc(&p->d_cb, 1, "callback parameters");
@@ -960,6 +1009,19 @@ static int prof_format(const sar_plan* p) {
     return p->values ? kProfValues : p->interp == SAR_INTERP_LINEAR ? kProfLinearPairs : kProfNearestPairs;
 }
 
+// Base-grid arguments of rows from pulse `first` on (sar_fir.cu).
+static FirArgs fir_args(const sar_plan* p, int first) {
+    FirArgs a;
+    a.wave = p->d_fir_wave;
+    a.half = p->d_half;
+    a.tw_n = p->d_tw_n;
+    a.taps = p->d_taps;
+    a.pair_taps = p->d_pair_taps;
+    a.Lg = p->Lg;
+    a.first = first;
+    return a;
+}
+
 // Upsampled profiles of pulses [begin, end): y row s is read at y + s * N; with pairs_out the
 // (value, difference) pairs of pulse s go to pairs_rows + s * Lg (the plan's buffer for a resident
 // plan; a ring slot, addressed from the block's first pulse, for a streamed one).
@@ -969,6 +1031,22 @@ static int upsample_rows(sar_plan* p, const float2* y, size_t begin, size_t end,
     for (size_t first = begin; first < end; first += (size_t)p->chunk) {
         const int rows = (int)std::min<size_t>(p->chunk, end - first);
         const int dbl = p->fft_double;
+        if (p->fir) {
+            FirArgs a = fir_args(p, (int)first);
+            a.y = y;
+            a.wfac = pairs_out ? p->d_wadj : nullptr;
+            a.prof = pairs_out ? (void*)pairs_rows : (void*)prof;
+            a.format = pairs_out ? prof_format(p) : kProfValues;
+            if (p->fir_layout.fused) {
+                SAR_CUDA(launch_fir_fused(a, p->fir_layout, rows, true, st), "fused upsampling");
+                continue;
+            }
+            SAR_CUDA(launch_pack_adjoint(y, p->d_fir_wave, p->d_spec, dbl, (int)p->N, p->fft_len, rows, (int)first, st), "pack");
+            int rc = run_fft(p, p->d_spec, rows, CUFFT_INVERSE, st);
+            if (rc) return rc;
+            SAR_CUDA(launch_fir_rows(p->d_spec, dbl, a, p->fir_layout, rows, st), "upsampling filter");
+            continue;
+        }
         if (pairs_out && p->fused_up) {
             SAR_CUDA(launch_upsample_pairs_fused(y, p->d_wave, p->d_wadj, p->d_tw_n, p->d_tw_m, pairs_rows, (int)p->N,
                                                  (long)p->M, p->Lg, p->bg0, rows, (int)first, prof_format(p), st),
@@ -1141,6 +1219,23 @@ static int downsample_rows(sar_plan* p, const float2* acc_rows, float2* y, size_
                            cudaStream_t st) {
     for (size_t first = begin; first < end; first += (size_t)p->chunk) {
         const int rows = (int)std::min<size_t>(p->chunk, end - first);
+        if (p->fir) {
+            FirArgs a = fir_args(p, (int)first);
+            a.acc = acc_rows;
+            a.y_out = y;
+            a.wfac = p->d_wfwd;
+            if (p->fir_layout.fused) {
+                SAR_CUDA(launch_fir_fused(a, p->fir_layout, rows, false, st), "fused downsampling");
+                continue;
+            }
+            SAR_CUDA(launch_fir_fold(p->d_spec, p->fft_double, a, p->fir_layout, rows, st), "downsampling filter");
+            int rc = run_fft(p, p->d_spec, rows, CUFFT_FORWARD, st);
+            if (rc) return rc;
+            SAR_CUDA(launch_extract_forward(p->d_spec, p->fft_double, p->d_fir_wave, p->d_wfwd, y, (int)p->N, p->fft_len, rows,
+                                            (int)first, st),
+                     "extract");
+            continue;
+        }
         if (p->fused_down) {
             SAR_CUDA(launch_downsample_forward_fused(acc_rows, p->d_wave, p->d_wfwd, p->d_tw_n, p->d_tw_m, y,
                                                      (int)p->N, (long)p->M, p->Lg, p->bg0, rows, (int)first, st),

@@ -24,6 +24,7 @@
 #include "sar_fir.cuh"
 #include "sar_host_prep.h"
 #include "sar_kernels.cuh"
+#include "sar_scatter.cuh"
 #include "sar_fft_cb.h"
 
 #include <cufftXt.h>
@@ -114,6 +115,9 @@ struct sar_plan {
     bool values = false;   // stored profiles are plain values (kProfValues), not pairs
     int seg_tiles = 0, segs_per_column = 0, ws = 0, pbf = 16;
     size_t n_strips = 0;
+    ScatterLayout scatter;         // forward scatter with a pulse per lane (linear sampling, plain bins)
+    GridConst gc_scatter{}, gc_fwd_image{};   // its lattice, and the image grid
+    int4* d_items = nullptr;
     int chunk = 0;
     std::vector<std::complex<double>> weights;
 
@@ -206,6 +210,7 @@ struct sar_plan {
         cudaFree(d_pair_taps);
         cudaFree(d_prof);
         cudaFree(d_strip);
+        cudaFree(d_items);
         cudaFree(d_flags);
         if (have_full) cufftDestroy(fft_full);
         if (have_tail) cufftDestroy(fft_tail);
@@ -572,6 +577,24 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             p->gc_fwd.precise_bins = precise;
             p->fwd_transposed = false;
         }
+        // Linear sampling with plain bins: the scatter with a pulse per lane, on the lattice along which bins
+        // change least (sar_scatter.cu); the strips below serve the other plans.  Images at most two strips
+        // across stay with them too: two partial sums per bin give the same bits in either order, so their
+        // forward projections are reproducible, which the many small runs of the other scatter are not.
+        if (p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins &&
+            (p->fwd_transposed ? p->gc_fwd.tiles_y : p->gc_fwd.tiles_x) > 2)
+            p->scatter = scatter_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+        if (p->scatter.ok) {
+            const ScatterLayout& L = p->scatter;
+            double ea[3], eb[3];
+            for (int c = 0; c < 3; ++c) {
+                ea[c] = L.vx * ex[c] + L.vy * ey[c];
+                eb[c] = L.wx * ex[c] + L.wy * ey[c];
+            }
+            p->gc_fwd_image = make_grid_const(ex, ey, ez, kappa, s_r, forward_bin_offset(p->interp), nx, ny, nz);
+            p->gc_scatter = make_grid_const(ea, eb, ez, kappa, s_r, forward_bin_offset(p->interp), nx, ny, nz);
+            p->ws = L.slots;
+        }
         // Forward strips: lines of tiles along the axis the scatter walks (columns along y; rows
         // along x for the transposed scatter; lattice columns for a sheared lattice, only their
         // tiles that hold image pixels), split into segments whose window fits shared memory.
@@ -584,8 +607,9 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             if (!strips_x) lattice_tile_range(p->gc_fwd, ln, &line_lo[ln], &line_hi[ln]);
             along = std::max(along, line_hi[ln] - line_lo[ln] + 1);
         }
-        p->forward_points = true;
+        p->forward_points = !p->scatter.ok;
         for (int pbf : {16, 8}) {
+            if (p->scatter.ok) break;
             int seg = along;
             while (true) {
                 const int segs = (along + seg - 1) / seg;
@@ -767,6 +791,11 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         }
         if ((rc = p->alloc(&p->d_steps, 9, "grid steps"))) return rc;
         SAR_CUDA(cudaMemcpy(p->d_steps, steps, sizeof steps, cudaMemcpyHostToDevice), "grid steps");
+    }
+    if (p->scatter.ok) {
+        const std::vector<int4>& items = p->scatter.items;
+        if ((rc = p->alloc(&p->d_items, items.size(), "scatter blocks"))) return rc;
+        SAR_CUDA(cudaMemcpy(p->d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice), "scatter blocks");
     }
     if (!strip_start.empty()) {
         if ((rc = p->alloc(&p->d_strip, strip_start.size(), "strip table"))) return rc;
@@ -1187,6 +1216,30 @@ int sar_adjoint(sar_plan* p, const void* y_dev, void* x_dev, void* stream) {
 
 // Grid scatter of pulses [first, first + count) into accumulator rows `acc` (row 0 = pulse `first`).
 static int scatter_pulses(sar_plan* p, const float2* x, float2* acc, size_t first, size_t count, cudaStream_t st) {
+    if (p->scatter.ok) {
+        const ScatterLayout& L = p->scatter;
+        ScatterArgs a;
+        a.img = p->gc_fwd_image;
+        a.lat = p->gc_scatter;
+        a.pulses = p->d_pulses + first;
+        a.x = x;
+        a.acc = acc;
+        a.items = p->d_items;
+        a.flags = p->d_flags;
+        a.num_items = (int)L.items.size();
+        a.S = (int)count;
+        a.Lg = p->Lg;
+        a.bg0 = (int)p->bg0;
+        a.vx = L.vx;
+        a.vy = L.vy;
+        a.wx = L.wx;
+        a.wy = L.wy;
+        a.lines = L.lines;
+        a.half = L.half;
+        a.slots = L.slots;
+        SAR_CUDA(launch_scatter(a, st), "forward scatter");
+        return SAR_OK;
+    }
     FpGridArgs a;
     a.g = p->gc_fwd;
     a.pulses = p->d_pulses + first;

@@ -1,0 +1,43 @@
+// sar_scatter.cuh -- forward scatter with a pulse per lane (sar_scatter.cu): layout and launch.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "sar_geom.cuh"
+
+namespace sar {
+
+constexpr int kWalk = 16;             // pixels of a line within a block
+constexpr int kScatterWarps = 4;    // warps (groups of 32 pulses) per CTA
+
+// The pixel lattice a scatter walks: pixel (a, b) is image pixel (i, j) = a v + b w, det(v, w) = +-1; a
+// block is `lines` lines (a) of kWalk pixels along w.
+struct ScatterLayout {
+    int vx = 1, vy = 0, wx = 0, wy = 1;
+    int lines = 16;
+    int half = 0;     // bins a block reaches on either side of its anchor's bin
+    int slots = 0;    // window slots per pulse
+    bool ok = false;
+    std::vector<int4> items;   // (a0, b0, blocks along w, plane) of each CTA's run of blocks
+};
+
+struct ScatterArgs {
+    GridConst img;              // the image grid (positions)
+    GridConst lat;              // the same with steps v, w (expansions)
+    const PulseGeom* pulses;    // [S]
+    const float2* x;            // image
+    float2* acc;                // [S][Lg], pre-zeroed
+    const int4* items;
+    unsigned* flags;
+    int num_items, S, Lg, bg0;
+    int vx, vy, wx, wy, lines, half, slots;
+};
+
+// Host-side choice of lattice, block and segments for linear sampling without split bins (see sar_scatter.cu).
+ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
+                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r);
+cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st);
+
+}  // namespace sar

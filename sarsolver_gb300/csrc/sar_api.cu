@@ -22,6 +22,7 @@
 
 #include "../../include/sargpu.h"
 #include "sar_fir.cuh"
+#include "sar_gather.cuh"
 #include "sar_host_prep.h"
 #include "sar_kernels.cuh"
 #include "sar_scatter.cuh"
@@ -115,6 +116,10 @@ struct sar_plan {
     bool values = false;   // stored profiles are plain values (kProfValues), not pairs
     int seg_tiles = 0, segs_per_column = 0, ws = 0, pbf = 16;
     size_t n_strips = 0;
+    GatherLayout gather;           // backprojection along iso-range lines (linear sampling, plain bins)
+    GridConst gc_gather{}, gc_adj_image{};   // its lattice, and the image grid
+    int4* d_tiles = nullptr;
+    float2* d_partial = nullptr;   // [gather.parts][P] partial images
     ScatterLayout scatter;         // forward scatter with a pulse per lane (linear sampling, plain bins)
     GridConst gc_scatter{}, gc_fwd_image{};   // its lattice, and the image grid
     int4* d_items = nullptr;
@@ -211,6 +216,8 @@ struct sar_plan {
         cudaFree(d_prof);
         cudaFree(d_strip);
         cudaFree(d_items);
+        cudaFree(d_tiles);
+        cudaFree(d_partial);
         cudaFree(d_flags);
         if (have_full) cufftDestroy(fft_full);
         if (have_tail) cufftDestroy(fft_tail);
@@ -540,6 +547,22 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
                 }
             }
         }
+        // Linear sampling with plain bins: the gather along iso-range lines (sar_gather.cu); the tile gather above
+        // serves the other plans.  Its tiles hold image pixels, so a tile's mean bin lies at most half a window
+        // outside the image's range: margins of two windows.
+        if (p->interp == SAR_INTERP_LINEAR && !p->gc_adj.precise_bins)
+            p->gather = gather_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+        if (p->gather.ok) {
+            const Lattice& L = p->gather.lattice;
+            double ea[3], eb[3];
+            for (int c = 0; c < 3; ++c) {
+                ea[c] = L.vx * ex[c] + L.vy * ey[c];
+                eb[c] = L.wx * ex[c] + L.wy * ey[c];
+            }
+            p->gc_adj_image = make_grid_const(ex, ey, ez, kappa, s_r, adjoint_bin_offset(p->interp), nx, ny, nz);
+            p->gc_gather = make_grid_const(ea, eb, ez, kappa, s_r, adjoint_bin_offset(p->interp), nx, ny, nz);
+            span_ww = std::max(span_ww, 2 * p->gather.ww + 8);
+        }
         p->bg0 = (long)std::floor(vmin) - span_ww / 2 - 4;
         const double span = std::ceil(vmax) + span_ww / 2 + 5 - (double)p->bg0;
         if (span > 2.0e9) return fail(SAR_ERR_NOT_SUPPORTED, "range span too large");
@@ -562,6 +585,7 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
                 break;
             }
         if (!p->staged && p->interp == SAR_INTERP_LINEAR) p->values = false;
+        if (p->gather.ok) p->values = true;   // three neighbouring values per run
         // Forward scatter layout: it walks the gather's lane axis (the transpose of its lane
         // choice), or, for linear sampling across the grid axes, a sheared lattice whose rows
         // follow the iso-range lines (choose_shear), walked with lanes along x.
@@ -588,8 +612,8 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             const ScatterLayout& L = p->scatter;
             double ea[3], eb[3];
             for (int c = 0; c < 3; ++c) {
-                ea[c] = L.vx * ex[c] + L.vy * ey[c];
-                eb[c] = L.wx * ex[c] + L.wy * ey[c];
+                ea[c] = L.lattice.vx * ex[c] + L.lattice.vy * ey[c];
+                eb[c] = L.lattice.wx * ex[c] + L.lattice.wy * ey[c];
             }
             p->gc_fwd_image = make_grid_const(ex, ey, ez, kappa, s_r, forward_bin_offset(p->interp), nx, ny, nz);
             p->gc_scatter = make_grid_const(ea, eb, ez, kappa, s_r, forward_bin_offset(p->interp), nx, ny, nz);
@@ -791,6 +815,12 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         }
         if ((rc = p->alloc(&p->d_steps, 9, "grid steps"))) return rc;
         SAR_CUDA(cudaMemcpy(p->d_steps, steps, sizeof steps, cudaMemcpyHostToDevice), "grid steps");
+    }
+    if (p->gather.ok) {
+        const std::vector<int4>& tiles = p->gather.tiles;
+        if ((rc = p->alloc(&p->d_tiles, tiles.size(), "gather tiles"))) return rc;
+        SAR_CUDA(cudaMemcpy(p->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice), "gather tiles");
+        if (p->gather.parts > 1 && (rc = p->alloc(&p->d_partial, (size_t)p->gather.parts * P, "partial images"))) return rc;
     }
     if (p->scatter.ok) {
         const std::vector<int4>& items = p->scatter.items;
@@ -1136,6 +1166,36 @@ static PointArgs point_args(sar_plan* p, int bin_rule) {
 // Grid gather of pulses [first, first + count) from pairs rows `pairs` (row 0 = pulse `first`).
 static int gather_pulses(sar_plan* p, const float4* pairs, size_t first, size_t count, float2* x, int accumulate,
                          cudaStream_t st) {
+    if (p->gather.ok) {
+        const GatherLayout& L = p->gather;
+        GatherArgs a;
+        a.img = p->gc_adj_image;
+        a.lat = p->gc_gather;
+        a.pulses = p->d_pulses + first;
+        a.prof = reinterpret_cast<const float2*>(pairs);
+        a.x = x;
+        a.partial = p->d_partial;
+        a.tiles = p->d_tiles;
+        a.flags = p->d_flags;
+        a.num_tiles = (int)L.tiles.size();
+        a.S = (int)count;
+        a.Lg = p->Lg;
+        a.bg0 = (int)p->bg0;
+        a.ww = L.ww;
+        a.pb = L.pb;
+        a.warps = L.warps;
+        a.parts = gather_parts(L, count, p->P);
+        a.accumulate = accumulate ? 1 : 0;
+        a.vx = L.lattice.vx;
+        a.vy = L.lattice.vy;
+        a.wx = L.lattice.wx;
+        a.wy = L.lattice.wy;
+        a.pixels = p->P;
+        a.wait_budget = p->wait_budget;
+        a.hold_first_stage = p->hold_first_stage;
+        SAR_CUDA(launch_gather(a, st), "backprojection");
+        return SAR_OK;
+    }
     BpGridArgs a;
     a.g = p->gc_adj;
     a.pulses = p->d_pulses + first;
@@ -1230,10 +1290,10 @@ static int scatter_pulses(sar_plan* p, const float2* x, float2* acc, size_t firs
         a.S = (int)count;
         a.Lg = p->Lg;
         a.bg0 = (int)p->bg0;
-        a.vx = L.vx;
-        a.vy = L.vy;
-        a.wx = L.wx;
-        a.wy = L.wy;
+        a.vx = L.lattice.vx;
+        a.vy = L.lattice.vy;
+        a.wx = L.lattice.wx;
+        a.wy = L.lattice.wy;
         a.lines = L.lines;
         a.half = L.half;
         a.slots = L.slots;

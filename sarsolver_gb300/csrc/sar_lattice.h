@@ -1,0 +1,171 @@
+// sar_lattice.h -- pixel lattices whose second axis follows the iso-range lines of a collection (host-only): the
+// order in which the linear-sampling kernels walk a grid (sar_scatter.cu, sar_gather.cu).
+//
+// Lattice pixel (a, b) is image pixel (i, j) = a v + b w with integer steps v, w and det(v, w) = +-1, so every
+// image pixel is one lattice pixel.  Along w the range bin should change as little as possible; of the
+// directions with |w|^2 <= 5 the one with the least cost is taken.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <vector>
+
+namespace sar {
+
+struct Lattice {
+    int vx = 1, vy = 0, wx = 0, wy = 1;
+    bool ok = false;
+};
+
+// `cost(rate)`: instructions per pixel-pulse at a bin rate (bins per step along w).  lines x along: the block of
+// lattice pixels the kernel works on, for the share of blocks that straddle the image's edges.
+template <class COST>
+inline Lattice choose_lattice(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
+                              const double* ey, const double* ez, int nx, int ny, int nz, double s_r, int lines, int along,
+                              COST cost) {
+    Lattice best;
+    double c0[3];
+    for (int d = 0; d < 3; ++d)
+        c0[d] = origin[d] + 0.5 * ((nx - 1) * ex[d] + (ny - 1) * ey[d] + (nz - 1) * ez[d]);
+    const int cand[8][4] = {{0, 1, 1, 0}, {1, 0, 0, 1}, {1, 1, 1, 0}, {-1, 1, 1, 0},
+                            {2, 1, 1, 0}, {-2, 1, 1, 0}, {1, 2, 0, 1}, {-1, 2, 0, 1}};   // w, v
+    double sum[8] = {};
+    for (size_t s = 0; s < S; ++s) {
+        double gx = 0.0, gy = 0.0;   // bin rates along x and y at the scene centre
+        for (int ant = 0; ant < 2; ++ant) {
+            const double* p = (ant ? rx : tx) + 3 * s;
+            const double w[3] = {c0[0] - p[0], c0[1] - p[1], c0[2] - p[2]};
+            const double r = std::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+            if (!(r > 0.0)) return best;
+            gx += s_r * (w[0] * ex[0] + w[1] * ex[1] + w[2] * ex[2]) / r;
+            gy += s_r * (w[0] * ey[0] + w[1] * ey[1] + w[2] * ey[2]) / r;
+        }
+        if (!std::isfinite(gx) || !std::isfinite(gy)) return best;
+        for (int c = 0; c < 8; ++c) sum[c] += cost(std::fabs(cand[c][0] * gx + cand[c][1] * gy));
+    }
+    double least = INFINITY;
+    for (int c = 0; c < 8; ++c) {
+        const double bx = along * std::abs(cand[c][0]) + lines * std::abs(cand[c][2]);   // a block's extent in pixels
+        const double by = along * std::abs(cand[c][1]) + lines * std::abs(cand[c][3]);
+        const double total = sum[c] * (1.0 + 0.5 * bx / nx) * (1.0 + 0.5 * by / ny);
+        if (total < least) {
+            least = total;
+            best.wx = cand[c][0];
+            best.wy = cand[c][1];
+            best.vx = cand[c][2];
+            best.vy = cand[c][3];
+        }
+    }
+    best.ok = true;
+    return best;
+}
+
+// Bin excursion of a block about its anchor.  For a pixel at d from the anchor an antenna's range moves by at most
+// |u.d| + |d|^2 / (2 R), u the unit vector at the anchor; u is taken at the centres of 4 x 4 cells of the scene,
+// where it changes by at most Dc / R towards any anchor of the cell (Dc its half-diagonal and a block's).
+struct LatticeBounds {
+    double len_a = 0.0, len_b = 0.0, nearest = INFINITY;
+    std::vector<double> ra, rb, rest;   // per pulse: largest |rate| along v and w (metres per step), largest Dc / R
+    bool ok = false;
+
+    // Largest excursion (bins) over pixels up to ha steps along v and hb along w from an anchor.
+    double excursion(double ha, double hb, double s_r) const {
+        const double reach = ha * len_a + hb * len_b;
+        double h = 0.0;
+        for (size_t s = 0; s < ra.size(); ++s)
+            h = std::max(h, ha * ra[s] + hb * rb[s] + reach * rest[s] + reach * reach / nearest);
+        return h * s_r;
+    }
+};
+
+inline LatticeBounds lattice_bounds(const Lattice& L, const double* tx, const double* rx, size_t S, const double* origin,
+                                    const double* ex, const double* ey, const double* ez, int nx, int ny, int nz,
+                                    double most_a, double most_b) {
+    LatticeBounds B;
+    double ea[3], eb[3];
+    for (int d = 0; d < 3; ++d) {
+        ea[d] = L.vx * ex[d] + L.vy * ey[d];
+        eb[d] = L.wx * ex[d] + L.wy * ey[d];
+    }
+    auto len = [](const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]); };
+    B.len_a = len(ea);
+    B.len_b = len(eb);
+    const double block = most_a * B.len_a + most_b * B.len_b;
+    const double Dc = 0.125 * (nx * len(ex) + ny * len(ey)) + 0.5 * nz * len(ez) + 2.0 * block;
+    B.ra.assign(S, 0.0);
+    B.rb.assign(S, 0.0);
+    B.rest.assign(S, 0.0);
+    for (size_t s = 0; s < S; ++s)
+        for (int cell = 0; cell < 16; ++cell) {
+            const double fx = ((cell & 3) + 0.5) / 4.0 * (nx - 1), fy = ((cell >> 2) + 0.5) / 4.0 * (ny - 1);
+            double a = 0.0, b = 0.0, q = 0.0;
+            for (int ant = 0; ant < 2; ++ant) {
+                const double* p = (ant ? rx : tx) + 3 * s;
+                double u[3];
+                for (int d = 0; d < 3; ++d)
+                    u[d] = p[d] - (origin[d] + fx * ex[d] + fy * ey[d] + 0.5 * (nz - 1) * ez[d]);
+                const double r = len(u), R = r - Dc;
+                if (!(R > 0.0)) return B;
+                B.nearest = std::min(B.nearest, R);
+                a += std::fabs(u[0] * ea[0] + u[1] * ea[1] + u[2] * ea[2]) / r;
+                b += std::fabs(u[0] * eb[0] + u[1] * eb[1] + u[2] * eb[2]) / r;
+                q += Dc / R;
+            }
+            B.ra[s] = std::max(B.ra[s], a);
+            B.rb[s] = std::max(B.rb[s], b);
+            B.rest[s] = std::max(B.rest[s], q);
+        }
+    B.ok = true;
+    return B;
+}
+
+// Strips of `lines` lattice lines and the interval [b0, b1] of offsets along them that holds image pixels.
+struct LatticeStrip {
+    int a0;
+    long b0, b1;
+};
+
+inline std::vector<LatticeStrip> lattice_strips(const Lattice& L, int lines, int nx, int ny) {
+    const int det = L.vx * L.wy - L.vy * L.wx;
+    int a_lo = 0, a_hi = 0;
+    for (int corner = 0; corner < 4; ++corner) {
+        const int i = (corner & 1) ? nx - 1 : 0, j = (corner & 2) ? ny - 1 : 0, a = det * (L.wy * i - L.wx * j);
+        a_lo = corner ? std::min(a_lo, a) : a;
+        a_hi = corner ? std::max(a_hi, a) : a;
+    }
+    auto clip = [](int v, int w, int a, int n, long* lo, long* hi) {   // 0 <= v a + w b <= n - 1
+        const long p = (long)v * a;
+        if (w == 0) {
+            if (p < 0 || p > n - 1) *hi = *lo - 1;
+            return;
+        }
+        long l = -p, h = n - 1 - p;   // bounds of w b
+        if (w < 0) {
+            std::swap(l, h);
+            l = -l;
+            h = -h;
+        }
+        const long q = std::abs(w);
+        *lo = std::max(*lo, l >= 0 ? (l + q - 1) / q : -((-l) / q));
+        *hi = std::min(*hi, h >= 0 ? h / q : -((-h + q - 1) / q));
+    };
+    std::vector<LatticeStrip> strips;
+    for (int a0 = a_lo; a0 <= a_hi; a0 += lines) {
+        LatticeStrip s{a0, 0, -1};
+        bool any = false;
+        for (int a = a0; a < a0 + lines; ++a) {
+            long lo = -(1L << 40), hi = 1L << 40;
+            clip(L.vx, L.wx, a, nx, &lo, &hi);
+            if (lo <= hi) clip(L.vy, L.wy, a, ny, &lo, &hi);
+            if (lo > hi) continue;
+            s.b0 = any ? std::min(s.b0, lo) : lo;
+            s.b1 = any ? std::max(s.b1, hi) : hi;
+            any = true;
+        }
+        if (any) strips.push_back(s);
+    }
+    return strips;
+}
+
+}  // namespace sar

@@ -27,8 +27,8 @@
 #include <algorithm>
 #include <cmath>
 
-#include "sar_host_prep.h"
 #include "sar_kernels.cuh"
+#include "sar_pipe.cuh"
 #include "sar_scatter.cuh"
 
 namespace sar {
@@ -43,32 +43,41 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 
-__device__ __forceinline__ PulseGeom load_pulse(const PulseGeom* p) {
-    const float4* v = reinterpret_cast<const float4*>(p);
-    const float4 a = __ldg(v), b = __ldg(v + 1), c = __ldg(v + 2), d = __ldg(v + 3);
-    PulseGeom g;
-    g.atx_hi[0] = a.x; g.atx_hi[1] = a.y; g.atx_hi[2] = a.z; g.atx_lo[0] = a.w;
-    g.atx_lo[1] = b.x; g.atx_lo[2] = b.y; g.arx_hi[0] = b.z; g.arx_hi[1] = b.w;
-    g.arx_hi[2] = c.x; g.arx_lo[0] = c.y; g.arx_lo[1] = c.z; g.arx_lo[2] = c.w;
-    g.rref_hi = d.x; g.rref_lo = d.y; g.monostatic = d.z; g.pad = d.w;
-    return g;
-}
-
 constexpr float kRunSpan = 0.98f;   // bins a run of pixels may span (its taps then lie in three bins)
 constexpr float kDip = 0.1f;        // bins a run may fall below its end points (curvature)
 
-// Terms of two neighbouring lines (a, a + 1): phase cph + b1 d + b2 d^2 + c9 d^3 in radians and bin
-// cv + bv1 d + bv2 d^2, d the offset along the line.
-struct LinePair {
-    float2 cph, b1, b2, c9, cv, bv1, bv2;
+// A block's set with the phase's linear coefficients reduced: c1 = c1' + w1 with |c1'| <= 1/8 and w1 a multiple of 1/4
+// (w1 di is exact and dropped to its fraction); c2 = c2' + w2 with |c2'| <= 1/4 and w2 a multiple of 1/2, whose part
+// w2 d is a whole number of turns at even offsets and h = w2 mod 1 at odd ones.  A line's phases stay below ~2.5
+// turns instead of 4.5, and FP32 rounds them to half the error (512^2 x 1024 against 64 bits: 5.5e-7 instead of 7.8e-7).
+struct BlockSet {
+    Coeffs co;
+    float w1, h;
 };
 
-__device__ __forceinline__ LinePair line_pair(const Coeffs& co, float di) {
+__device__ __forceinline__ void reduce_turns(BlockSet& q) {
+    q.w1 = 0.25f * rintf(4.f * q.co.c[1]);
+    const float w2 = 0.5f * rintf(2.f * q.co.c[2]);
+    q.co.c[1] -= q.w1;
+    q.co.c[2] -= w2;
+    q.h = w2 - rintf(w2);
+}
+
+// Terms of two neighbouring lines (a, a + 1): phase cph[d mod 2] + b1 d + b2 d^2 + c9 d^3 in radians and bin
+// cv + bv1 d + bv2 d^2, d the offset along the line.
+struct LinePair {
+    float2 cph[2], b1, b2, c9, cv, bv1, bv2;
+};
+
+__device__ __forceinline__ LinePair line_pair(const BlockSet& q, float di) {
+    const Coeffs& co = q.co;
     const float2 D = mk(di, di + 1.f), K = dup(SC_TWO_PI), SH = dup(SAR_SHIFTER), NSH = dup(-SAR_SHIFTER), M1 = dup(-1.f);
     LinePair t;
-    float2 ph = fma2(fma2(fma2(dup(co.c[6]), D, dup(co.c[3])), D, dup(co.c[1])), D, dup(co.c[0]));
-    ph = fma2(add2(add2(ph, SH), NSH), M1, ph);   // mod 1: the line's phases stay below ~5 cycles
-    t.cph = mul2(ph, K);
+    float2 w = mul2(dup(q.w1), D);
+    w = fma2(add2(add2(w, SH), NSH), M1, w);   // mod 1, exact
+    const float2 ph = add2(fma2(fma2(fma2(dup(co.c[6]), D, dup(co.c[3])), D, dup(co.c[1])), D, dup(co.c[0])), w);
+    t.cph[0] = mul2(ph, K);
+    t.cph[1] = mul2(add2(ph, dup(q.h)), K);
     t.b1 = mul2(fma2(fma2(dup(co.c[7]), D, dup(co.c[4])), D, dup(co.c[2])), K);
     t.b2 = mul2(fma2(dup(co.c[8]), D, dup(co.c[5])), K);
     t.c9 = dup(co.c[9] * SC_TWO_PI);
@@ -78,9 +87,9 @@ __device__ __forceinline__ LinePair line_pair(const Coeffs& co, float di) {
     return t;
 }
 
-// c = x exp(i phase) for the two lines' pixels at offset d (XN = -im).
-__device__ __forceinline__ void contribution(const LinePair& t, float2 d, float4 X, float2 XN, float2* cr, float2* ci) {
-    const float2 ph = fma2(fma2(fma2(t.c9, d, t.b2), d, t.b1), d, t.cph);
+// c = x exp(i phase) for the two lines' pixels at offset rr - 8 (XN = -im).
+__device__ __forceinline__ void contribution(const LinePair& t, int rr, float2 d, float4 X, float2 XN, float2* cr, float2* ci) {
+    const float2 ph = fma2(fma2(fma2(t.c9, d, t.b2), d, t.b1), d, t.cph[rr & 1]);
     float2 sn, cn;
     __sincosf(ph.x, &sn.x, &cn.x);
     __sincosf(ph.y, &sn.y, &cn.y);
@@ -93,13 +102,13 @@ __device__ __forceinline__ int wrap(int x, int W) { return (int)min((unsigned)x,
 
 // A block's lines with runs of G pixels; dip bounds how far the bin falls below a run's end points.
 template <int G>
-__device__ __forceinline__ void walk_runs(const Coeffs& co, const float4* xs, const float2* xn, float2* win, int off, int W,
+__device__ __forceinline__ void walk_runs(const BlockSet& q, const float4* xs, const float2* xn, float2* win, int off, int W,
                                           int lines) {
     const float2 SH = dup(SAR_SHIFTER), NSH = dup(-SAR_SHIFTER), M1 = dup(-1.f);
-    const float2 ndip = dup(-0.25f * (G - 1) * (G - 1) * fabsf(co.v[5]));
+    const float2 ndip = dup(-0.25f * (G - 1) * (G - 1) * fabsf(q.co.v[5]));
 #pragma unroll 1
     for (int l = 0; l < lines / 2; ++l) {
-        const LinePair t = line_pair(co, (float)(2 * l - lines / 2));
+        const LinePair t = line_pair(q, (float)(2 * l - lines / 2));
         const float4* xl = xs + l * kWalk;
         const float2* nl = xn + l * kWalk;
 #pragma unroll
@@ -114,7 +123,7 @@ __device__ __forceinline__ void walk_runs(const Coeffs& co, const float4* xs, co
             for (int rr = g0; rr < g0 + G; ++rr) {
                 const float2 d = dup((float)(rr - 8));
                 float2 cr, ci;
-                contribution(t, d, xl[rr], nl[rr], &cr, &ci);
+                contribution(t, rr, d, xl[rr], nl[rr], &cr, &ci);
                 const float2 av = fma2(fma2(t.bv2, d, t.bv1), d, cva);
                 const float2 aa = mk(fabsf(av.x), fabsf(av.y));
                 Cr = add2(Cr, cr);
@@ -147,19 +156,19 @@ __device__ __forceinline__ void walk_runs(const Coeffs& co, const float4* xs, co
 }
 
 // Both taps of every pixel (the bin moves too fast for runs).
-__device__ __forceinline__ void walk_taps(const Coeffs& co, const float4* xs, const float2* xn, float2* win, int off, int W,
+__device__ __forceinline__ void walk_taps(const BlockSet& q, const float4* xs, const float2* xn, float2* win, int off, int W,
                                           int lines) {
     const float2 SH = dup(SAR_SHIFTER), NSH = dup(-SAR_SHIFTER), M1 = dup(-1.f);
 #pragma unroll 1
     for (int l = 0; l < lines / 2; ++l) {
-        const LinePair t = line_pair(co, (float)(2 * l - lines / 2));
+        const LinePair t = line_pair(q, (float)(2 * l - lines / 2));
         const float4* xl = xs + l * kWalk;
         const float2* nl = xn + l * kWalk;
 #pragma unroll 4
         for (int rr = 0; rr < kWalk; ++rr) {
             const float2 d = dup((float)(rr - 8));
             float2 cr, ci;
-            contribution(t, d, xl[rr], nl[rr], &cr, &ci);
+            contribution(t, rr, d, xl[rr], nl[rr], &cr, &ci);
             const float2 v = fma2(fma2(t.bv2, d, t.bv1), d, t.cv);
             const float2 r = add2(v, SH);
             const float2 s = fma2(add2(r, NSH), M1, v);
@@ -256,7 +265,8 @@ __global__ void __launch_bounds__(32 * kScatterWarps, 4) scatter_kernel(const Sc
     for (int blk = 0; blk < item.z; ++blk) {
         fetch(blk + 1, &p, &q);   // in flight while this block is walked
         AnchorExpansion ae = expand_anchor(anchors[blk & 1], pg, a.lat);
-        Coeffs co;
+        BlockSet set;
+        Coeffs& co = set.co;
         phase_coeffs(ae, a.lat, co.c);
         const df vb = anchor_bin(ae, a.lat);
         const int base = base_bin_of(vb, 1.0f);
@@ -281,6 +291,7 @@ __global__ void __launch_bounds__(32 * kScatterWarps, 4) scatter_kernel(const Sc
             if (live) atomicOr(a.flags, FLAG_STRIP_WINDOW);
             co = Coeffs{};
         }
+        reduce_turns(set);
         // runs: the bin moves by less than kRunSpan over G pixels of a line (|rate| over the block, plus the
         // fall below the end points)
         const float rate = fabsf(co.v[2]) + 8.f * fabsf(co.v[4]) + 16.f * fabsf(co.v[5]), c2 = fabsf(co.v[5]);
@@ -288,13 +299,13 @@ __global__ void __launch_bounds__(32 * kScatterWarps, 4) scatter_kernel(const Sc
         const float4* bx = xs + (blk & 1) * block_px;
         const float2* bn = xn + (blk & 1) * block_px;
         if (__all_sync(0xffffffffu, 15.f * rate + 56.25f * c2 < kRunSpan && 56.25f * c2 < kDip))
-            walk_runs<16>(co, bx, bn, win, off, W, a.lines);
+            walk_runs<16>(set, bx, bn, win, off, W, a.lines);
         else if (__all_sync(0xffffffffu, 7.f * rate + 12.25f * c2 < kRunSpan && 12.25f * c2 < kDip))
-            walk_runs<8>(co, bx, bn, win, off, W, a.lines);
+            walk_runs<8>(set, bx, bn, win, off, W, a.lines);
         else if (__all_sync(0xffffffffu, 3.f * rate + 2.25f * c2 < kRunSpan && 2.25f * c2 < kDip))
-            walk_runs<4>(co, bx, bn, win, off, W, a.lines);
+            walk_runs<4>(set, bx, bn, win, off, W, a.lines);
         else
-            walk_taps(co, bx, bn, win, off, W, a.lines);
+            walk_taps(set, bx, bn, win, off, W, a.lines);
         stage(blk + 1, p, q);   // the other buffer: its last readers passed the previous barrier
         __syncthreads();
     }
@@ -329,153 +340,46 @@ double run_cost(double rate) {
 
 }  // namespace
 
-// The CTAs' runs of blocks: for every strip of `lines` lattice lines the interval of offsets that holds
-// image pixels, cut into segments so that a launch has about five waves of CTAs.
+// The CTAs' runs of blocks: each strip of `lines` lattice lines cut into segments so that a launch has about
+// five waves of CTAs.
 static void scatter_items(size_t S, int nx, int ny, int nz, ScatterLayout* L) {
-    const int vx = L->vx, vy = L->vy, wx = L->wx, wy = L->wy, det = vx * wy - vy * wx;
-    int a_lo = 0, a_hi = 0;
-    for (int corner = 0; corner < 4; ++corner) {
-        const int i = (corner & 1) ? nx - 1 : 0, j = (corner & 2) ? ny - 1 : 0, a = det * (wy * i - wx * j);
-        a_lo = corner ? std::min(a_lo, a) : a;
-        a_hi = corner ? std::max(a_hi, a) : a;
-    }
-    auto clip = [](int v, int w, int a, int n, long* lo, long* hi) {   // 0 <= v a + w b <= n - 1
-        const long p = (long)v * a;
-        if (w == 0) {
-            if (p < 0 || p > n - 1) *hi = *lo - 1;
-            return;
-        }
-        long l = -p, h = n - 1 - p;   // bounds of w b
-        if (w < 0) {
-            std::swap(l, h);
-            l = -l;
-            h = -h;
-        }
-        const long q = std::abs(w);
-        *lo = std::max(*lo, l >= 0 ? (l + q - 1) / q : -((-l) / q));
-        *hi = std::min(*hi, h >= 0 ? h / q : -((-h + q - 1) / q));
-    };
-    std::vector<int4> strips;
+    const std::vector<LatticeStrip> strips = lattice_strips(L->lattice, L->lines, nx, ny);
     long total = 0;
-    for (int a0 = a_lo; a0 <= a_hi; a0 += L->lines) {
-        long b0 = 0, b1 = -1;
-        bool any = false;
-        for (int a = a0; a < a0 + L->lines; ++a) {
-            long lo = -(1L << 40), hi = 1L << 40;
-            clip(vx, wx, a, nx, &lo, &hi);
-            if (lo <= hi) clip(vy, wy, a, ny, &lo, &hi);
-            if (lo > hi) continue;
-            b0 = any ? std::min(b0, lo) : lo;
-            b1 = any ? std::max(b1, hi) : hi;
-            any = true;
-        }
-        if (!any) continue;
-        const int n = (int)((b1 - b0) / kWalk) + 1;
-        total += n;
-        strips.push_back(make_int4(a0, (int)b0, n, 0));
-    }
+    for (const LatticeStrip& t : strips) total += (t.b1 - t.b0) / kWalk + 1;
     const size_t groups = (S + 32 * kScatterWarps - 1) / (32 * kScatterWarps);
-    const long len = std::max<long>(1, (long)((double)total * nz * groups / (152.0 * 12 / kScatterWarps * 5)));
+    const long len = std::max<long>(1, (long)((double)total * nz * groups / (152.0 * 3 * 5)));
     L->items.clear();
     for (int k = 0; k < nz; ++k)
-        for (const int4& t : strips) {
-            const int cuts = (int)((t.z + len - 1) / len);
-            for (int c = 0; c < cuts; ++c) {
-                const int p = (int)((long)t.z * c / cuts), q = (int)((long)t.z * (c + 1) / cuts);
-                L->items.push_back(make_int4(t.x, t.y + p * kWalk, q - p, k));
+        for (const LatticeStrip& t : strips) {
+            const long n = (t.b1 - t.b0) / kWalk + 1, cuts = (n + len - 1) / len;
+            for (long c = 0; c < cuts; ++c) {
+                const long p = n * c / cuts, q = n * (c + 1) / cuts;
+                L->items.push_back(make_int4(t.a0, (int)(t.b0 + p * kWalk), (int)(q - p), k));
             }
         }
 }
 
 ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
                              const double* ey, const double* ez, int nx, int ny, int nz, double s_r) {
-    ScatterLayout best;
-    double c0[3];
-    for (int d = 0; d < 3; ++d)
-        c0[d] = origin[d] + 0.5 * ((nx - 1) * ex[d] + (ny - 1) * ey[d] + (nz - 1) * ez[d]);
-    // bin rates along x and y at the scene centre, per pulse
-    std::vector<double> gx(S), gy(S);
-    for (size_t s = 0; s < S; ++s) {
-        gx[s] = gy[s] = 0.0;
-        for (int ant = 0; ant < 2; ++ant) {
-            const double* p = (ant ? rx : tx) + 3 * s;
-            const double w[3] = {c0[0] - p[0], c0[1] - p[1], c0[2] - p[2]};
-            const double r = std::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-            if (!(r > 0.0)) return best;
-            gx[s] += s_r * (w[0] * ex[0] + w[1] * ex[1] + w[2] * ex[2]) / r;
-            gy[s] += s_r * (w[0] * ey[0] + w[1] * ey[1] + w[2] * ey[2]) / r;
-        }
-        if (!std::isfinite(gx[s]) || !std::isfinite(gy[s])) return best;
-    }
-    // directions w of at most length sqrt(5) with an axis v that completes them to a basis
-    const int cand[8][4] = {{0, 1, 1, 0}, {1, 0, 0, 1}, {1, 1, 1, 0}, {-1, 1, 1, 0},
-                            {2, 1, 1, 0}, {-2, 1, 1, 0}, {1, 2, 0, 1}, {-1, 2, 0, 1}};
-    double least = INFINITY;
-    for (const auto& c : cand) {
-        double cost = 0.0;
-        for (size_t s = 0; s < S; ++s) cost += run_cost(std::fabs(c[0] * gx[s] + c[1] * gy[s]));
-        // blocks that straddle the image's edges: their extent along x and y, over the image's
-        const double bx = 16.0 * (std::abs(c[0]) + std::abs(c[2])), by = 16.0 * (std::abs(c[1]) + std::abs(c[3]));
-        cost *= (1.0 + 0.5 * bx / nx) * (1.0 + 0.5 * by / ny);
-        if (cost < least) {
-            least = cost;
-            best.wx = c[0];
-            best.wy = c[1];
-            best.vx = c[2];
-            best.vy = c[3];
-        }
-    }
-    // Window: for a pixel at d from its block's anchor (|line| <= lines / 2, |offset| <= 8) an antenna's range
-    // moves by at most |u.d| + |d|^2 / (2 R), u the unit vector at the anchor.  u is taken at the centres
-    // of 4 x 4 cells of the scene, where it changes by at most Dc / R towards any anchor of the cell (Dc its
-    // half-diagonal and a block's).  Lines are halved until the windows leave room for three CTAs per SM.
-    double ea[3], eb[3];
-    for (int d = 0; d < 3; ++d) {
-        ea[d] = best.vx * ex[d] + best.vy * ey[d];
-        eb[d] = best.wx * ex[d] + best.wy * ey[d];
-    }
-    auto len = [](const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]); };
-    const double block = 8.0 * (len(ea) + len(eb));
-    const double Dc = 0.125 * (nx * len(ex) + ny * len(ey)) + 0.5 * nz * len(ez) + 2.0 * block;
-    std::vector<double> ra(S, 0.0), rb(S, 0.0), rest(S, 0.0);   // largest rates and D / R of each pulse
-    double nearest = INFINITY;
-    for (size_t s = 0; s < S; ++s)
-        for (int cell = 0; cell < 16; ++cell) {
-            const double fx = ((cell & 3) + 0.5) / 4.0 * (nx - 1), fy = ((cell >> 2) + 0.5) / 4.0 * (ny - 1);
-            double a = 0.0, b = 0.0, q = 0.0;
-            for (int ant = 0; ant < 2; ++ant) {
-                const double* p = (ant ? rx : tx) + 3 * s;
-                double u[3];
-                for (int d = 0; d < 3; ++d)
-                    u[d] = p[d] - (origin[d] + fx * ex[d] + fy * ey[d] + 0.5 * (nz - 1) * ez[d]);
-                const double r = len(u), R = r - Dc;
-                if (!(R > 0.0)) return best;
-                nearest = std::min(nearest, R);
-                a += std::fabs(u[0] * ea[0] + u[1] * ea[1] + u[2] * ea[2]) / r;
-                b += std::fabs(u[0] * eb[0] + u[1] * eb[1] + u[2] * eb[2]) / r;
-                q += Dc / R;
-            }
-            ra[s] = std::max(ra[s], a);
-            rb[s] = std::max(rb[s], b);
-            rest[s] = std::max(rest[s], q);
-        }
-    for (best.lines = 16; best.lines >= 2; best.lines /= 2) {
-        const double ha = 0.5 * best.lines, hb = 8.0, reach = ha * len(ea) + hb * len(eb);
-        double h = 0.0;
-        for (size_t s = 0; s < S; ++s)
-            h = std::max(h, ha * ra[s] + hb * rb[s] + reach * rest[s] + reach * reach / nearest);
-        h = h * s_r + 0.1;
+    ScatterLayout L;
+    L.lattice = choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, 16, kWalk, run_cost);
+    if (!L.lattice.ok) return L;
+    const LatticeBounds B = lattice_bounds(L.lattice, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, 8.0, 8.0);
+    if (!B.ok) return L;
+    // lines are halved until the windows leave room for three CTAs per SM
+    for (L.lines = 16; L.lines >= 2; L.lines /= 2) {
+        const double h = B.excursion(0.5 * L.lines, 8.0, s_r) + 0.1;
         if (!(h < 4096.0)) continue;
         // taps from half a bin (the anchor's fraction), half a bin of rounding and kDip below to two bins above
-        best.half = (int)std::ceil(h + 1.0 + kDip);
-        best.slots = best.half + (int)std::ceil(h + 4.0);
-        if (scatter_smem(best.slots, best.lines).total <= 75 * 1024) {
-            best.ok = true;
+        L.half = (int)std::ceil(h + 1.0 + kDip);
+        L.slots = L.half + (int)std::ceil(h + 4.0);
+        if (scatter_smem(L.slots, L.lines).total <= 75 * 1024) {
+            L.ok = true;
+            scatter_items(S, nx, ny, nz, &L);
             break;
         }
     }
-    if (best.ok) scatter_items(S, nx, ny, nz, &best);
-    return best;
+    return L;
 }
 
 }  // namespace sar

@@ -6,16 +6,16 @@
 #include <vector>
 
 #include "sar_geom.cuh"
+#include "sar_lattice.h"
 
 namespace sar {
 
 constexpr int kWalk = 16;             // pixels of a line within a block
 constexpr int kScatterWarps = 4;    // warps (groups of 32 pulses) per CTA
 
-// The pixel lattice a scatter walks: pixel (a, b) is image pixel (i, j) = a v + b w, det(v, w) = +-1; a
-// block is `lines` lines (a) of kWalk pixels along w.
+// How a scatter walks its lattice: blocks of `lines` lines (along v) of kWalk pixels along w.
 struct ScatterLayout {
-    int vx = 1, vy = 0, wx = 0, wy = 1;
+    Lattice lattice;
     int lines = 16;
     int half = 0;     // bins a block reaches on either side of its anchor's bin
     int slots = 0;    // window slots per pulse

@@ -316,6 +316,14 @@ int sar_resample_phase_history(const void *ph_dev, size_t S, size_t N, const dou
                                double centre_freq, double sample_bandwidth, double sign_multiplier, double c_eff,
                                size_t new_N, const double *window, const double *kernel, size_t kernel_length,
                                const int *row0, size_t num_rows, void *out_dev, void *stream);
+/* The same with the caller's device scratch (256-byte aligned, sar_resample_workspace bytes) instead of an
+ * allocation of its own; stream-ordered: returns once the host arrays have been read, not when the result is there. */
+size_t sar_resample_workspace(size_t S, size_t N, size_t new_N, size_t kernel_length, size_t num_rows);
+int sar_resample_phase_history_ws(const void *ph_dev, size_t S, size_t N, const double *delta_range,
+                                  double centre_freq, double sample_bandwidth, double sign_multiplier, double c_eff,
+                                  size_t new_N, const double *window, const double *kernel, size_t kernel_length,
+                                  const int *row0, size_t num_rows, void *out_dev, void *workspace_dev,
+                                  size_t workspace_bytes, void *stream);
 
 /* ------------------------------------------------ 5. CPHD signal arrays (before the operator)
  * sar_cphd_decode: widen one CPHD signal array, copied to the device as it lies in the file

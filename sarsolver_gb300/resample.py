@@ -48,7 +48,12 @@ def range_changes(old_srps, new_srp, trans_posns, rec_posns) -> np.ndarray:
     tx, rx = np.asarray(trans_posns, np.float64), np.asarray(rec_posns, np.float64)
     old = np.asarray(old_srps, np.float64)
     new = np.broadcast_to(np.asarray(new_srp, np.float64), old.shape)
-    dist = lambda a, b: np.sqrt(((a - b) ** 2).sum(axis=-1))
+
+    def dist(a, b):   # by columns: numpy's reductions over an axis of three cost ten times as much
+        d = a - b
+        d *= d
+        return np.sqrt(d[..., 0] + d[..., 1] + d[..., 2])
+
     return np.ascontiguousarray((dist(tx, new) + dist(rx, new)) - (dist(tx, old) + dist(rx, old)))
 
 
@@ -100,8 +105,10 @@ def get_downsample_kernel(downsample_ratio: float) -> np.ndarray:
 
 def bad_slow_times(aperture) -> np.ndarray:
     """Pulses with a non-finite transmitter, receiver or SRP position (base/measurement.py:326-339)."""
-    ok = (np.isfinite(aperture.transmitter_positions).all(axis=1) & np.isfinite(aperture.receiver_positions).all(axis=1)
-          & np.isfinite(aperture.stab_ref_posns).all(axis=1))
+    posns = [np.asarray(p) for p in (aperture.transmitter_positions, aperture.receiver_positions, aperture.stab_ref_posns)]
+    if all(np.isfinite(p).all() for p in posns):
+        return np.zeros(0, dtype=np.int64)
+    ok = np.isfinite(posns[0]).all(axis=1) & np.isfinite(posns[1]).all(axis=1) & np.isfinite(posns[2]).all(axis=1)
     return np.nonzero(~ok)[0]
 
 
@@ -148,8 +155,10 @@ def resample_dataset(dataset, fast_downsample_factor: float = 1.0, slow_downsamp
     L = taps.shape[0]
     T = (S - L) // D - 1
     # windows [D t, D t + L) free of non-finite pulses, by a prefix count of bad pulses
+    bad = np.zeros(S, dtype=bool)
+    bad[bad_slow_times(ap)] = True
     badflag = np.zeros(S + 1, dtype=np.int64)
-    badflag[1:] = np.cumsum(np.isin(np.arange(S), bad_slow_times(ap)))
+    np.cumsum(bad, out=badflag[1:])
     cand = D * np.arange(max(T, 0), dtype=np.int64)
     starts = cand[(badflag[cand + L] - badflag[cand]) == 0]
     row0 = np.ascontiguousarray(starts.astype(np.int32))
@@ -164,13 +173,19 @@ def resample_dataset(dataset, fast_downsample_factor: float = 1.0, slow_downsamp
     out = torch.empty((len(starts), n), dtype=torch.complex64, device=dev)
     lib = _lib.load()
     with torch.cuda.device(dev):
-        _lib.check(lib.sar_resample_phase_history(
+        # scratch from PyTorch's allocator: kept between calls, and ordered on the current stream
+        need = lib.sar_resample_workspace(S, N, n, L, len(starts))
+        work = torch.empty(need, dtype=torch.uint8, device=dev)
+        _lib.check(lib.sar_resample_phase_history_ws(
             ctypes.c_void_p(x.data_ptr()), S, N, dr.ctypes.data_as(ctypes.c_void_p), float(ap.centre_frequency),
             float(ap.sample_bandwidth), float(ap.sign_multiplier), float(ap.c_eff), n,
             win.ctypes.data_as(ctypes.c_void_p), ktab.ctypes.data_as(ctypes.c_void_p), L,
-            row0.ctypes.data_as(ctypes.c_void_p), len(starts), ctypes.c_void_p(out.data_ptr()), _stream(dev)),
-            "sar_resample_phase_history")
-    wave = fast_freq_downsample(np.asarray(ap.waveform_fft)[None, :], n, safety_factor, device=dev)[0]
+            row0.ctypes.data_as(ctypes.c_void_p), len(starts), ctypes.c_void_p(out.data_ptr()),
+            ctypes.c_void_p(work.data_ptr()), need, _stream(dev)), "sar_resample_phase_history")
+    # the waveform is one row: transformed here in FP64, while the device works
+    modes = np.fft.ifft(np.fft.ifftshift(np.asarray(ap.waveform_fft, dtype=np.complex128)))
+    kept = np.concatenate([modes[:n // 2], modes[N - (n - n // 2):]])
+    wave = np.fft.fftshift(np.fft.fft(win * kept))
     wt = np.asarray(ap.slow_time_weighting, dtype=np.complex128)
     # sum_k taps[k] wt[s0 + k] for every window start s0 (a correlation, evaluated at the starts)
     new_wt = np.correlate(wt, np.conj(taps), mode="valid")[starts] if len(starts) else np.zeros(0, np.complex128)

@@ -99,3 +99,29 @@ def test_resampling_throughput_report():
     print(f"resample {S}x{N} -> {T}x{n}: {dt * 1e3:.2f} ms wall ({dev_ms:.2f} ms between events on the stream), "
           f"{moved / dt / 1e9:.0f} GB/s over the main passes")
     assert T > 0 and n == 4097
+
+
+@pytest.mark.parametrize("S,N,fast,slow,move", [
+    (16, 512, 1.7, 1, True), (40, 1024, 3.0, 3, True), (25, 2048, 1.0, 2, False), (12, 4096, 2.9, 1, True),
+    (30, 8192, 2.0, 2, True), (33, 511, 1.3, 2, True), (20, 1000, 2.5, 1, True), (9, 17, 1.0, 1, True),
+    (200, 300, 2.0, 12, True), (5000, 1200, 4.0, 1, True)])   # a filter of 60 taps; several chunks of work rows
+def test_resampling_matches_oracle(S, N, fast, slow, move):
+    """The filter before the transforms (fused for N = 512 ... 8192, chunked work rows otherwise) against the
+    FP64 restatement: rounding of two FP32 transforms and L products, a few 1e-7; 2e-6 leaves a factor of five."""
+    from oracle import resample as ora
+    rng = np.random.default_rng(S + N)
+    tx = np.stack([np.full(S, 9e3), np.linspace(-300, 300, S), np.full(S, 4e3)], axis=-1) + 0.1 * rng.standard_normal((S, 3))
+    srps = rng.standard_normal((S, 3)) if move else np.zeros((S, 3))
+    new = np.array([20.0, -10.0, 0.0]) if move else np.zeros(3)
+    ph = rng.standard_normal((S, N)) + 1j * rng.standard_normal((S, N))
+    wave, wt = rng.standard_normal(N) + 1j * rng.standard_normal(N), rng.standard_normal(S) + 0j
+    ap = NumpySimpleSarAperture(tx, tx.copy(), srps, 10e9, 200e6, waveform_fft=wave, slow_time_weighting=wt)
+    out = rs.resample_dataset(NumpySimpleSarDataset(ap, ph), fast, slow, new_srp=new)
+    n = min(int(1.0 + N / fast), N)
+    moved = ora.move_srps(ph, srps, new, tx, tx, 10e9, 200e6)
+    down, taps = ora.fast_freq_downsample(moved, n, 1.2), ora.downsample_kernel(slow)
+    L = len(taps)
+    T = (S - L) // slow - 1
+    want = np.stack([(taps[:, None] * down[slow * t:slow * t + L]).sum(axis=0) for t in range(T)])
+    assert rel(out.phase_history(), want) < 2e-6
+    assert rel(out.aperture.waveform_fft, ora.fast_freq_downsample(wave[None], n, 1.2)[0]) < 1e-6

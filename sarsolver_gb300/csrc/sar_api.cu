@@ -119,7 +119,8 @@ struct sar_plan {
     GatherLayout gather;           // backprojection along iso-range lines (linear sampling, plain bins)
     GridConst gc_gather{}, gc_adj_image{};   // its lattice, and the image grid
     int4* d_tiles = nullptr;
-    float2* d_partial = nullptr;   // [gather.parts][P] partial images
+    float2* d_partial = nullptr;   // [gather.parts or point_parts][P] partial images
+    int point_parts = 1;           // shares of the pulses of the unstructured backprojection
     ScatterLayout scatter;         // forward scatter with a pulse per lane (linear sampling, plain bins)
     GridConst gc_scatter{}, gc_fwd_image{};   // its lattice, and the image grid
     int4* d_items = nullptr;
@@ -822,6 +823,10 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         SAR_CUDA(cudaMemcpy(p->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice), "gather tiles");
         if (p->gather.parts > 1 && (rc = p->alloc(&p->d_partial, (size_t)p->gather.parts * P, "partial images"))) return rc;
     }
+    if (!grid) {
+        p->point_parts = point_parts(S, P);
+        if (p->point_parts > 1 && (rc = p->alloc(&p->d_partial, (size_t)p->point_parts * P, "partial images"))) return rc;
+    }
     if (p->scatter.ok) {
         const std::vector<int4>& items = p->scatter.items;
         if ((rc = p->alloc(&p->d_items, items.size(), "scatter blocks"))) return rc;
@@ -1266,7 +1271,7 @@ int sar_adjoint(sar_plan* p, const void* y_dev, void* x_dev, void* stream) {
     if (p->grid) {
         if ((rc = gather_pulses(p, p->d_prof, 0, p->S, (float2*)x_dev, 0, st))) return rc;
     } else {
-        SAR_CUDA(launch_bp_points(point_args(p, p->interp == SAR_INTERP_LINEAR ? BIN_LINEAR : BIN_ADJ_NEAREST), p->d_prof, (float2*)x_dev, 0, st),
+        SAR_CUDA(launch_bp_points(point_args(p, p->interp == SAR_INTERP_LINEAR ? BIN_LINEAR : BIN_ADJ_NEAREST), p->d_prof, (float2*)x_dev, p->d_partial, p->point_parts, st),
                  "backprojection");
     }
     mark(ev, 2, st);

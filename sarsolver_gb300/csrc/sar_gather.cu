@@ -309,6 +309,12 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float2* __restrict
     }
 }
 
+cudaError_t launch_sum_parts(const float2* partial, float2* x, size_t pixels, int parts, int accumulate, cudaStream_t st) {
+    sum_parts_kernel<<<(unsigned)std::min<size_t>((pixels + 255) / 256, 152 * 8), 256, 0, st>>>(partial, x, pixels, parts,
+                                                                                             accumulate);
+    return cudaGetLastError();
+}
+
 // Measured (GB300, this kernel alone, against the tile gather before): 2048^2 x 4096 pulses 12.4 ms (14.3);
 // 1024^2 x 2048 1.52 ms (1.88); 512^2 x 1024 0.22 ms (0.28).  19.6 instructions per pixel-pulse, of which the
 // producers' about 2; issue 64 %, FMA pipe 62 %, special functions 57 % of their cycles.  Tried: sign and
@@ -324,10 +330,7 @@ cudaError_t launch_gather(const GatherArgs& a, cudaStream_t st) {
         return cudaGetLastError();
     };
     cudaError_t e = a.warps == 8 ? go(gather_kernel<8>, 320) : a.warps == 4 ? go(gather_kernel<4>, 160) : cudaErrorInvalidValue;
-    if (e != cudaSuccess || a.parts == 1) return e;
-    sum_parts_kernel<<<(unsigned)std::min<size_t>((a.pixels + 255) / 256, 152 * 8), 256, 0, st>>>(a.partial, a.x, a.pixels,
-                                                                                               a.parts, a.accumulate);
-    return cudaGetLastError();
+    return e != cudaSuccess || a.parts == 1 ? e : launch_sum_parts(a.partial, a.x, a.pixels, a.parts, a.accumulate, st);
 }
 
 // ------------------------------------------------------------------ layout

@@ -538,7 +538,7 @@ SAR_HD df point_range(const df3& alpha, df alpha2, const PointGeom& pt) {
     q.z = df_make(pt.qh[2], pt.ql[2]);
     df dot = df_dot3(alpha, q);
     df W = df_add(alpha2, df_make(pt.qh[3], pt.ql[3]));
-    W = df_sub(W, df_mulf(dot, 2.0f));
+    W = df_sub(W, df_make(2.0f * dot.hi, 2.0f * dot.lo));   // exact
     return df_sqrt(W);
 }
 

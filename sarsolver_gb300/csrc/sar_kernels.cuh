@@ -107,8 +107,13 @@ struct PointArgs {
     unsigned* flags;
     int values = 0;            // 1: the backprojection's profiles are plain values (kProfValues)
 };
-cudaError_t launch_bp_points(const PointArgs& a, const float4* pairs, float2* x, int accumulate,
+// Shares of the pulses that fill the GPU (each at least a stage of pulses), and the gather over them with
+// partial images [parts][P] when parts > 1.
+int point_parts(size_t S, size_t P);
+cudaError_t launch_bp_points(const PointArgs& a, const float4* pairs, float2* x, float2* partial, int parts,
                              cudaStream_t st);
+// x (+)= sum of partial images [parts][pixels], added in order (sar_gather.cu).
+cudaError_t launch_sum_parts(const float2* partial, float2* x, size_t pixels, int parts, int accumulate, cudaStream_t st);
 cudaError_t launch_fp_points(const PointArgs& a, const float2* x, float2* acc, cudaStream_t st);
 
 // FFT-side kernels (K1 / K4).  y is [S][N] fftshifted along fast time; spec is [rows][M] of

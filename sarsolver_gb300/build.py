@@ -22,7 +22,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fno-fast-math"]
 CUDA_UNITS = ["sar_kernels.cu", "sar_fir.cu", "sar_scatter.cu", "sar_gather.cu", "sar_api.cu", "sar_noalloc.cu", "sar_cgls.cu", "sar_unet.cu", "sar_resample.cu", "sar_cphd.cu", "sar_pdhg.cu", "sar_probe.cu"]
-HEADERS = ["sar_geom.cuh", "sar_host_prep.h", "sar_kernels.cuh", "sar_stockham.cuh", "sar_fir.cuh", "sar_lattice.h", "sar_scatter.cuh", "sar_gather.cuh", "sar_pipe.cuh", "unet_tc.cuh", "sar_fft_cb.h", "sar_solver_common.cuh"]
+HEADERS = ["sar_geom.cuh", "sar_host_prep.h", "sar_kernels.cuh", "sar_stockham.cuh", "sar_fir.cuh", "sar_lattice.h", "sar_scatter.cuh", "sar_gather.cuh", "sar_pipe.cuh", "sar_exact.cuh", "unet_tc.cuh", "sar_fft_cb.h", "sar_solver_common.cuh"]
 # cuFFT load/store callbacks: compiled to LTO-IR, embedded in the library as a byte array and
 # handed to cufftXtSetJITCallback at plan creation.
 CALLBACK_UNIT = "sar_fft_callbacks.cu"

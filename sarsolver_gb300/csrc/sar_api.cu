@@ -89,7 +89,8 @@ bool finite3(const double* v, size_t n) {
 // Shared-memory budgets: two tile CTAs per SM.
 constexpr size_t kBpSmemBudget = 110 * 1024;
 constexpr size_t kFpSmemBudget = 110 * 1024;
-constexpr size_t kFpRingSmemBudget = 220 * 1024;   // ring windows: one CTA per SM
+constexpr size_t kFpRingTwoBudget = 113 * 1024 - 256;   // ring windows: two CTAs per SM (228 KB, 1 KB each reserved)
+constexpr size_t kFpRingSmemBudget = 220 * 1024;   // one CTA per SM
 constexpr size_t kSpecBudget = (size_t)4 << 30;   // bytes of FFT work rows per chunk
 
 }  // namespace
@@ -677,8 +678,8 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
                             }
                         }
                 const int ws = (need + 31) & ~31;
-                if (fp_grid_ws_smem_bytes(ws, pbf, p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins) <=
-                    kFpSmemBudget) {
+                if (fp_grid_ws_smem_bytes(ws, pbf, p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins, 0,
+                                          p->interp == SAR_INTERP_NEAREST_REF) <= kFpSmemBudget) {
                     p->seg_tiles = seg;
                     p->segs_per_column = segs;
                     p->ws = ws;
@@ -695,29 +696,31 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         }
         // Ring windows (split bins): where strip windows hold only one or two tiles (a 32-pixel tile
         // spans ~1200 bins at upsample 128), every CTA would clear and merge a whole window for 1024
-        // pixels per pulse.  A ring of W = 2^k >= 2 H + 1 slots per pulse instead holds one tile's
+        // pixels per pulse.  A ring of at least 2 H + 1 slots per pulse instead holds one tile's
         // range (its base bin +- H, H from the look directions as for the gather's windows) and a CTA
-        // walks its whole line, adding and clearing only the bins each tile step leaves behind.
+        // walks its whole line, adding and clearing only the bins each tile step leaves behind.  Two CTAs
+        // per SM where the rings allow it, else one.
         if (p->gc_fwd.precise_bins && (p->forward_points || p->seg_tiles <= 2)) {
-            const double hd = tile_halfspan_directional(tx, rx, S, origin, ex, ey, ez, kTile, p->gc_fwd.tiles_x,
-                                                        p->gc_fwd.tiles_y, nz, s_r);
-            const double h = hd >= 0.0 ? hd : 0.5 * grid_tile_window(g, s_r);
+            const Lattice plain{1, 0, 0, 1, true};
+            const LatticeBounds B = lattice_bounds(plain, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, 16.0, 16.0);
+            const double h = B.ok ? B.excursion(16.0, 16.0, s_r) : 0.5 * grid_tile_window(g, s_r);
             if (h >= 0.0 && h < 1.0e6) {
-                const int H = (int)std::ceil(h) + 4;
-                int W = 32;
-                while (W < 2 * H + 1) W *= 2;
-                for (int pbf : {16, 8})
-                    if (fp_grid_ws_smem_bytes(W, pbf, 0) <= kFpRingSmemBudget) {
-                        p->ring_half = H;
-                        p->ws = W;
-                        p->pbf = pbf;
-                        p->seg_tiles = along;
-                        p->segs_per_column = 1;
-                        p->n_strips = (size_t)nz * lines;
-                        strip_start.assign(p->n_strips * S, 0);   // not read with ring windows
-                        p->forward_points = false;
-                        break;
-                    }
+                const int H = (int)std::ceil(h) + 4, W = (2 * H + 1 + 31) & ~31;
+                for (size_t budget : {kFpRingTwoBudget, kFpRingSmemBudget}) {
+                    if (p->ring_half) break;
+                    for (int pbf : {16, 8})
+                        if (fp_grid_ws_smem_bytes(W, pbf, 0, 1, p->interp == SAR_INTERP_NEAREST_REF) <= budget) {
+                            p->ring_half = H;
+                            p->ws = W;
+                            p->pbf = pbf;
+                            p->seg_tiles = along;
+                            p->segs_per_column = 1;
+                            p->n_strips = (size_t)nz * lines;
+                            strip_start.assign(p->n_strips * S, 0);   // not read with ring windows
+                            p->forward_points = false;
+                            break;
+                        }
+                }
             }
         }
         if (p->forward_points) {

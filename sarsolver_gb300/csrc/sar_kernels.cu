@@ -18,6 +18,7 @@
 // (value at the interpolation midpoint, difference to the next bin) so that one 16-byte
 // load gives a linearly interpolated sample.
 #include "sar_kernels.cuh"
+#include "sar_exact.cuh"
 #include "sar_pipe.cuh"
 #include "sar_stockham.cuh"
 
@@ -155,49 +156,6 @@ __device__ __forceinline__ PixelEval eval_pixel(const ColumnTerms& ct, float c9,
     return e;
 }
 
-// Nearest-bin sampling on the grid paths.  The FP32 bin coordinate s (about the chosen bin, in
-// [-0.5, 0.5]) is within ~5e-6 bins of the FP64 position (split bins, sar_geom.cuh); where |s|
-// exceeds kNearEdge the bin is decided again from the per-pixel double-float range with the
-// unstructured path's exact rule (exact_bin: FP64 rounding of the same value, ties away from
-// zero), so the grid kernels pick the bins the per-pixel path picks.  About 1e-4 of the
-// pixel·pulses take this branch.
-constexpr float kNearEdge = 0.49995f;
-
-// Stored-span index (bins from bg0) of grid pixel (i, j, k) for pulse s under nearest rule `rule`:
-// pixel offset from the grid origin in FP64 as the host forms it, then the double-float range and
-// rounding of the per-pixel kernels (eval_point).
-__device__ __noinline__ int exact_grid_bin(const double* __restrict__ steps, const PulseGeom* __restrict__ pulses,
-                                           const float4* __restrict__ alpha2, float sr_hi, float sr_lo, int bg0,
-                                           int rule, int i, int j, int k, int s) {
-    double q[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        q[c] = __dadd_rn(__dadd_rn(__dmul_rn((double)i, steps[c]), __dmul_rn((double)j, steps[3 + c])),
-                         __dmul_rn((double)k, steps[6 + c]));
-    const double qq = __dadd_rn(__dadd_rn(__dmul_rn(q[0], q[0]), __dmul_rn(q[1], q[1])), __dmul_rn(q[2], q[2]));
-    PointGeom pt;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        pt.qh[c] = __double2float_rn(q[c]);
-        pt.ql[c] = __double2float_rn(__dsub_rn(q[c], (double)pt.qh[c]));
-    }
-    pt.qh[3] = __double2float_rn(qq);
-    pt.ql[3] = __double2float_rn(__dsub_rn(qq, (double)pt.qh[3]));
-    const PulseGeom pg = load_pulse(pulses + s);
-    const float4 a2 = __ldg(alpha2 + s);
-    df r = point_range(pulse_tx(pg), df_make(a2.x, a2.y), pt);
-    if (pg.monostatic != 0.0f)
-        r = df_mulf(r, 2.0f);
-    else
-        r = df_add(r, point_range(pulse_rx(pg), df_make(a2.z, a2.w), pt));
-    r = df_sub(r, df_make(pg.rref_hi, pg.rref_lo));
-    const df V = df_sub(df_mul(df_make(sr_hi, sr_lo), r), df_make((float)bg0, 0.0f));
-    int gi;
-    float sf;
-    exact_bin(V, bg0, rule, &gi, &sf);
-    return gi;
-}
-
 // ------------------------------------------------------------------- K2 (grid, wide windows)
 // Fallback for tiles whose range window is too wide to stage in shared memory: coefficient sets
 // per block of pulses in shared memory, profile pairs read straight from global memory (L2).
@@ -249,9 +207,9 @@ __global__ void __launch_bounds__(kThreads, 2) bp_grid_kernel(const BpGridArgs a
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
                     if (fabsf(e4[r].sf) > kNearEdge)
-                        gi4[r] = min(max(exact_grid_bin(a.steps, a.pulses, a.alpha2, g.s_r.hi, g.s_r.lo, a.bg0,
-                                                        BIN_ADJ_NEAREST, ti * kTile + (threadIdx.x & 31),
-                                                        tj * kTile + 4 * (threadIdx.x >> 5) + r, k, s0 + pi),
+                        gi4[r] = min(max(exact_grid_sample<false>(a.steps, a.pulses, a.alpha2, g.kappa, g.s_r, a.bg0, BIN_ADJ_NEAREST,
+                                                           ti * kTile + (threadIdx.x & 31),
+                                                           tj * kTile + 4 * (threadIdx.x >> 5) + r, k, s0 + pi).gi,
                                          0), a.Lg - 1);
             }
 #pragma unroll
@@ -715,8 +673,8 @@ __global__ void __launch_bounds__(kWsThreads, 2) bp_grid_ws_pair_kernel(const Bp
                         // either way; for pair windows where the producer placed it
                         const int g0 = VALUES ? base0[b * pb + 2 * pp + h] - ww / 2 - a.bg0
                                               : min(max(base0[b * pb + 2 * pp + h] - ww / 2 - a.bg0, 0), a.Lg - ww);
-                        const int gi = exact_grid_bin(a.steps, a.pulses, a.alpha2, g.s_r.hi, g.s_r.lo, a.bg0,
-                                                      BIN_ADJ_NEAREST, px, py, k, sp + h);
+                        const int gi = exact_grid_sample<false>(a.steps, a.pulses, a.alpha2, g.kappa, g.s_r, a.bg0,
+                                                         BIN_ADJ_NEAREST, px, py, k, sp + h).gi;
                         const unsigned w = min((unsigned)(gi - g0), idx_max);
                         if (LANES_Y || VALUES) {
                             if (h) ib = w; else ia = w;
@@ -868,17 +826,19 @@ constexpr int kXtStride = kTile + 1;   // staged image tile: 32 lines of 33 valu
 
 __device__ __forceinline__ size_t align_up(size_t n, size_t a) { return (n + a - 1) & ~(a - 1); }
 
-__host__ __device__ inline int window_slots(int ws) { return ws + (ws >> 4) + 1; }
+// Ring windows are not padded: they hold wide tiles, whose lanes' bins spread over the banks by themselves, and
+// without the padding two CTAs fit an SM at upsample 128.
+__host__ __device__ inline int window_slots(int ws, int ring) { return ring ? ws : ws + (ws >> 4) + 1; }
 
 struct FpWsLayout {
-    size_t win, coef, xt, base, fast, wst, bars, anchors, total;
+    size_t win, coef, xt, base, fast, wst, bars, anchors, queue, total;
 };
 
 // wide_x: image values staged as (re, re, im, im) (the linear run-window kernels), else (re, im).
-__host__ __device__ inline FpWsLayout fp_ws_layout(int ws, int pbf, int wide_x) {
+__host__ __device__ inline FpWsLayout fp_ws_layout(int ws, int pbf, int wide_x, int ring, int nearest) {
     FpWsLayout L;
     L.win = 0;
-    L.coef = L.win + (size_t)pbf * window_slots(ws) * sizeof(float2);
+    L.coef = L.win + (size_t)pbf * window_slots(ws, ring) * sizeof(float2);
     L.coef = (L.coef + 15) & ~(size_t)15;
     L.xt = L.coef + (size_t)2 * pbf * 4 * kSetF4 * sizeof(float4);
     L.base = L.xt + (size_t)2 * kTile * kXtStride * (wide_x ? sizeof(float4) : sizeof(float2));
@@ -886,15 +846,21 @@ __host__ __device__ inline FpWsLayout fp_ws_layout(int ws, int pbf, int wide_x) 
     L.wst = L.fast + (size_t)2 * pbf * sizeof(int);
     L.bars = (L.wst + (size_t)pbf * sizeof(int) + 7) & ~(size_t)7;
     L.anchors = L.bars + 4 * sizeof(uint64_t);
-    L.total = L.anchors + (size_t)kWsProducers * 4 * sizeof(df3);
+    L.queue = L.anchors + (size_t)kWsProducers * 4 * sizeof(df3);
+    L.total = L.queue + (nearest ? (size_t)8 * kNearQueue * sizeof(int2) : 0);
     return L;
 }
 
-size_t fp_grid_ws_smem_bytes(int ws, int pbf, int wide_x) { return fp_ws_layout(ws, pbf, wide_x).total; }
+size_t fp_grid_ws_smem_bytes(int ws, int pbf, int wide_x, int ring, int nearest) {
+    return fp_ws_layout(ws, pbf, wide_x, ring, nearest).total;
+}
 
 // Window slot of bin w: one padding slot every 16 bins, so lanes whose bins differ by a
 // multiple of 16 do not share a shared-memory bank pair.
-__device__ __forceinline__ int wslot(int w) { return w + (w >> 4); }
+template <bool RING>
+__device__ __forceinline__ int wslot(int w) { return RING ? w : w + (w >> 4); }
+// Ring slot of x in [0, 2 ws).
+__device__ __forceinline__ int ring_wrap(int x, int ws) { return (int)min((unsigned)x, (unsigned)(x - ws)); }
 
 template <bool PRECISE>
 struct RowEval {
@@ -917,8 +883,9 @@ __device__ __forceinline__ RowEval<PRECISE> scatter_eval(const ColumnTerms& ct, 
     return e;
 }
 
+template <bool RING = false>
 __device__ __forceinline__ void rmw_add(float2* wp, int idx, float w, float cr, float ci) {
-    float2* q = wp + wslot(idx);
+    float2* q = wp + wslot<RING>(idx);
     float2 u = *q;
     u.x = fmaf(w, cr, u.x);
     u.y = fmaf(w, ci, u.y);
@@ -929,127 +896,150 @@ __device__ __forceinline__ void rmw_add(float2* wp, int idx, float w, float cr, 
 __device__ __forceinline__ float2 staged_value(const float2 v) { return v; }
 __device__ __forceinline__ float2 staged_value(const float4 v) { return make_float2(v.x, v.z); }
 
-// What the nearest-bin scatter needs to decide a bin again exactly (exact_grid_bin): the pixel of
-// row 0 / lane 0 of the half tile, the walk direction, both pulses and their window starts.
-struct NearCtx {
-    const double* steps;
-    const PulseGeom* pulses;
-    const float4* alpha2;
-    float sr_hi, sr_lo;
-    int bg0, i0, j0, k, transposed;
-    int sp, sq;     // pulse indices
-    int wsp, wsq;   // first bin (absolute) of each pulse's window
-    int a_off, shear;   // lattice pixel (i, j) is image pixel (i + a_off + shear j, j)
-};
-
 // 16 rows of one half tile for the pulse pair (p, q).  MODE 2: bins n, n+1 of different lanes
-// disjoint (one phase per row); MODE 1: bins n distinct (two phases); MODE 0: atomics.  Nearest
-// bins within 5e-5 of a rounding boundary are decided again exactly; such a bin may equal a
-// neighbouring lane's, so those contributions go in with atomics in a phase of their own.
-// RING: ring windows (ws a power of two; off_p / off_q are the pulses' absolute base bins and a
-// bin's slot is its absolute index mod ws), else strip windows (off = base - window start).
+// disjoint (one phase per row); MODE 1: bins n distinct (two phases); MODE 0: atomics.
+// RING: ring windows (off_p / off_q + bin is a slot before wrapping, in [0, 2 ws)), else strip windows
+// (off = base - window start).
 template <bool LINEAR, bool PRECISE, int MODE, bool TWO, typename XT, bool RING = false>
 __device__ __forceinline__ void scatter_rows(const ColumnTerms& ctp, float c9p, float w9p, float ibp,
                                              const ColumnTerms& ctq, float c9q, float w9q, float ibq,
                                              const XT* xrow, float2* wp, float2* wq, int off_p, int off_q,
-                                             int ws, int lane, const NearCtx& nc) {
-    const int mask = ws - 1;
+                                             int ws, int lane) {
+    auto slot = [&](int i) { return RING ? ring_wrap(i, ws) : (int)min((unsigned)i, (unsigned)(ws - 2)); };
     // the slot after slot i (the second tap of linear sampling)
-    auto next = [&](int i) { return RING ? ((i + 1) & mask) : i + 1; };
+    auto next = [&](int i) { return RING ? ring_wrap(i + 1, ws) : i + 1; };
     // the lane's phase constant and its rate along the rows mod 1 (rows are integer offsets)
     ColumnTerms cp = ctp, cq = ctq;
     cp.cph -= rintf(cp.cph);
     cp.b1 -= rintf(cp.b1);
     cq.cph -= rintf(cq.cph);
     cq.b1 -= rintf(cq.b1);
-    unsigned edge = 0;   // nearest bins: bit 2 row + h for the pulse h contribution near a rounding boundary
 #pragma unroll 2
     for (int rr = 0; rr < 16; ++rr) {
         const float dj = (float)(rr - 8);
         const float2 xv = staged_value(xrow[rr * kXtStride + lane]);
         const RowEval<PRECISE> ep = scatter_eval<PRECISE>(cp, c9p, w9p, ibp, dj, xv);
-        const int ip = RING ? ((ep.bp.n + off_p) & mask) : (int)min((unsigned)(ep.bp.n + off_p), (unsigned)(ws - 2));
+        const int ip = slot(ep.bp.n + off_p);
         RowEval<PRECISE> eq;
         int iq = 0;
         if (TWO) {
             eq = scatter_eval<PRECISE>(cq, c9q, w9q, ibq, dj, xv);
-            iq = RING ? ((eq.bp.n + off_q) & mask) : (int)min((unsigned)(eq.bp.n + off_q), (unsigned)(ws - 2));
+            iq = slot(eq.bp.n + off_q);
         }
         if (LINEAR) {
             const float w0p = 0.5f - ep.bp.s, w1p = 0.5f + ep.bp.s;
             const float w0q = TWO ? 0.5f - eq.bp.s : 0.f, w1q = TWO ? 0.5f + eq.bp.s : 0.f;
             if (MODE == 2) {
-                rmw_add(wp, ip, w0p, ep.cr, ep.ci);
-                rmw_add(wp, next(ip), w1p, ep.cr, ep.ci);
+                rmw_add<RING>(wp, ip, w0p, ep.cr, ep.ci);
+                rmw_add<RING>(wp, next(ip), w1p, ep.cr, ep.ci);
                 if (TWO) {
-                    rmw_add(wq, iq, w0q, eq.cr, eq.ci);
-                    rmw_add(wq, next(iq), w1q, eq.cr, eq.ci);
+                    rmw_add<RING>(wq, iq, w0q, eq.cr, eq.ci);
+                    rmw_add<RING>(wq, next(iq), w1q, eq.cr, eq.ci);
                 }
                 __syncwarp();
             } else if (MODE == 1) {
-                rmw_add(wp, ip, w0p, ep.cr, ep.ci);
-                if (TWO) rmw_add(wq, iq, w0q, eq.cr, eq.ci);
+                rmw_add<RING>(wp, ip, w0p, ep.cr, ep.ci);
+                if (TWO) rmw_add<RING>(wq, iq, w0q, eq.cr, eq.ci);
                 __syncwarp();
-                rmw_add(wp, next(ip), w1p, ep.cr, ep.ci);
-                if (TWO) rmw_add(wq, next(iq), w1q, eq.cr, eq.ci);
+                rmw_add<RING>(wp, next(ip), w1p, ep.cr, ep.ci);
+                if (TWO) rmw_add<RING>(wq, next(iq), w1q, eq.cr, eq.ci);
                 __syncwarp();
             } else {
-                float2* a0 = wp + wslot(ip);
-                float2* a1 = wp + wslot(next(ip));
+                float2* a0 = wp + wslot<RING>(ip);
+                float2* a1 = wp + wslot<RING>(next(ip));
                 atomicAdd(&a0->x, w0p * ep.cr); atomicAdd(&a0->y, w0p * ep.ci);
                 atomicAdd(&a1->x, w1p * ep.cr); atomicAdd(&a1->y, w1p * ep.ci);
                 if (TWO) {
-                    float2* b0 = wq + wslot(iq);
-                    float2* b1 = wq + wslot(next(iq));
+                    float2* b0 = wq + wslot<RING>(iq);
+                    float2* b1 = wq + wslot<RING>(next(iq));
                     atomicAdd(&b0->x, w0q * eq.cr); atomicAdd(&b0->y, w0q * eq.ci);
                     atomicAdd(&b1->x, w1q * eq.cr); atomicAdd(&b1->y, w1q * eq.ci);
                 }
             }
         } else {
-            if (PRECISE)   // decided again after the rows, off the common path
-                edge |= ((fabsf(ep.bp.s) > kNearEdge ? 1u : 0u) | (TWO && fabsf(eq.bp.s) > kNearEdge ? 2u : 0u))
-                        << (2 * rr);
             if (MODE >= 1) {
-                rmw_add(wp, ip, 1.0f, ep.cr, ep.ci);
-                if (TWO) rmw_add(wq, iq, 1.0f, eq.cr, eq.ci);
+                rmw_add<RING>(wp, ip, 1.0f, ep.cr, ep.ci);
+                if (TWO) rmw_add<RING>(wq, iq, 1.0f, eq.cr, eq.ci);
                 __syncwarp();
             } else {
-                float2* a0 = wp + wslot(ip);
+                float2* a0 = wp + wslot<RING>(ip);
                 atomicAdd(&a0->x, ep.cr); atomicAdd(&a0->y, ep.ci);
                 if (TWO) {
-                    float2* b0 = wq + wslot(iq);
+                    float2* b0 = wq + wslot<RING>(iq);
                     atomicAdd(&b0->x, eq.cr); atomicAdd(&b0->y, eq.ci);
                 }
             }
         }
     }
-    if (!LINEAR && PRECISE && __any_sync(0xffffffffu, edge != 0u)) {
-        // Contributions whose FP32 bin position lay within 5e-5 of a rounding boundary: the exact bin
-        // from the per-pixel double-float range; where it differs from the FP32 bin (where the rows
-        // added it) the contribution moves there, with shared-memory atomics (the lanes' exact bins
-        // may coincide).  The row's evaluation is repeated exactly as the rows made it.
-        for (unsigned m = edge; m != 0u; m &= m - 1u) {
-            const int bit = __ffs(m) - 1, rr = bit >> 1, h = bit & 1;
-            const float dj = (float)(rr - 8);
-            const float2 xv = staged_value(xrow[rr * kXtStride + lane]);
-            const RowEval<PRECISE> e = h ? scatter_eval<PRECISE>(cq, c9q, w9q, ibq, dj, xv)
-                                         : scatter_eval<PRECISE>(cp, c9p, w9p, ibp, dj, xv);
-            const int off = h ? off_q : off_p;
-            const int i32 = RING ? ((e.bp.n + off) & mask) : (int)min((unsigned)(e.bp.n + off), (unsigned)(ws - 2));
-            const int pj = nc.j0 + (nc.transposed ? lane : rr);
-            const int pi = nc.i0 + (nc.transposed ? rr : lane) + nc.a_off + nc.shear * pj;
-            const int bx = exact_grid_bin(nc.steps, nc.pulses, nc.alpha2, nc.sr_hi, nc.sr_lo, nc.bg0, BIN_FWD_NEAREST,
-                                          pi, pj, nc.k, h ? nc.sq : nc.sp) + nc.bg0;
-            const int ix = RING ? (bx & mask) : min(max(bx - (h ? nc.wsq : nc.wsp), 0), ws - 1);
-            if (ix == i32) continue;
-            float2* w = h ? wq : wp;
-            atomicAdd(&w[wslot(i32)].x, -e.cr);
-            atomicAdd(&w[wslot(i32)].y, -e.ci);
-            atomicAdd(&w[wslot(ix)].x, e.cr);
-            atomicAdd(&w[wslot(ix)].y, e.ci);
+}
+
+// Nearest bins with exact integer parts: the same with both pulses' polynomials, phases and products in packed
+// instructions (20 instructions per pixel-pulse against 56).  near_terms holds a half tile's polynomials of the
+// pulse pair, phases in radians; near_bins the bins of one row, for the rows and again for the notes.
+struct NearTerms {
+    float2 cph, b1, b2, c9, cv, bv1, bv2, w9, ci, ib;
+};
+__device__ __forceinline__ NearTerms near_terms(const ColumnTerms& p, float c9p, float w9p, float ibp, const ColumnTerms& q,
+                                                float c9q, float w9q, float ibq) {
+    const float2 K = f2(SAR_TWO_PI, SAR_TWO_PI);
+    NearTerms t;
+    t.cph = mul2(f2(p.cph - rintf(p.cph), q.cph - rintf(q.cph)), K);
+    t.b1 = mul2(f2(p.b1 - rintf(p.b1), q.b1 - rintf(q.b1)), K);
+    t.b2 = mul2(f2(p.b2, q.b2), K);
+    t.c9 = mul2(f2(c9p, c9q), K);
+    t.cv = f2(p.cv, q.cv);
+    t.bv1 = f2(p.bv1, q.bv1);
+    t.bv2 = f2(p.bv2, q.bv2);
+    t.w9 = f2(w9p, w9q);
+    t.ci = f2(p.ci, q.ci);
+    t.ib = f2(ibp, ibq);
+    return t;
+}
+__device__ __forceinline__ float2 near_bins(const NearTerms& t, float2 d, float2* s) {   // shifter form
+    const float2 v = fma2(fma2(fma2(t.w9, d, t.bv2), d, t.bv1), d, t.cv);
+    const float2 r = add2(v, f2(SAR_SHIFTER, SAR_SHIFTER));
+    *s = fma2(add2(r, f2(-SAR_SHIFTER, -SAR_SHIFTER)), f2(-1.f, -1.f), v);
+    return add2(r, fma2(t.ib, d, t.ci));   // + the exact integer part
+}
+
+// Returns a mask of the contributions near a rounding boundary: bit 2 row + h for pulse h of the pair.
+template <int MODE, bool TWO, bool RING>
+__device__ __forceinline__ unsigned scatter_rows_near(const NearTerms& t, const float2* xrow, float2* wp, float2* wq,
+                                                      int off_p, int off_q, int ws, int lane) {
+    auto slot = [&](int i) { return wslot<RING>(RING ? ring_wrap(i, ws) : (int)min((unsigned)i, (unsigned)(ws - 2))); };
+    unsigned edge = 0;
+#pragma unroll 4
+    for (int rr = 0; rr < 16; ++rr) {
+        const float2 d = f2((float)(rr - 8), (float)(rr - 8));
+        const float2 xv = xrow[rr * kXtStride + lane];
+        const float2 XR = f2(xv.x, xv.x), XI = f2(xv.y, xv.y);
+        const float2 ph = fma2(fma2(fma2(t.c9, d, t.b2), d, t.b1), d, t.cph);
+        float2 s;
+        const float2 r = near_bins(t, d, &s);
+        edge |= (fabsf(s.x) > kNearEdge ? 1u : 0u) << (2 * rr);
+        if (TWO) edge |= (fabsf(s.y) > kNearEdge ? 2u : 0u) << (2 * rr);
+        float2 sn, cn;
+        __sincosf(ph.x, &sn.x, &cn.x);
+        __sincosf(ph.y, &sn.y, &cn.y);
+        const float2 xs = mul2(XI, sn);
+        const float2 cr = fma2(XR, cn, f2(-xs.x, -xs.y)), ci = fma2(XR, sn, mul2(XI, cn));
+        float2* a = wp + slot(__float_as_int(r.x) - SAR_SHIFTER_BITS + off_p);
+        float2* b = wq + slot(__float_as_int(r.y) - SAR_SHIFTER_BITS + off_q);
+        if (MODE >= 1) {
+            const float2 u = *a, v = TWO ? *b : f2(0.f, 0.f);
+            *a = add2(u, f2(cr.x, ci.x));
+            if (TWO) *b = add2(v, f2(cr.y, ci.y));
+            __syncwarp();
+        } else {
+            atomicAdd(&a->x, cr.x);
+            atomicAdd(&a->y, ci.x);
+            if (TWO) {
+                atomicAdd(&b->x, cr.y);
+                atomicAdd(&b->y, ci.y);
+            }
         }
-        __syncwarp();
     }
+    return edge;
 }
 
 // MODES 5, 4 and 3 (linear bins): the producer has shown that a sub-tile's bin is monotonic down
@@ -1146,42 +1136,49 @@ __device__ __forceinline__ int pair_mode(int a, int b) {
     return min(min(a, b), 1);
 }
 
+// Returns the mask of scatter_rows_near (nearest bins), else 0.
 template <bool LINEAR, bool PRECISE, bool TWO, typename XT, bool RING = false>
-__device__ __forceinline__ void scatter_half(int mode, const ColumnTerms& ctp, float c9p, float w9p, float ibp,
-                                             const ColumnTerms& ctq, float c9q, float w9q, float ibq,
-                                             const XT* xrow, float2* wp, float2* wq, int off_p, int off_q,
-                                             int ws, int lane, const NearCtx& nc) {
+__device__ __forceinline__ unsigned scatter_half(int mode, const ColumnTerms& ctp, float c9p, float w9p, float ibp,
+                                                 const ColumnTerms& ctq, float c9q, float w9q, float ibq,
+                                                 const XT* xrow, float2* wp, float2* wq, int off_p, int off_q,
+                                                 int ws, int lane) {
+    if constexpr (!LINEAR && PRECISE) {
+        const NearTerms t = near_terms(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq);
+        return mode >= 1 ? scatter_rows_near<1, TWO, RING>(t, xrow, wp, wq, off_p, off_q, ws, lane)
+                         : scatter_rows_near<0, TWO, RING>(t, xrow, wp, wq, off_p, off_q, ws, lane);
+    }
     if constexpr (LINEAR && !PRECISE && !RING) {
-        if (mode == 5) {
-            scatter_rows_runs<TWO, 16>(ctp, c9p, ctq, c9q, xrow, wp, wq, off_p, off_q, ws, lane);
-            return;
-        }
-        if (mode == 4) {
-            scatter_rows_runs<TWO, 8>(ctp, c9p, ctq, c9q, xrow, wp, wq, off_p, off_q, ws, lane);
-            return;
-        }
-        if (mode == 3) {
-            scatter_rows_runs<TWO, 4>(ctp, c9p, ctq, c9q, xrow, wp, wq, off_p, off_q, ws, lane);
-            return;
+        if (mode >= 3) {
+            if (mode == 5)
+                scatter_rows_runs<TWO, 16>(ctp, c9p, ctq, c9q, xrow, wp, wq, off_p, off_q, ws, lane);
+            else if (mode == 4)
+                scatter_rows_runs<TWO, 8>(ctp, c9p, ctq, c9q, xrow, wp, wq, off_p, off_q, ws, lane);
+            else
+                scatter_rows_runs<TWO, 4>(ctp, c9p, ctq, c9q, xrow, wp, wq, off_p, off_q, ws, lane);
+            return 0u;
         }
     }
-    if (mode >= 2)
-        scatter_rows<LINEAR, PRECISE, 2, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q, ws, lane,
-                                              nc);
-    else if (mode == 1)
-        scatter_rows<LINEAR, PRECISE, 1, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q, ws, lane,
-                                              nc);
-    else
-        scatter_rows<LINEAR, PRECISE, 0, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q, ws, lane,
-                                              nc);
+    if constexpr (LINEAR || !PRECISE) {
+        if (mode >= 2)
+            scatter_rows<LINEAR, PRECISE, 2, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
+                                                            ws, lane);
+        else if (mode == 1)
+            scatter_rows<LINEAR, PRECISE, 1, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
+                                                            ws, lane);
+        else
+            scatter_rows<LINEAR, PRECISE, 0, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
+                                                            ws, lane);
+    }
+    return 0u;
 }
 
 // Adds the window slots of bins [lo, hi] (absolute) of one pulse into its accumulator row and clears
-// them (ring windows: the bins a tile step leaves behind, and the last tile's at the end).
-__device__ __forceinline__ void ring_flush(float2* wp, int lo, int hi, int mask, const FpGridArgs& a, int s,
+// them (ring windows: the bins a tile step leaves behind, and the last tile's at the end).  The ring holds bins from
+// `first` on, bin `first` in slot `rot`.
+__device__ __forceinline__ void ring_flush(float2* wp, int lo, int hi, int first, int rot, const FpGridArgs& a, int s,
                                            int lane) {
     for (int bin = lo + lane; bin <= hi; bin += 32) {
-        float2* q = wp + wslot(bin & mask);
+        float2* q = wp + ring_wrap(bin - first + rot, a.ws);
         const float2 v = *q;
         if (v.x == 0.f && v.y == 0.f) continue;
         *q = make_float2(0.f, 0.f);
@@ -1198,12 +1195,12 @@ __device__ __forceinline__ void ring_flush(float2* wp, int lo, int hi, int mask,
 // its whole line of tiles and, between tiles, each warp adds and clears the bins its pulses leave
 // behind, so windows no longer bound the length of a strip (1-tile strips at upsample 128 otherwise).
 template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false>
-__global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(const FpGridArgs a) {
+__global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws_kernel(const FpGridArgs a) {
     extern __shared__ __align__(16) unsigned char fsm[];
-    const int pbf = a.pbf, ws = a.ws, wslots = window_slots(ws);
+    const int pbf = a.pbf, ws = a.ws, wslots = window_slots(ws, RING);
     constexpr bool WIDE_X = LINEAR && !PRECISE;
     using XT = typename std::conditional<WIDE_X, float4, float2>::type;
-    const FpWsLayout L = fp_ws_layout(ws, pbf, WIDE_X);
+    const FpWsLayout L = fp_ws_layout(ws, pbf, WIDE_X, RING, !LINEAR);
     float2* win = reinterpret_cast<float2*>(fsm + L.win);
     float4* coef0 = reinterpret_cast<float4*>(fsm + L.coef);
     XT* xt0 = reinterpret_cast<XT*>(fsm + L.xt);
@@ -1342,9 +1339,38 @@ __global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(co
     tt.di2 = di * di;
     tt.di3 = tt.di2 * di;
     bool ok = true;
-    // ring windows: the base bin of each of this warp's pulses (warp + 8 k) at the previous tile
-    const int mask = ws - 1, rh = a.ring_half;
+    // ring windows: the base bin of each of this warp's pulses (warp + 8 k) at the previous tile; wst holds the slot
+    // of bin base - rh
+    const int rh = a.ring_half;
     int prev_base[kMaxStagePulses / (kWsConsumers / 32)];
+    // near-boundary notes (nearest bins): the contribution's absolute FP32 bin; lane, row, half, pulse and tile
+    int2* queue = reinterpret_cast<int2*>(fsm + L.queue) + warp * kNearQueue;
+    int notes = 0;
+    auto settle = [&](int keep) {
+        while (notes > keep) {
+            const int n = min(32, notes);
+            notes -= n;
+            __syncwarp();   // the notes were written by other lanes
+            if (lane >= n) continue;
+            const int2 e = queue[notes + lane];
+            const int l = e.y & 31, rr = e.y >> 5 & 15, half = e.y >> 9 & 1, p = e.y >> 10 & 31, t = (int)((unsigned)e.y >> 15);
+            const int ti = TRANSPOSED ? t0 + t : line, tj = TRANSPOSED ? line : t0 + t;
+            const int pj = tj * kTile + (TRANSPOSED ? l : 16 * half + rr);
+            const int pi = ti * kTile + (TRANSPOSED ? 16 * half + rr : l) + g.a_off + g.shear * pj;
+            if (pi < 0 || pi >= g.img_nx || pj >= g.ny) continue;
+            const ExactSample x = exact_grid_sample<true>(a.steps, a.pulses, a.alpha2, g.kappa, g.s_r, a.bg0, BIN_FWD_NEAREST, pi, pj,
+                                                    k, s0 + p);
+            const int g32 = e.x - a.bg0;
+            if (x.gi == g32 || min(x.gi, g32) < 0 || max(x.gi, g32) >= a.Lg) continue;
+            const float2 xv = a.x[((size_t)k * g.ny + pj) * g.img_nx + pi];
+            float sn, cn;
+            __sincosf(SAR_TWO_PI * x.f, &sn, &cn);
+            const float cr = fmaf(xv.x, cn, -xv.y * sn), ci = fmaf(xv.x, sn, xv.y * cn);
+            float2* row = a.acc + (size_t)(s0 + p) * a.Lg;
+            atomicAdd(row + g32, make_float2(-cr, -ci));
+            atomicAdd(row + x.gi, make_float2(cr, ci));
+        }
+    };
     for (int t = 0; t < ntile; ++t) {
         const int b = t & 1;
         if (ok && !mbar_wait(&bars[b], (t >> 1) & 1, 32, 256)) ok = false;
@@ -1356,11 +1382,16 @@ __global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(co
                 if (p >= npb) break;
                 const int nb = base0[b * pbf + p];
                 if (t > 0 && nb != prev_base[k]) {
-                    const int ob = prev_base[k];
+                    const int ob = prev_base[k], rot = wst[p];
                     if (nb > ob)
-                        ring_flush(win + p * wslots, ob - rh, min(ob + rh, nb - rh - 1), mask, a, s0 + p, lane);
+                        ring_flush(win + p * wslots, ob - rh, min(ob + rh, nb - rh - 1), ob - rh, rot, a, s0 + p, lane);
                     else
-                        ring_flush(win + p * wslots, max(ob - rh, nb + rh + 1), ob + rh, mask, a, s0 + p, lane);
+                        ring_flush(win + p * wslots, max(ob - rh, nb + rh + 1), ob + rh, ob - rh, rot, a, s0 + p, lane);
+                    __syncwarp();
+                    if (lane == 0) {
+                        const int moved = (rot + (nb - ob)) % ws;
+                        wst[p] = moved < 0 ? moved + ws : moved;
+                    }
                 }
                 prev_base[k] = nb;
             }
@@ -1377,8 +1408,8 @@ __global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(co
                 const int pq = two ? p2 : p;
                 float2* wp = win + p * wslots;
                 float2* wq = win + pq * wslots;
-                const int off_p = base0[b * pbf + p] - wst[p];    // ring: the absolute base bin
-                const int off_q = base0[b * pbf + pq] - wst[pq];
+                const int off_p = RING ? wst[p] + rh : base0[b * pbf + p] - wst[p];
+                const int off_q = RING ? wst[pq] + rh : base0[b * pbf + pq] - wst[pq];
                 const int mode = two ? pair_mode(fast0[b * pbf + p], fast0[b * pbf + p2]) : fast0[b * pbf + p];
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
@@ -1390,31 +1421,29 @@ __global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(co
                     const ColumnTerms ctq =
                         load_column<PRECISE, TRANSPOSED>(coef + (pq * 4 + qs) * kSetF4, tt, c9q, w9q, ibq);
                     const XT* xrow = xt + 16 * half * kXtStride;
-                    NearCtx nc;
-                    if (!LINEAR) {
-                        nc.steps = a.steps;
-                        nc.pulses = a.pulses;
-                        nc.alpha2 = a.alpha2;
-                        nc.sr_hi = g.s_r.hi;
-                        nc.sr_lo = g.s_r.lo;
-                        nc.bg0 = a.bg0;
-                        nc.transposed = TRANSPOSED;
-                        nc.i0 = (TRANSPOSED ? t0 + t : line) * kTile + (TRANSPOSED ? 16 * half : 0);
-                        nc.j0 = (TRANSPOSED ? line : t0 + t) * kTile + (TRANSPOSED ? 0 : 16 * half);
-                        nc.k = k;
-                        nc.sp = s0 + p;
-                        nc.sq = s0 + pq;
-                        nc.wsp = wst[p];
-                        nc.wsq = wst[pq];
-                        nc.a_off = g.a_off;
-                        nc.shear = g.shear;
+                    const unsigned edge =
+                        two ? scatter_half<LINEAR, PRECISE, true, XT, RING>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow,
+                                                                            wp, wq, off_p, off_q, ws, lane)
+                            : scatter_half<LINEAR, PRECISE, false, XT, RING>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq,
+                                                                             xrow, wp, wq, off_p, off_q, ws, lane);
+                    if constexpr (!LINEAR && PRECISE) {
+                        unsigned left = edge;
+                        for (unsigned m; (m = __ballot_sync(0xffffffffu, left != 0u)) != 0u;) {   // one note per lane and turn
+                            if (left) {
+                                const int bit = __ffs(left) - 1, rr = bit >> 1, h = bit & 1;
+                                left &= left - 1u;
+                                const NearTerms nt = near_terms(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq);
+                                float2 sv;
+                                const float2 r = near_bins(nt, f2((float)(rr - 8), (float)(rr - 8)), &sv);
+                                const int n32 = __float_as_int(h ? r.y : r.x) - SAR_SHIFTER_BITS;
+                                const int ph = h ? pq : p;
+                                queue[notes + __popc(m & ((1u << lane) - 1u))] =
+                                    make_int2(base0[b * pbf + ph] + n32, lane | rr << 5 | half << 9 | ph << 10 | t << 15);
+                            }
+                            notes += __popc(m);
+                            if (notes >= 32) settle(31);
+                        }
                     }
-                    if (two)
-                        scatter_half<LINEAR, PRECISE, true, XT, RING>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq,
-                                                                      xrow, wp, wq, off_p, off_q, ws, lane, nc);
-                    else
-                        scatter_half<LINEAR, PRECISE, false, XT, RING>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq,
-                                                                       xrow, wp, wq, off_p, off_q, ws, lane, nc);
                 }
             }
         }
@@ -1425,20 +1454,21 @@ __global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(co
         if (lane == 0) raise_flag(a.flags, FLAG_WAIT_TIMEOUT);
         return;
     }
+    if (!LINEAR && PRECISE) settle(0);
     __syncwarp();
     if constexpr (RING) {   // the last tile's ranges
 #pragma unroll
         for (int k = 0; k < kMaxStagePulses / (kWsConsumers / 32); ++k) {
             const int p = warp + k * (kWsConsumers / 32);
             if (p >= npb) break;
-            ring_flush(win + p * wslots, prev_base[k] - rh, prev_base[k] + rh, mask, a, s0 + p, lane);
+            ring_flush(win + p * wslots, prev_base[k] - rh, prev_base[k] + rh, prev_base[k] - rh, wst[p], a, s0 + p, lane);
         }
     } else {
         // merge this warp's windows into the global accumulator
         for (int p = warp; p < npb; p += kWsConsumers / 32) {
             const float2* wp = win + p * wslots;
             for (int w = lane; w < ws; w += 32) {
-                const float2 v = wp[wslot(w)];
+                const float2 v = wp[wslot<false>(w)];
                 if (v.x == 0.f && v.y == 0.f) continue;
                 const long gi = (long)wst[p] + w - a.bg0;
                 if (gi < 0 || gi >= a.Lg) {
@@ -1454,7 +1484,7 @@ __global__ void __launch_bounds__(kWsThreads, RING ? 1 : 2) fp_grid_ws_kernel(co
 
 template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false>
 static cudaError_t launch_fp_grid_ws_t(const FpGridArgs& a, cudaStream_t st) {
-    const size_t smem = fp_grid_ws_smem_bytes(a.ws, a.pbf, LINEAR && !PRECISE);
+    const size_t smem = fp_grid_ws_smem_bytes(a.ws, a.pbf, LINEAR && !PRECISE, RING, !LINEAR);
     const int lines = TRANSPOSED ? a.g.tiles_y : a.g.tiles_x;
     const dim3 grid((unsigned)(a.segs_per_column * lines * a.g.nz), (unsigned)((a.S + a.pbf - 1) / a.pbf));
     cudaError_t e = cudaFuncSetAttribute(fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING>,
@@ -1478,8 +1508,8 @@ static cudaError_t launch_fp_grid_ws_o(const FpGridArgs& a, cudaStream_t st) {
 
 cudaError_t launch_fp_grid_ws(const FpGridArgs& a, cudaStream_t st) {
     if (a.pbf < 8 || a.pbf > 32 || (a.pbf & 7) || a.ws < 32 || (a.ws & 31)) return cudaErrorInvalidValue;
-    // ring windows: split bins, a power-of-two ring holding a tile's whole range
-    if (a.ring_half > 0 && (!a.g.precise_bins || (a.ws & (a.ws - 1)) || 2 * a.ring_half + 1 > a.ws))
+    // ring windows: split bins, a ring holding a tile's whole range
+    if (a.ring_half > 0 && (!a.g.precise_bins || 2 * a.ring_half + 1 > a.ws))
         return cudaErrorInvalidValue;
     if (!a.linear && a.g.precise_bins && (!a.steps || !a.alpha2)) return cudaErrorInvalidValue;
     return a.transposed ? launch_fp_grid_ws_o<true>(a, st) : launch_fp_grid_ws_o<false>(a, st);

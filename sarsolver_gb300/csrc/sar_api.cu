@@ -549,11 +549,15 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
                 }
             }
         }
-        // Linear sampling with plain bins: the gather along iso-range lines (sar_gather.cu); the tile gather above
-        // serves the other plans.  Its tiles hold image pixels, so a tile's mean bin lies at most half a window
+        // The gather along iso-range lines (sar_gather.cu); the tile gather above serves the plans that have no layout
+        // for it (windows that do not fit shared memory, antennas within the scene).  Its tiles hold image pixels, so a tile's mean bin lies at most half a window
         // outside the image's range: margins of two windows.
-        if (p->interp == SAR_INTERP_LINEAR && !p->gc_adj.precise_bins)
-            p->gather = gather_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+        {
+            const int bins = p->interp == SAR_INTERP_NEAREST_REF ? GATHER_NEAREST
+                             : p->gc_fwd.precise_bins            ? GATHER_LINEAR
+                                                                 : GATHER_RUNS;
+            p->gather = gather_layout(bins, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+        }
         if (p->gather.ok) {
             const Lattice& L = p->gather.lattice;
             double ea[3], eb[3];
@@ -563,6 +567,7 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             }
             p->gc_adj_image = make_grid_const(ex, ey, ez, kappa, s_r, adjoint_bin_offset(p->interp), nx, ny, nz);
             p->gc_gather = make_grid_const(ea, eb, ez, kappa, s_r, adjoint_bin_offset(p->interp), nx, ny, nz);
+            p->gc_gather.precise_bins = p->gather.bins != GATHER_RUNS;
             span_ww = std::max(span_ww, 2 * p->gather.ww + 8);
         }
         p->bg0 = (long)std::floor(vmin) - span_ww / 2 - 4;
@@ -1185,6 +1190,9 @@ static int gather_pulses(sar_plan* p, const float4* pairs, size_t first, size_t 
         a.partial = p->d_partial;
         a.tiles = p->d_tiles;
         a.flags = p->d_flags;
+        a.bins = L.bins;
+        a.steps = p->d_steps;
+        a.alpha2 = p->d_alpha2 ? p->d_alpha2 + first : nullptr;
         a.num_tiles = (int)L.tiles.size();
         a.S = (int)count;
         a.Lg = p->Lg;
@@ -1192,6 +1200,7 @@ static int gather_pulses(sar_plan* p, const float4* pairs, size_t first, size_t 
         a.ww = L.ww;
         a.pb = L.pb;
         a.warps = L.warps;
+        a.across = L.across;
         a.parts = gather_parts(L, count, p->P);
         a.accumulate = accumulate ? 1 : 0;
         a.vx = L.lattice.vx;

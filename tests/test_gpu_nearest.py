@@ -1,4 +1,5 @@
-"""Nearest-bin sampling on the grid kernels against the per-pixel path, which decides every bin exactly: narrow and
+"""Nearest-bin sampling on the grid kernels (and linear sampling with bins split into integer and fraction, which
+shares the gather) against the per-pixel path, which decides every bin exactly: narrow and
 wide windows (upsample 8 and 128), looks along the grid axes and between them, ragged images and pulse counts, several
 planes, bistatic pulses, short range, and geometries that put every sample within 5e-5 bins of a rounding boundary
 (every note of the exact re-decision queues taken, and overflowing).  Tolerance: the operator's own, 1e-5 relative
@@ -20,9 +21,9 @@ def cuda_required():
         pytest.skip("no CUDA device")
 
 
-def check(case, upsample, rng):
-    plan = SarPlan(case.scene, case.aperture, upsample_ratio=upsample, interp="nearest_ref", path="grid")
-    general = SarPlan(case.scene, case.aperture, upsample_ratio=upsample, interp="nearest_ref", path="points")
+def check(case, upsample, rng, interp="nearest_ref"):
+    plan = SarPlan(case.scene, case.aperture, upsample_ratio=upsample, interp=interp, path="grid")
+    general = SarPlan(case.scene, case.aperture, upsample_ratio=upsample, interp=interp, path="points")
     x = crandn(rng, case.scene.num_scatterers)
     y = crandn(rng, case.aperture.num_slow_times, case.aperture.num_freqs)
     x, y = torch.from_numpy(x), torch.from_numpy(y)
@@ -31,22 +32,24 @@ def check(case, upsample, rng):
     assert plan.device_flags() == 0
 
 
-@pytest.mark.parametrize("upsample", [8.0, 128.0])
+@pytest.mark.parametrize("interp,upsample", [("nearest_ref", 8.0), ("nearest_ref", 128.0), ("linear", 64.0)])
 @pytest.mark.parametrize("az,shape,spacing,pulses,degrees,bistatic,radius", [
     (0.0, (1, 33, 97), 0.25, 33, 3.0, False, 10.0e3), (90.0, (1, 97, 33), 0.25, 31, 3.0, False, 10.0e3),
     (45.0, (1, 70, 70), 0.25, 40, 2.0, False, 10.0e3), (63.0, (1, 100, 177), 0.25, 129, 2.0, False, 10.0e3),
     (153.0, (2, 31, 98), 0.25, 64, 2.0, False, 10.0e3), (14.0, (1, 84, 74), 0.3, 50, 4.0, True, 10.0e3),
     (20.0, (1, 1, 200), 0.5, 5, 1.0, False, 10.0e3), (70.0, (3, 66, 1), 0.5, 1, 1.0, False, 10.0e3),
     (33.0, (1, 70, 80), 0.9, 20, 3.0, False, 10.0e3), (10.0, (1, 78, 88), 0.25, 40, 60.0, False, 2.0e3),
-    (0.0, (1, 150, 140), 0.3, 530, 3.0, False, 10.0e3)])
-def test_nearest_matches_oracle(az, shape, spacing, pulses, degrees, bistatic, radius, upsample):
+    (0.0, (1, 150, 140), 0.3, 530, 3.0, False, 10.0e3),
+    (33.0, (1, 260, 140), 0.3, 37, 3.0, False, 10.0e3), (60.0, (1, 140, 290), 0.5, 21, 3.0, True, 10.0e3),   # wide windows
+    (5.0, (1, 300, 40), 0.15, 90, 2.0, False, 10.0e3)])
+def test_grid_matches_points(az, shape, spacing, pulses, degrees, bistatic, radius, interp, upsample):
     rng = np.random.default_rng(int(az) + pulses)
     tx = spotlight(pulses, degrees, radius, 0.5 * radius, az)
     rx = spotlight(pulses, 0.5 * degrees, 0.8 * radius, 0.3 * radius, az + 20.0) if bistatic else tx.copy()
     ap = NumpySimpleSarAperture(tx, rx, np.zeros((pulses, 3)), 10.0e9, 200.0e6, num_freqs=512,
                                 slow_time_weighting=np.exp(1j * rng.uniform(-3, 3, pulses)))
     dims = [2.0 * (shape[0] - 1), spacing * (shape[1] - 1), spacing * (shape[2] - 1)]
-    check(Case(GridSarScene(list(shape), dims), ap, upsample, {}), upsample, rng)
+    check(Case(GridSarScene(list(shape), dims), ap, upsample, {}), upsample, rng, interp)
 
 
 @pytest.mark.parametrize("upsample,step", [(8.0, 1), (8.0, 3), (128.0, 16), (128.0, 37)])

@@ -220,8 +220,9 @@ int conv_forward(Src s0, Src s1, int images, int H, int W, int taps, const bf16*
     return SAR_OK;
 }
 
-// dw[Cout][taps * Ctot] += sum_pixels dz[p][co] * (x0 ++ x1)[p + tap][ci]  (FP32 accumulate).
-int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int W, int taps, float* dw,
+// dw[Cout][taps * Ctot] += sum_pixels dz[p][co] * (x0 ++ x1)[p + tap][ci]  (FP32 accumulate), and, where db is given,
+// db[co] += sum_pixels dz[p][co].
+int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int W, int taps, float* dw, float* db,
                unsigned* flags, cudaStream_t st) {
     using namespace unet;
     const int nsrc = s1.p ? 2 : 1;
@@ -265,6 +266,7 @@ int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int 
     const int stage = 128 * 128 * 2 + BN * 128 * 2;
     a.stages = std::max(2, std::min(6, (kSmemBudget - 2048) / stage));
     a.dw = dw;
+    a.db = db;
     a.flags = flags;
     const size_t smem = 1024 + (size_t)a.stages * stage + (2 * a.stages + 2) * 8 + 16;
     dim3 grid((unsigned)splits, (unsigned)mtiles, (unsigned)ntiles);
@@ -300,103 +302,104 @@ __global__ void prep_input_kernel(const float2* __restrict__ z, float scale, bf1
     }
 }
 
+// The kernels below move eight channels (16 bytes) a thread; widths and channel counts are powers of two, so a vector's
+// place is found with shifts.  (With two channels a thread and divisions they ran at a third of the memory rate.)
+struct Vec8 {
+    uint4 q;
+    __device__ __forceinline__ float2 get(int i) const {
+        return __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&q)[i]);
+    }
+    __device__ __forceinline__ void set(int i, float x, float y) {
+        reinterpret_cast<__nv_bfloat162*>(&q)[i] = __floats2bfloat162_rn(x, y);
+    }
+};
+__device__ __forceinline__ Vec8 vec8(const bf16* p, size_t i) { return Vec8{__ldg(reinterpret_cast<const uint4*>(p) + i)}; }
+
+// Vector i of an image [n][h][1 << lw][8 << lc]: column, row of the whole batch, channel vector.
+struct Place {
+    int c, x;
+    size_t y;
+};
+__device__ __forceinline__ Place place(size_t i, int lw, int lc) {
+    return Place{(int)(i & ((1u << lc) - 1)), (int)((i >> lc) & ((1u << lw) - 1)), i >> (lc + lw)};
+}
+// Vector of the pixel (x, y) of an image twice as wide and high.
+__device__ __forceinline__ size_t fine(const Place& p, int lw, int lc) {
+    return (((2 * p.y) << (lw + 1)) + 2 * p.x << lc) + p.c;
+}
+
 // 2x2 average pool, NHWC: in [n][2h][2w][C] -> out [n][h][w][C].
-__global__ void avgpool_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int images, int H, int W, int C) {
-    const int h = H / 2, w = W / 2, cv = C / 2;
-    const size_t total = (size_t)images * h * w * cv;
+__global__ void avgpool_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, size_t total, int lw, int lc) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int c2 = (int)(i % cv);
-        size_t r = i / cv;
-        const int x = (int)(r % w);
-        r /= w;
-        const int y = (int)(r % h);
-        const size_t n = r / h;
-        const __nv_bfloat162* src = reinterpret_cast<const __nv_bfloat162*>(in);
-        const size_t b = ((n * H + 2 * y) * W + 2 * x) * cv + c2;
-        const float2 a = __bfloat1622float2(src[b]), bb = __bfloat1622float2(src[b + cv]);
-        const float2 c = __bfloat1622float2(src[b + (size_t)W * cv]), d = __bfloat1622float2(src[b + (size_t)W * cv + cv]);
-        reinterpret_cast<__nv_bfloat162*>(out)[i] =
-            __floats2bfloat162_rn(0.25f * (a.x + bb.x + c.x + d.x), 0.25f * (a.y + bb.y + c.y + d.y));
+        const size_t b = fine(place(i, lw, lc), lw, lc), right = (size_t)1 << lc, down = (size_t)2 << (lw + lc);
+        const Vec8 va = vec8(in, b), vb = vec8(in, b + right), vc = vec8(in, b + down), vd = vec8(in, b + down + right);
+        Vec8 o;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 p = va.get(k), q = vb.get(k), r = vc.get(k), s = vd.get(k);
+            o.set(k, 0.25f * (p.x + q.x + r.x + s.x), 0.25f * (p.y + q.y + r.y + s.y));
+        }
+        reinterpret_cast<uint4*>(out)[i] = o.q;
     }
 }
 
-// Nearest 2x upsample, NHWC: in [n][h][w][C] -> out [n][2h][2w][C].
-__global__ void upsample_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int images, int h, int w, int C) {
-    const int cv = C / 8;   // 16-byte vectors
-    const size_t total = (size_t)images * 4 * h * w * cv;
+// Nearest 2x upsample, NHWC: in [n][h][w][C] -> out [n][2h][2w][C]; a thread per input vector.
+__global__ void upsample_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, size_t total, int lw, int lc) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % cv);
-        size_t r = i / cv;
-        const int X = (int)(r % (2 * w));
-        r /= 2 * w;
-        const int Y = (int)(r % (2 * h));
-        const size_t n = r / (2 * h);
-        reinterpret_cast<uint4*>(out)[i] = reinterpret_cast<const uint4*>(in)[((n * h + Y / 2) * w + X / 2) * cv + c];
+        const size_t b = fine(place(i, lw, lc), lw, lc), right = (size_t)1 << lc, down = (size_t)2 << (lw + lc);
+        const Vec8 v = vec8(in, i);
+        uint4* o = reinterpret_cast<uint4*>(out);
+        o[b] = v.q;
+        o[b + right] = v.q;
+        o[b + down] = v.q;
+        o[b + down + right] = v.q;
     }
 }
 
 // Backward of the nearest upsample followed by the ReLU mask of its input:
 // out[n][y][x][c] = (sum of g over the 2x2 children) * (act[n][y][x][c] > 0).
 __global__ void upsample_bwd_mask_kernel(const bf16* __restrict__ g, const bf16* __restrict__ act, bf16* __restrict__ out,
-                                         int images, int h, int w, int C) {
-    const int cv = C / 2;
-    const size_t total = (size_t)images * h * w * cv;
-    const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(g);
+                                         size_t total, int lw, int lc) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int c2 = (int)(i % cv);
-        size_t r = i / cv;
-        const int x = (int)(r % w);
-        r /= w;
-        const int y = (int)(r % h);
-        const size_t n = r / h;
-        const size_t W2 = 2 * (size_t)w;
-        const size_t b = ((n * 2 * h + 2 * y) * W2 + 2 * x) * cv + c2;
-        const float2 a = __bfloat1622float2(g2[b]), bb = __bfloat1622float2(g2[b + cv]);
-        const float2 c = __bfloat1622float2(g2[b + W2 * cv]), d = __bfloat1622float2(g2[b + W2 * cv + cv]);
-        const float2 m = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(act)[i]);
-        const float sx = m.x > 0.f ? a.x + bb.x + c.x + d.x : 0.f;
-        const float sy = m.y > 0.f ? a.y + bb.y + c.y + d.y : 0.f;
-        reinterpret_cast<__nv_bfloat162*>(out)[i] = __floats2bfloat162_rn(sx, sy);
+        const size_t b = fine(place(i, lw, lc), lw, lc), right = (size_t)1 << lc, down = (size_t)2 << (lw + lc);
+        const Vec8 va = vec8(g, b), vb = vec8(g, b + right), vc = vec8(g, b + down), vd = vec8(g, b + down + right);
+        const Vec8 vm = vec8(act, i);
+        Vec8 o;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 p = va.get(k), q = vb.get(k), r = vc.get(k), s = vd.get(k), m = vm.get(k);
+            o.set(k, m.x > 0.f ? p.x + q.x + r.x + s.x : 0.f, m.y > 0.f ? p.y + q.y + r.y + s.y : 0.f);
+        }
+        reinterpret_cast<uint4*>(out)[i] = o.q;
     }
 }
 
 // Gradient of an encoder output that feeds both a skip connection and a 2x2 average pool:
-// out = (g_skip + g_pool[parent] / 4) * (act > 0), all [n][H][W][C] except g_pool [n][H/2][W/2][C].
+// out = (g_skip + g_pool[parent] / 4) * (act > 0), all [n][2h][2w][C] except g_pool [n][h][w][C]; a thread per
+// vector of g_pool.
 __global__ void pool_bwd_add_mask_kernel(const bf16* __restrict__ gpool, const bf16* __restrict__ gskip,
-                                         const bf16* __restrict__ act, bf16* __restrict__ out, int images, int H, int W,
-                                         int C) {
-    const int cv = C / 2;
-    const size_t total = (size_t)images * H * W * cv;
+                                         const bf16* __restrict__ act, bf16* __restrict__ out, size_t total, int lw,
+                                         int lc) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int c2 = (int)(i % cv);
-        size_t r = i / cv;
-        const int x = (int)(r % W);
-        r /= W;
-        const int y = (int)(r % H);
-        const size_t n = r / H;
-        const float2 gp = __bfloat1622float2(
-            reinterpret_cast<const __nv_bfloat162*>(gpool)[((n * (H / 2) + y / 2) * (W / 2) + x / 2) * cv + c2]);
-        const float2 gs = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(gskip)[i]);
-        const float2 m = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(act)[i]);
-        reinterpret_cast<__nv_bfloat162*>(out)[i] =
-            __floats2bfloat162_rn(m.x > 0.f ? gs.x + 0.25f * gp.x : 0.f, m.y > 0.f ? gs.y + 0.25f * gp.y : 0.f);
-    }
-}
-
-// db[c] += sum_p dz[p][c].  256 threads = (256 / C) pixel lanes x C channels (C divides 256),
-// grid-stride over pixels with coalesced rows, a shared-memory sum over the pixel lanes and one
-// atomic per channel per CTA.
-__global__ void bias_grad_kernel(const bf16* __restrict__ dz, size_t P, int C, float* __restrict__ db) {
-    __shared__ float part[256];
-    const int lanes = blockDim.x / C, c = threadIdx.x % C, pl = threadIdx.x / C;
-    float acc = 0.f;
-    for (size_t p = (size_t)blockIdx.x * lanes + pl; p < P; p += (size_t)gridDim.x * lanes) acc += bf(dz[p * C + c]);
-    part[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x < C) {
-        float sum = 0.f;
-        for (int l = 0; l < lanes; ++l) sum += part[l * C + threadIdx.x];
-        atomicAdd(db + threadIdx.x, sum);
+        const size_t b = fine(place(i, lw, lc), lw, lc);
+        const Vec8 vp = vec8(gpool, i);
+        Vec8 vs[4], vm[4];
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+            const size_t j = b + ((size_t)(ch & 1) << lc) + ((size_t)(ch & 2) << (lw + lc));
+            vs[ch] = vec8(gskip, j);
+            vm[ch] = vec8(act, j);
+        }
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+            Vec8 o;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 gp = vp.get(k), gs = vs[ch].get(k), m = vm[ch].get(k);
+                o.set(k, m.x > 0.f ? gs.x + 0.25f * gp.x : 0.f, m.y > 0.f ? gs.y + 0.25f * gp.y : 0.f);
+            }
+            reinterpret_cast<uint4*>(out)[b + ((size_t)(ch & 1) << lc) + ((size_t)(ch & 2) << (lw + lc))] = o.q;
+        }
     }
 }
 
@@ -424,6 +427,12 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
         v[i] = vi;
         p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
     }
+}
+
+int log2i(int n) {   // n a power of two
+    int l = 0;
+    while ((1 << l) < n) ++l;
+    return l;
 }
 
 unsigned ew_grid(size_t n) {
@@ -543,12 +552,8 @@ int layer_backward(sar_unet* n, int i, cudaStream_t st) {
     Src s0, s1;
     n->inputs(i, &s0, &s1);
     const int h = n->H >> l.level, w = n->W >> l.level;
-    const size_t P = n->pixels(l.level);
-    U_CALL(conv_wgrad(s0, s1, n->dz[i], l.cout, n->B, h, w, l.taps, n->grads + n->w_off[i], n->flags, st));
-    const size_t lanes = 256 / l.cout;
-    bias_grad_kernel<<<(unsigned)std::max<size_t>(1, std::min<size_t>((size_t)device_sms() * 4, P / (lanes * 16))), 256,
-                       0, st>>>(n->dz[i], P, l.cout, n->grads + n->b_off[i]);
-    U_CUDA(cudaGetLastError(), "bias gradient");
+    U_CALL(conv_wgrad(s0, s1, n->dz[i], l.cout, n->B, h, w, l.taps, n->grads + n->w_off[i],
+                      n->grads + n->b_off[i], n->flags, st));
     if (i == 0) return SAR_OK;
     Dst d0, d1;
     switch (i) {
@@ -574,16 +579,16 @@ int do_forward(sar_unet* n, const float2* in, float scale, float* out, cudaStrea
         U_CALL(layer_forward(n, i0, nullptr, st));
         U_CALL(layer_forward(n, i0 + 1, nullptr, st));
         if (lvl < 3) {
-            const size_t np = n->pixels(lvl + 1) * (size_t)(n->c << lvl) / 2;
-            avgpool_kernel<<<ew_grid(np), 256, 0, st>>>(n->a[i0 + 1], n->p[lvl], n->B, n->H >> lvl, n->W >> lvl,
-                                                        n->c << lvl);
+            const size_t np = n->pixels(lvl + 1) * (size_t)(n->c << lvl) / 8;
+            avgpool_kernel<<<ew_grid(np), 256, 0, st>>>(n->a[i0 + 1], n->p[lvl], np, log2i(n->W >> (lvl + 1)),
+                                                        log2i((n->c << lvl) / 8));
         }
     }
     for (int lvl = 2; lvl >= 0; --lvl) {
         const int src = lvl == 2 ? 7 : (lvl == 1 ? 9 : 11);   // decoder input from the level below
         const int C = n->L[src].cout;
-        const size_t nu = n->pixels(lvl) * (size_t)C / 8;
-        upsample_kernel<<<ew_grid(nu), 256, 0, st>>>(n->a[src], n->u[lvl], n->B, n->H >> (lvl + 1), n->W >> (lvl + 1), C);
+        const size_t nu = n->pixels(lvl + 1) * (size_t)C / 8;
+        upsample_kernel<<<ew_grid(nu), 256, 0, st>>>(n->a[src], n->u[lvl], nu, log2i(n->W >> (lvl + 1)), log2i(C / 8));
         const int i0 = lvl == 2 ? 8 : (lvl == 1 ? 10 : 12);
         U_CALL(layer_forward(n, i0, nullptr, st));
         U_CALL(layer_forward(n, i0 + 1, nullptr, st));
@@ -605,9 +610,9 @@ int do_backward(sar_unet* n, const float2* gout, cudaStream_t st) {
         U_CALL(layer_backward(n, cat, st));    // -> du[lvl], de[lvl]
         const int below = cat - 1;             // 11, 9, 7: output upsampled into this level
         const int C = n->L[below].cout;
-        const size_t nb = n->pixels(lvl + 1) * (size_t)C / 2;
-        upsample_bwd_mask_kernel<<<ew_grid(nb), 256, 0, st>>>(n->du[lvl], n->a[below], n->dz[below], n->B,
-                                                              n->H >> (lvl + 1), n->W >> (lvl + 1), C);
+        const size_t nb = n->pixels(lvl + 1) * (size_t)C / 8;
+        upsample_bwd_mask_kernel<<<ew_grid(nb), 256, 0, st>>>(n->du[lvl], n->a[below], n->dz[below], nb,
+                                                              log2i(n->W >> (lvl + 1)), log2i(C / 8));
     }
     U_CALL(layer_backward(n, 7, st));          // bottleneck -> dz[6]
     // Encoder, bottom level first: first conv of level lvl -> dp[lvl-1]; pooled + skip gradients
@@ -617,9 +622,9 @@ int do_backward(sar_unet* n, const float2* gout, cudaStream_t st) {
         U_CALL(layer_backward(n, first, st));  // -> dp[lvl - 1]
         const int enc = first - 1;             // 5, 3, 1
         const int C = n->L[enc].cout;
-        const size_t ne = n->pixels(lvl - 1) * (size_t)C / 2;
-        pool_bwd_add_mask_kernel<<<ew_grid(ne), 256, 0, st>>>(n->dp[lvl - 1], n->de[lvl - 1], n->a[enc], n->dz[enc], n->B,
-                                                              n->H >> (lvl - 1), n->W >> (lvl - 1), C);
+        const size_t ne = n->pixels(lvl) * (size_t)C / 8;
+        pool_bwd_add_mask_kernel<<<ew_grid(ne), 256, 0, st>>>(n->dp[lvl - 1], n->de[lvl - 1], n->a[enc], n->dz[enc], ne,
+                                                              log2i(n->W >> lvl), log2i(C / 8));
         U_CALL(layer_backward(n, enc, st));    // -> dz[enc - 1]
     }
     U_CALL(layer_backward(n, 0, st));
@@ -822,7 +827,7 @@ int sar_conv2d_wgrad_bf16(const void* x0, int c0, const void* x1, int c1, const 
                           int width, int taps, float* dw, unsigned* flags_dev, void* stream) {
     if (!x0 || !dz || !dw || !flags_dev) return fail(SAR_ERR_INVALID_ARGUMENT, "null argument");
     return conv_wgrad(Src{(const bf16*)x0, c0}, Src{(const bf16*)x1, x1 ? c1 : 0}, (const bf16*)dz, cout, batch, height,
-                      width, taps, dw, flags_dev, (cudaStream_t)stream);
+                      width, taps, dw, nullptr, flags_dev, (cudaStream_t)stream);
 }
 
 }  // extern "C"

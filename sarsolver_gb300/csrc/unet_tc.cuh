@@ -76,6 +76,26 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, unsigned 
     }
 }
 
+// Position in a ring of stages: slot and times round it, counted up (64-bit divisions by the number of stages took
+// longer than a stage's loads).
+struct Ring {
+    int s = 0;
+    unsigned round = 0;
+    __device__ __forceinline__ void next(int stages) {
+        if (++s == stages) {
+            s = 0;
+            ++round;
+        }
+    }
+};
+// Every load issued into the ring (`full` barriers) has landed: before the CTA may exit.
+__device__ __forceinline__ void drain(const Ring& r, uint64_t* full, int stages, unsigned* flags) {
+    for (int s = 0; s < stages; ++s) {
+        const unsigned rounds = r.round + (s < r.s ? 1u : 0u);
+        if (rounds > 0 && !bar_wait(&full[s], (rounds - 1) & 1, 256)) atomicOr(flags, kFlagTimeout);
+    }
+}
+
 __device__ __forceinline__ void tma_prefetch(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
@@ -279,37 +299,41 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
         tma_prefetch(&maps.src[0]);
         if (a.nsrc > 1) tma_prefetch(&maps.src[1]);
         tma_prefetch(&maps.wts);
-        long long g = 0;
+        Ring r;
         bool stop = false;
         for (int it = blockIdx.x; it < items && !stop; it += gridDim.x) {
             const int mt = it / ntn, n0 = (it % ntn) * a.BN;
             const int img = mt / per_img, rem = mt % per_img;
             const int x0 = (rem % a.tiles_x) * a.BW, y0 = (rem / a.tiles_x) * a.BH;
-            for (int kb = 0; kb < nkb; ++kb, ++g) {
-                const int s = (int)(g % a.stages);
-                const long long round = g / a.stages;
-                if (g >= a.stages && !bar_wait(&empty[s], (uint32_t)((round - 1) & 1), 256)) {
+            int c = 0, dy = a.taps == 9 ? -1 : 0, dx = dy;
+            for (int kb = 0; kb < nkb; ++kb) {
+                if (r.round > 0 && !bar_wait(&empty[r.s], (uint32_t)((r.round - 1) & 1), 256)) {
                     atomicOr(a.flags, kFlagTimeout);
                     timed_out = 1;
                     stop = true;
                     break;
                 }
-                const int tap = kb / kpt, c = (kb % kpt) * BK;
                 const int src = c >= a.C0 ? 1 : 0, cs = src ? c - a.C0 : c;
-                const int dy = a.taps == 9 ? tap / 3 - 1 : 0, dx = a.taps == 9 ? tap % 3 - 1 : 0;
-                uint8_t* st = smem + s * stage_bytes;
-                bar_expect_tx(&full[s], (uint32_t)stage_bytes);
-                tma_4d(st, &maps.src[src], cs, x0 + dx, y0 + dy, img, &full[s]);
-                tma_2d(st + a_bytes, &maps.wts, tap * a.Ctot + c, n0, &full[s]);
+                uint8_t* st = smem + r.s * stage_bytes;
+                bar_expect_tx(&full[r.s], (uint32_t)stage_bytes);
+                tma_4d(st, &maps.src[src], cs, x0 + dx, y0 + dy, img, &full[r.s]);
+                tma_2d(st + a_bytes, &maps.wts, kb * BK, n0, &full[r.s]);
+                r.next(a.stages);
+                c += BK;
+                if (c == a.Ctot) {
+                    c = 0;
+                    if (++dx > 1) {
+                        dx = -1;
+                        ++dy;
+                    }
+                }
             }
         }
-        // Drain: every issued load has landed before the CTA may exit.
-        for (long long k = (g > a.stages ? g - a.stages : 0); k < g; ++k)
-            if (!bar_wait(&full[k % a.stages], (uint32_t)((k / a.stages) & 1), 256)) atomicOr(a.flags, kFlagTimeout);
+        drain(r, full, a.stages, a.flags);
     } else if (warp == 1 && lane == 0) {
         const uint32_t idesc = idesc_bf16(128, a.BN, false, false);
         const uint32_t lay = swizzle_layout(BK * 2), sbo = 8 * BK * 2;
-        long long g = 0;
+        Ring r;
         int i = 0;
         bool stop = false;
         for (int it = blockIdx.x; it < items && !stop; it += gridDim.x, ++i) {
@@ -321,9 +345,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
             }
             tc_after();
             const uint32_t tacc = tmem + (uint32_t)(b * ncols);
-            for (int kb = 0; kb < nkb; ++kb, ++g) {
-                const int s = (int)(g % a.stages);
-                if (!bar_wait(&full[s], (uint32_t)((g / a.stages) & 1), 64)) {
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int s = r.s;
+                if (!bar_wait(&full[s], (uint32_t)(r.round & 1), 64)) {
                     atomicOr(a.flags, kFlagTimeout);
                     timed_out = 1;
                     stop = true;
@@ -336,6 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
                     mma_bf16(tacc, smem_desc(sa + 32 * k, 16, sbo, lay), smem_desc(sb + 32 * k, 16, sbo, lay), idesc,
                              (kb | k) != 0);
                 mma_commit(&empty[s]);
+                r.next(a.stages);
             }
             mma_commit(&tfull[b]);   // also on the timeout path, so the epilogue warps are released
         }
@@ -380,8 +405,60 @@ struct WgradArgs {
     int num_tiles, tiles_per_split;
     int BN, stages;
     float* dw;   // FP32 [Cout][taps * Ctot], accumulated
+    float* db;   // FP32 [Cout], accumulated, or null
     unsigned* flags;
 };
+
+// The bias gradient, db[n] += sum of dZ over this CTA's share of its pixels (the K blocks are dealt out to the CTAs
+// that read them, gridDim.y), by the four warps that otherwise wait for the accumulator: FP32 sums of the staged dZ
+// boxes, a pair of channels per thread.  Read again by a kernel of its own, dZ took 9 us a layer and a launch.
+template <int COB>
+__device__ __forceinline__ void sum_dz(const WgradArgs& a, const uint8_t* dz0, int stage_bytes, uint64_t* full,
+                                       uint64_t* empty, int nkb, int n0, float* bsum) {
+    constexpr int WORDS = COB / 2, LANES = 128 / WORDS;   // channel pairs of a row, rows read at a time
+    const int t = threadIdx.x - 64, word = t % WORDS, row0 = t / WORDS, lane = threadIdx.x & 31;
+    const int boxes = a.BN / COB;
+    float2 sum[4] = {};   // BN <= 128
+    for (int i = t; i < a.BN; i += 128) bsum[i] = 0.f;
+    Ring r;
+    bool ok = true;
+    int turn = blockIdx.y;   // K blocks until this CTA's next
+    for (int kb = 0; kb < nkb; ++kb, r.next(a.stages)) {
+        if (!__all_sync(0xffffffffu, bar_wait(&full[r.s], r.round & 1, 256))) {
+            ok = false;
+            break;
+        }
+        if (turn == 0) {
+            turn = gridDim.y;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j >= boxes) break;
+                const uint8_t* box = dz0 + r.s * stage_bytes + j * 128 * COB * 2;
+#pragma unroll 8
+                for (int p = row0; p < 128; p += LANES) {
+                    const int chunk = (word >> 2) ^ (COB == 64 ? p & 7 : (p >> 1) & 3);   // the copy's swizzle
+                    const float2 v = __bfloat1622float2(
+                        *reinterpret_cast<const __nv_bfloat162*>(box + p * COB * 2 + chunk * 16 + (word & 3) * 4));
+                    sum[j].x += v.x;
+                    sum[j].y += v.y;
+                }
+            }
+        }
+        --turn;
+        __syncwarp();
+        if (lane == 0) bar_try_arrive(&empty[r.s]);
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j >= boxes) break;
+        atomicAdd(&bsum[j * COB + 2 * word], sum[j].x);
+        atomicAdd(&bsum[j * COB + 2 * word + 1], sum[j].y);
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (ok)
+        for (int i = t; i < a.BN; i += 128) atomicAdd(a.db + n0 + i, bsum[i]);
+}
 
 template <int CIB, int COB>
 __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_constant__ WgradMaps maps,
@@ -399,6 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
     uint64_t* done = empty + a.stages;
     uint32_t* tslot = (uint32_t*)(done + 1);
     __shared__ int timed_out;
+    __shared__ float bsum[128];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ngroups = (a.taps + TPG - 1) / TPG;
@@ -414,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
     if (threadIdx.x == 0) {
         for (int s = 0; s < a.stages; ++s) {
             bar_init(&full[s], 1);
-            bar_init(&empty[s], 1);
+            bar_init(&empty[s], a.db ? 5 : 1);   // the MMAs, and the four warps that sum dZ
         }
         bar_init(done, 1);
         bar_fence_init();
@@ -431,10 +509,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
     if (warp == 0 && lane == 0) {
         tma_prefetch(&maps.x[src]);
         tma_prefetch(&maps.dz);
-        int issued = 0;
+        Ring r;
         for (int kb = 0; kb < nkb; ++kb) {
-            const int s = kb % a.stages, round = kb / a.stages;
-            if (kb >= a.stages && !bar_wait(&empty[s], (round - 1) & 1, 256)) {
+            const int s = r.s;
+            if (r.round > 0 && !bar_wait(&empty[s], (r.round - 1) & 1, 256)) {
                 atomicOr(a.flags, kFlagTimeout);
                 timed_out = 1;
                 break;
@@ -456,17 +534,17 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
                 tma_4d(st + j * A_BOX, &maps.x[src], cs, x0 + dx, y0 + dy, img, &full[s]);
             }
             for (int j = 0; j < nb; ++j) tma_4d(st + A_BYTES + j * B_BOX, &maps.dz, n0 + j * COB, x0, y0, img, &full[s]);
-            ++issued;
+            r.next(a.stages);
         }
-        for (int kb = max(0, issued - a.stages); kb < issued; ++kb)
-            if (!bar_wait(&full[kb % a.stages], (kb / a.stages) & 1, 256)) atomicOr(a.flags, kFlagTimeout);
+        drain(r, full, a.stages, a.flags);
     } else if (warp == 1 && lane == 0) {
         const uint32_t idesc = idesc_bf16(128, a.BN, true, true);
         const uint32_t la = swizzle_layout(CIB * 2), lb = swizzle_layout(COB * 2);
         const uint32_t atom_a = 8 * CIB * 2, atom_b = 8 * COB * 2;
-        for (int kb = 0; kb < nkb; ++kb) {
-            const int s = kb % a.stages, round = kb / a.stages;
-            if (!bar_wait(&full[s], round & 1, 64)) {
+        Ring r;
+        for (int kb = 0; kb < nkb; ++kb, r.next(a.stages)) {
+            const int s = r.s;
+            if (!bar_wait(&full[s], r.round & 1, 64)) {
                 atomicOr(a.flags, kFlagTimeout);
                 timed_out = 1;
                 break;
@@ -481,6 +559,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
         }
         mma_commit(done);
     } else if (warp >= 2) {
+        if (a.db) sum_dz<COB>(a, smem + A_BYTES, stage_bytes, full, empty, nkb, n0, bsum);
         const bool ok = __all_sync(0xffffffffu, bar_wait(done, 0, 1024));
         const bool go = ok && nkb > 0 && __shfl_sync(0xffffffffu, timed_out, 0) == 0;
         tc_after();

@@ -132,7 +132,6 @@ struct Dst {
     bf16* p = nullptr;
     int C = 0;
     const bf16* mask = nullptr;
-    int accumulate = 0;
 };
 
 int pixel_box(int W, int H, int* bw, int* bh) {
@@ -141,6 +140,44 @@ int pixel_box(int W, int H, int* bw, int* bh) {
     if (*bw * *bh != 128 || W % *bw || H % *bh)
         return fail(SAR_ERR_NOT_SUPPORTED, "image %dx%d: W must be a power of two >= 16 and H a multiple of 128/min(W,128)", W, H);
     return SAR_OK;
+}
+
+// Rows per item, CTAs an SM (0: use conv_fwd_kernel) and shared memory of conv_row_kernel.  It is taken where the SMs
+// have eight 128-pixel tiles each; with fewer its longer start shows, and the loads it saves do not.  Two rows an item
+// while both accumulator sets leave TMEM for two CTAs, as many CTAs an SM as fit (registers allow three), and the
+// filter resident if that costs no CTA, else a ring of at least four blocks.  The rows' ring holds what the tiles read
+// at one tap and two slots more.
+//
+// Measured at 512^2, one image, against conv_fwd_kernel: 32 -> 32 channels 15.8 us (20.3), 96 -> 32 34.3 (46.2),
+// 32 -> 96 26.2 (35.7).  At 256^2: 32 -> 64 10 to 12 us (9.5), 64 -> 64 13.2 (12.9), 192 -> 64 25.2 to 29 (27.2); at
+// 128^2 it is slower throughout.
+struct RowLayout {
+    unet::RowRing ring{0, 0, 0, 0};
+    int per_sm = 0;
+    size_t smem = 0;
+};
+RowLayout row_layout(int bk, int bn, int kpt, int ntn, int images, int H, int W) {
+    const int slot = unet::row_slot(bk), block = bn * bk * 2, nkb = 9 * kpt, cols = (int)unet::tmem_cols(bn);
+    RowLayout L;
+    if ((long)images * H * (W / 128) < 8L * device_sms()) return L;
+    const int R = 8 * cols <= 512 ? 2 : 1;
+    for (int per_sm = 3; per_sm >= 1; --per_sm)
+        for (int resident : {1, 0}) {
+            if (2 * R * cols * per_sm > 512 || (resident && ntn > 1)) continue;
+            int room = (int)(227 * 1024 / per_sm) - 1024 - 1024 - 2048 - 8192;   // reserved, alignment, barriers, epilogue
+            int na = R * kpt + 2, nb = resident ? nkb : 4;
+            room -= na * slot + nb * block;
+            if (room < 0) continue;
+            while (na < std::min(2 * (R + 2) * kpt, 32) && room >= slot) ++na, room -= slot;
+            while (!resident && nb < std::min(nkb, 8) && room >= block) ++nb, room -= block;
+            L.ring = unet::RowRing{R, na, nb, resident};
+            L.per_sm = per_sm;
+            L.smem = 1024 + (size_t)na * slot + (size_t)nb * block + (2 * (na + nb) + 4) * 8 + 16;
+            // no more CTAs than TMEM has room for share an SM (one beyond would wait in tcgen05.alloc)
+            L.smem = std::max(L.smem, (size_t)227 * 1024 / (per_sm + 1) + 1024);
+            return L;
+        }
+    return L;
 }
 
 // y = conv(x0 ++ x1) with weights wk [Nout][taps * (C0 + C1)] (bf16), epilogue per ConvArgs.
@@ -162,10 +199,13 @@ int conv_forward(Src s0, Src s1, int images, int H, int W, int taps, const bf16*
         BN /= 2;
     }
     if (!out_f32 && d0.C + (d1.p ? d1.C : 0) != Nout) return fail(SAR_ERR_INVALID_ARGUMENT, "conv: output split != Nout");
+    RowLayout rows;
+    if (taps == 9 && bw == 128) rows = row_layout(BK, BN, Ctot / BK, Nout / BN, images, H, W);
     ConvMaps maps;
     memset(&maps, 0, sizeof maps);
-    U_CALL(map_nhwc(&maps.src[0], s0.p, s0.C, W, H, images, BK, bw, bh));
-    if (nsrc > 1) U_CALL(map_nhwc(&maps.src[1], s1.p, s1.C, W, H, images, BK, bw, bh));
+    const int box = rows.per_sm ? kRowPixels : bw;
+    U_CALL(map_nhwc(&maps.src[0], s0.p, s0.C, W, H, images, BK, box, bh));
+    if (nsrc > 1) U_CALL(map_nhwc(&maps.src[1], s1.p, s1.C, W, H, images, BK, box, bh));
     U_CALL(map_matrix(&maps.wts, wk, taps * Ctot, Nout, BK, BN));
     ConvArgs a;
     memset(&a, 0, sizeof a);
@@ -192,19 +232,31 @@ int conv_forward(Src s0, Src s1, int images, int H, int W, int taps, const bf16*
     a.outc[1] = d1.C;
     a.mask[0] = d0.mask;
     a.mask[1] = d1.mask;
-    a.accumulate[0] = d0.accumulate;
-    a.accumulate[1] = d1.accumulate;
     a.out_f32 = out_f32;
     a.f32_keep = f32_keep;
     a.flags = flags;
+    a.images = images;
+    if (rows.per_sm) {
+        const int items = images * a.tiles_x * ((H + rows.ring.rows - 1) / rows.ring.rows) * (Nout / BN);
+        dim3 grid((unsigned)std::min(items, device_sms() * rows.per_sm));
+        auto go = [&](auto kern) -> int {
+            U_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows.smem), "smem attr");
+            kern<<<grid, kRowThreads, rows.smem, st>>>(maps, a, rows.ring);
+            return SAR_OK;
+        };
+        const bool two = rows.ring.rows == 2;
+        U_CALL(bk64 ? (two ? go(conv_row_kernel<64, 2>) : go(conv_row_kernel<64, 1>))
+                    : (two ? go(conv_row_kernel<32, 2>) : go(conv_row_kernel<32, 1>)));
+        U_CUDA(cudaGetLastError(), "conv forward launch");
+        return SAR_OK;
+    }
     size_t smem = 1024 + (size_t)a.stages * stage + (2 * a.stages + 4) * 8 + 16;
     // Persistent grid: as many CTAs as fit on the SMs, by shared memory and by TMEM (two
     // accumulators each).  When TMEM is the tighter limit the shared-memory request is raised so
     // that no more CTAs than that share an SM (a CTA beyond it would wait in tcgen05.alloc).
-    a.images = images;
     const int items = images * a.tiles_x * a.tiles_y * (Nout / BN);
     const size_t sm_smem = 227u * 1024u;
-    const int by_smem = std::max(1, (int)(sm_smem / smem));
+    const int by_smem = std::max(1, (int)(sm_smem / (smem + 9216)));   // with the static and reserved shared memory
     const int by_tmem = std::max(1, (int)(512u / (2u * tmem_cols(BN))));
     const int per_sm = std::max(1, std::min(by_smem, by_tmem));
     if (by_tmem < by_smem) smem = std::max(smem, sm_smem / (size_t)(per_sm + 1) + 1024);
@@ -541,7 +593,7 @@ int layer_forward(sar_unet* n, int i, float* out_f32, cudaStream_t st) {
     Src s0, s1;
     n->inputs(i, &s0, &s1);
     const int h = n->H >> l.level, w = n->W >> l.level;
-    Dst d0{i < 14 ? n->a[i] : nullptr, l.cout, nullptr, 0};
+    Dst d0{i < 14 ? n->a[i] : nullptr, l.cout, nullptr};
     return conv_forward(s0, s1, n->B, h, w, l.taps, n->wf[i], l.cout, n->params + n->b_off[i], l.relu, d0, Dst{},
                         i == 14 ? out_f32 : nullptr, 2, n->flags, st);
 }
@@ -557,13 +609,13 @@ int layer_backward(sar_unet* n, int i, cudaStream_t st) {
     if (i == 0) return SAR_OK;
     Dst d0, d1;
     switch (i) {
-        case 2: d0 = Dst{n->dp[0], l.c0, nullptr, 0}; break;
-        case 4: d0 = Dst{n->dp[1], l.c0, nullptr, 0}; break;
-        case 6: d0 = Dst{n->dp[2], l.c0, nullptr, 0}; break;
-        case 8: d0 = Dst{n->du[2], l.c0, nullptr, 0}; d1 = Dst{n->de[2], l.c1, nullptr, 0}; break;
-        case 10: d0 = Dst{n->du[1], l.c0, nullptr, 0}; d1 = Dst{n->de[1], l.c1, nullptr, 0}; break;
-        case 12: d0 = Dst{n->du[0], l.c0, nullptr, 0}; d1 = Dst{n->de[0], l.c1, nullptr, 0}; break;
-        default: d0 = Dst{n->dz[i - 1], l.c0, s0.p, 0}; break;   // previous layer feeds this one directly
+        case 2: d0 = Dst{n->dp[0], l.c0, nullptr}; break;
+        case 4: d0 = Dst{n->dp[1], l.c0, nullptr}; break;
+        case 6: d0 = Dst{n->dp[2], l.c0, nullptr}; break;
+        case 8: d0 = Dst{n->du[2], l.c0, nullptr}; d1 = Dst{n->de[2], l.c1, nullptr}; break;
+        case 10: d0 = Dst{n->du[1], l.c0, nullptr}; d1 = Dst{n->de[1], l.c1, nullptr}; break;
+        case 12: d0 = Dst{n->du[0], l.c0, nullptr}; d1 = Dst{n->de[0], l.c1, nullptr}; break;
+        default: d0 = Dst{n->dz[i - 1], l.c0, s0.p}; break;   // previous layer feeds this one directly
     }
     // Backward data: dX = conv(dz, flipped transposed filter); its input channels are l.cout.
     return conv_forward(Src{n->dz[i], l.cout}, Src{}, n->B, h, w, l.taps, n->wt[i], l.c0 + l.c1, nullptr, 0, d0, d1,
@@ -819,7 +871,7 @@ int sar_conv2d_forward_bf16(const void* x0, int c0, const void* x1, int c1, int 
                             void* stream) {
     if (!x0 || !w || !y || !flags_dev) return fail(SAR_ERR_INVALID_ARGUMENT, "null argument");
     return conv_forward(Src{(const bf16*)x0, c0}, Src{(const bf16*)x1, x1 ? c1 : 0}, batch, height, width, taps,
-                        (const bf16*)w, cout, bias, relu, Dst{(bf16*)y, cout, nullptr, 0}, Dst{}, nullptr, 0, flags_dev,
+                        (const bf16*)w, cout, bias, relu, Dst{(bf16*)y, cout, nullptr}, Dst{}, nullptr, 0, flags_dev,
                         (cudaStream_t)stream);
 }
 

@@ -11,7 +11,7 @@
 //    padding).  Weights come as 2-D TMA boxes of the [N][taps * C] matrix.  Both operands are
 //    K-major with a BK * 2-byte swizzle (128 B for BK = 64, 64 B for BK = 32).  The same kernel
 //    runs the backward-data pass with the flipped, transposed filter.  The epilogue adds the
-//    bias, applies ReLU or a ReLU-derivative mask, can add into the destination, splits the
+//    bias, applies ReLU or a ReLU-derivative mask, splits the
 //    columns over two destination tensors (the two halves of a concatenated input) and can write
 //    FP32 (the network output).
 //  * conv_wgrad_kernel<CIB, COB>: weight gradient  dW[co][tap, ci] = sum_pixel dZ[pixel][co] *
@@ -114,6 +114,15 @@ __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* m, int c0, 
         : "memory");
 }
 
+// One lane of the warp, by the instruction that lets the compiler keep the chosen lane's operands in uniform registers
+// (tcgen05.mma takes them there): behind `lane == 0` each MMA first moved its descriptors over, 50 to 70 cycles
+// against the 40 of an N = 32 MMA.
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(slot)), "r"(cols)
                  : "memory");
@@ -157,12 +166,25 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Shared-memory matrix descriptor (tcgen05): start address, leading / stride byte offsets (both
-// >> 4), descriptor version 1, swizzle layout in bits 61-63 (2 = 128 B, 4 = 64 B).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | ((uint64_t)layout << 61);
-}
+// Shared-memory matrix descriptor (tcgen05): start address, leading / stride byte offsets (all >> 4), descriptor
+// version 1, swizzle layout in bits 61-63 (2 = 128 B, 4 = 64 B).  In halves, so that the lane that issues the MMAs
+// only adds to the low one: it is a single thread's serial chain, and forming both descriptors anew for each MMA took
+// 200 cycles, several times the MMA's own.
+struct Desc {
+    uint32_t lo, hi;
+    __device__ __forceinline__ Desc(uint32_t addr, uint32_t lbo, uint32_t sbo, uint32_t layout)
+        : lo((addr >> 4) | ((lbo >> 4) << 16)), hi((sbo >> 4) | (1u << 14) | (layout << 29)) {}
+    __device__ __forceinline__ Desc moved(uint32_t bytes) const {
+        Desc d = *this;
+        d.lo += bytes >> 4;
+        return d;
+    }
+    __device__ __forceinline__ uint64_t at(uint32_t bytes) const {   // `bytes` further on: a constant
+        uint64_t d;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo + (bytes >> 4)), "r"(hi));
+        return d;
+    }
+};
 __host__ __device__ constexpr uint32_t swizzle_layout(int row_bytes) { return row_bytes == 128 ? 2u : 4u; }
 
 // Instruction descriptor of kind::f16: FP32 accumulator, bf16 A and B, K- or MN-major operands,
@@ -189,24 +211,43 @@ struct ConvArgs {
     __nv_bfloat16* out[2];             // columns [0, outc[0]) -> out[0], the rest -> out[1]
     int outc[2];
     const __nv_bfloat16* mask[2];      // zero the value where mask <= 0 (same layout as out)
-    int accumulate[2];                 // add into the destination
     float* out_f32;                    // when set: columns [0, f32_keep) as FP32 [pixel][f32_keep]
     int f32_keep;
     unsigned* flags;
 };
 
-// Epilogue of one output tile: 32 columns at a time from this warp's TMEM lanes.
+// Epilogue of one output tile: 32 columns at a time from this warp's TMEM lanes, a pixel per lane.  The rounded values
+// go through shared memory (2 KB a warp; 16-byte chunks swizzled by the pixel, so that neither side has bank conflicts)
+// to a mapping of four lanes per pixel, whose stores fill whole sectors and, with 32 channels, whole lines; stored a
+// pixel per lane, each 16-byte piece was a sector of its own, and the epilogue took 2400 cycles a tile.
 template <int BK>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tacc, int q, int lane, int img, int x0,
-                                              int y0, int n0) {
-    const int row = 32 * q + lane;
-    const int px = x0 + row % a.BW, py = y0 + row / a.BW;
-    const size_t pix = ((size_t)img * a.H + py) * a.W + px;
+                                              int y0, int n0, uint4* stage) {
+    const int lw = 31 - __clz(a.BW);   // BW is a power of two
+    auto pixel = [&](int row) {
+        return ((size_t)img * a.H + y0 + (row >> lw)) * a.W + x0 + (row & (a.BW - 1));
+    };
+    const int chunk = lane & 3, row0 = lane >> 2;   // of the lane's stores: pixels row0 + 8 j
     for (int c0 = 0; c0 < a.BN; c0 += 32) {
+        const int n = n0 + c0, d = n >= a.outc[0] ? 1 : 0, ch = d ? n - a.outc[0] : n;
+        uint4 mask[4];
+        if (!a.out_f32 && a.mask[d]) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                mask[j] = __ldg(reinterpret_cast<const uint4*>(a.mask[d] + pixel(32 * q + row0 + 8 * j) * a.outc[d] + ch) + chunk);
+        }
         float v[32];
         tmem_ld32(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, v);
-        const int n = n0 + c0;
-        if (a.bias) {
+        if (a.bias && ((uintptr_t)a.bias & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 w = __ldg(reinterpret_cast<const float4*>(a.bias + n + i));
+                v[i] += w.x;
+                v[i + 1] += w.y;
+                v[i + 2] += w.z;
+                v[i + 3] += w.w;
+            }
+        } else if (a.bias) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += __ldg(a.bias + n + i);
         }
@@ -215,40 +256,35 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tacc, 
             for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.f);
         }
         if (a.out_f32) {
+            const size_t pix = pixel(32 * q + lane);
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 if (n + i < a.f32_keep) a.out_f32[pix * a.f32_keep + n + i] = v[i];
             continue;
         }
-        const int d = n >= a.outc[0] ? 1 : 0;
-        const int ch = d ? n - a.outc[0] : n;
-        __nv_bfloat16* dst = a.out[d] + pix * a.outc[d] + ch;
-        if (a.mask[d]) {
-            const uint4* m4 = reinterpret_cast<const uint4*>(a.mask[d] + pix * a.outc[d] + ch);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint4 mm = m4[j];
-                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mm);
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (!(__bfloat162float(mb[i]) > 0.f)) v[8 * j + i] = 0.f;
-            }
-        }
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (a.accumulate[d]) {
-                const uint4 old = d4[j];
-                const __nv_bfloat16* ob = reinterpret_cast<const __nv_bfloat16*>(&old);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[8 * j + i] += __bfloat162float(ob[i]);
-            }
             uint4 pk;
             __nv_bfloat162* pb = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
             for (int i = 0; i < 4; ++i) pb[i] = __floats2bfloat162_rn(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
-            d4[j] = pk;
+            stage[4 * lane + (j ^ ((lane >> 1) & 3))] = pk;
         }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int row = row0 + 8 * j;
+            uint4 pk = stage[4 * row + (chunk ^ ((row >> 1) & 3))];
+            if (a.mask[d]) {   // zero where mask <= 0 or not a number
+                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mask[j]);
+                __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(&pk);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (!(__bfloat162float(mb[i]) > 0.f)) pb[i] = __float2bfloat16_rn(0.f);
+            }
+            *(reinterpret_cast<uint4*>(a.out[d] + pixel(32 * q + row) * a.outc[d] + ch) + chunk) = pk;
+        }
+        __syncwarp();
     }
 }
 
@@ -267,8 +303,9 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
     uint64_t* tempty = tfull + 2;         // [2]
     uint32_t* tslot = (uint32_t*)(tempty + 2);
     __shared__ int timed_out;
+    __shared__ uint4 stage_out[4][128];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int per_img = a.tiles_x * a.tiles_y;
     const int ntn = a.Nout / a.BN;
     const int items = a.images * per_img * ntn;
@@ -292,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
     }
     __syncthreads();
     tc_after();
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
     const int kpt = a.Ctot / BK, nkb = a.taps * kpt;
 
     if (warp == 0 && lane == 0) {
@@ -330,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
             }
         }
         drain(r, full, a.stages, a.flags);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_lane()) {
         const uint32_t idesc = idesc_bf16(128, a.BN, false, false);
         const uint32_t lay = swizzle_layout(BK * 2), sbo = 8 * BK * 2;
         Ring r;
@@ -353,12 +390,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
                     stop = true;
                     break;
                 }
-                tc_after();
                 const uint32_t sa = su32(smem + s * stage_bytes), sb = sa + a_bytes;
+                const Desc da(sa, 16, sbo, lay), db(sb, 16, sbo, lay);
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)
-                    mma_bf16(tacc, smem_desc(sa + 32 * k, 16, sbo, lay), smem_desc(sb + 32 * k, 16, sbo, lay), idesc,
-                             (kb | k) != 0);
+                for (int k = 0; k < BK / 16; ++k) mma_bf16(tacc, da.at(32 * k), db.at(32 * k), idesc, (kb | k) != 0);
                 mma_commit(&empty[s]);
                 r.next(a.stages);
             }
@@ -379,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
                 const int mt = it / ntn, n0 = (it % ntn) * a.BN;
                 const int img = mt / per_img, rem = mt % per_img;
                 conv_epilogue<BK>(a, tmem + (uint32_t)(b * ncols), q, lane, img, (rem % a.tiles_x) * a.BW,
-                                  (rem / a.tiles_x) * a.BH, n0);
+                                  (rem / a.tiles_x) * a.BH, n0, stage_out[q]);
             }
             tc_before();
             __syncwarp();
@@ -390,6 +425,192 @@ __global__ void __launch_bounds__(kThreads, 1) conv_fwd_kernel(const __grid_cons
     if (warp == 1) {
         tc_after();
         tmem_dealloc(tmem, 2 * ncols);
+    }
+}
+
+// 3x3 convolutions of images at least 128 pixels wide.  An item is 128 pixels of R neighbouring image rows, each row a
+// tile with an accumulator of its own.  The nine taps of the R tiles read R + 2 rows of 130 pixels: each is loaded once
+// per channel block, and the taps along x are the same box from one pixel further on (the descriptor's start address
+// moves by a pixel; the swizzle goes by the address).  Filters that fit are loaded once per CTA and stay; larger ones
+// run through a ring of their own, fed by a warp of its own.  A tile's K blocks are summed in the same order as in
+// conv_fwd_kernel (taps, then channels), so the results are the same bits.
+//
+// Bound: the one lane that issues the MMAs.  An N = 32 MMA takes 40 cycles when they follow each other, and some 100 with
+// the waits and addresses between them; hence R tiles to one filter block, and several CTAs an SM.
+constexpr int kRowThreads = 224;   // and warp 6: the filter's loads
+constexpr int kRowPixels = 130;
+__host__ __device__ constexpr int row_slot(int bk) { return (kRowPixels * bk * 2 + 1023) & ~1023; }
+
+struct RowRing {
+    int rows;        // R
+    int na, nb;      // slots of rows (a channel block each) and of filter blocks
+    int resident;    // nb holds the whole filter
+};
+
+template <int BK, int R>
+__global__ void __launch_bounds__(kRowThreads, 3) conv_row_kernel(const __grid_constant__ ConvMaps maps, const ConvArgs a,
+                                                                  const RowRing ring) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    constexpr int SLOT = row_slot(BK), ROW = BK * 2;
+    const int b_bytes = a.BN * ROW;
+    uint8_t* wts = smem + ring.na * SLOT;
+    uint64_t* afull = (uint64_t*)(wts + ring.nb * b_bytes);
+    uint64_t* aempty = afull + ring.na;
+    uint64_t* bfull = aempty + ring.na;
+    uint64_t* bempty = bfull + ring.nb;
+    uint64_t* tfull = bempty + ring.nb;   // [2]
+    uint64_t* tempty = tfull + 2;         // [2]
+    uint32_t* tslot = (uint32_t*)(tempty + 2);
+    __shared__ int timed_out;
+    __shared__ uint4 stage_out[4][128];
+
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int groups = (a.H + R - 1) / R;
+    const int per_img = a.tiles_x * groups, ntn = a.Nout / a.BN, items = a.images * per_img * ntn;
+    const uint32_t ncols = tmem_cols(a.BN);   // of an accumulator; two sets of R
+    const int kpt = a.Ctot / BK, nkb = 9 * kpt;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ring.na; ++s) {
+            bar_init(&afull[s], 1);
+            bar_init(&aempty[s], 1);
+        }
+        for (int s = 0; s < ring.nb; ++s) {
+            bar_init(&bfull[s], 1);
+            bar_init(&bempty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            bar_init(&tfull[b], 1);
+            bar_init(&tempty[b], 4);
+        }
+        bar_fence_init();
+        timed_out = 0;
+    }
+    if (warp == 1) {
+        tmem_alloc(tslot, 2 * R * ncols);
+        tmem_relinquish();
+    }
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
+    auto give_up = [&] {
+        atomicOr(a.flags, kFlagTimeout);
+        timed_out = 1;
+    };
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch(&maps.src[0]);
+        if (a.nsrc > 1) tma_prefetch(&maps.src[1]);
+        Ring r;
+        bool stop = false;
+        for (int it = blockIdx.x; it < items && !stop; it += gridDim.x) {
+            const int mt = it / ntn, img = mt / per_img, rem = mt % per_img;
+            const int x0 = (rem % a.tiles_x) * 128, y0 = rem / a.tiles_x * R;
+            for (int row = -1; row <= R && !stop; ++row)
+                for (int c = 0; c < a.Ctot; c += BK, r.next(ring.na)) {
+                    if (r.round > 0 && !bar_wait(&aempty[r.s], (r.round - 1) & 1, 256)) {
+                        give_up();
+                        stop = true;
+                        break;
+                    }
+                    const int src = c >= a.C0 ? 1 : 0;
+                    bar_expect_tx(&afull[r.s], (uint32_t)(kRowPixels * ROW));
+                    tma_4d(smem + r.s * SLOT, &maps.src[src], src ? c - a.C0 : c, x0 - 1, y0 + row, img, &afull[r.s]);
+                }
+        }
+        drain(r, afull, ring.na, a.flags);
+    } else if (warp == 6 && lane == 0) {
+        tma_prefetch(&maps.wts);
+        Ring r;
+        bool stop = false;
+        for (int it = blockIdx.x; it < items && !stop; it += gridDim.x) {
+            const int n0 = (it % ntn) * a.BN;
+            for (int kb = 0; kb < nkb; ++kb, r.next(ring.nb)) {
+                if (r.round > 0 && !bar_wait(&bempty[r.s], (r.round - 1) & 1, 256)) {
+                    give_up();
+                    stop = true;
+                    break;
+                }
+                bar_expect_tx(&bfull[r.s], (uint32_t)b_bytes);
+                tma_2d(wts + r.s * b_bytes, &maps.wts, kb * BK, n0, &bfull[r.s]);
+            }
+            if (ring.resident) break;
+        }
+        drain(r, bfull, ring.nb, a.flags);
+    } else if (warp == 1 && elect_lane()) {
+        const uint32_t idesc = idesc_bf16(128, a.BN, false, false);
+        const uint32_t lay = swizzle_layout(ROW), sbo = 8 * ROW;
+        const Desc da0(su32(smem), 16, sbo, lay), db0(su32(wts), 16, sbo, lay);
+        Ring rb;
+        int first = 0;        // slot of the item's first row
+        uint32_t phase = 0;   // a bit per slot of rows: the phase that its next load completes
+        int i = 0;
+        bool stop = false;
+        auto wrap = [&](int s) { return s >= ring.na ? s - ring.na : s; };
+        for (int it = blockIdx.x; it < items && !stop; it += gridDim.x, ++i) {
+            const int b = i & 1;
+            if (i >= 2 && !bar_wait(&tempty[b], (uint32_t)(((i >> 1) - 1) & 1), 256)) {
+                give_up();
+                break;
+            }
+            tc_after();
+            const uint32_t tacc = tmem + (uint32_t)(b * R) * ncols;
+            if (ring.resident) rb = Ring{};
+            for (int dy = 0; dy < 3 && !stop; ++dy, first = wrap(first + kpt))   // first: row dy, which tile 0 reads
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx)
+                    for (int c = 0; c < kpt && !stop; ++c, rb.next(ring.nb)) {
+                        if ((!ring.resident || i == 0) && !bar_wait(&bfull[rb.s], rb.round & 1, 64)) stop = true;
+                        const Desc db = db0.moved(rb.s * b_bytes);
+                        int s = wrap(first + c);
+#pragma unroll
+                        for (int j = 0; j < R; ++j, s = wrap(s + kpt)) {
+                            // a row is first read at dx = 0 by the tile that comes to it first, last at dx = 2
+                            if (dx == 0 && (dy == 0 || j == R - 1)) {
+                                if (!stop && !bar_wait(&afull[s], phase >> s & 1, 64)) stop = true;
+                                phase ^= 1u << s;
+                            }
+                            if (stop) continue;
+                            const Desc da = da0.moved(s * SLOT + dx * ROW);
+#pragma unroll
+                            for (int k = 0; k < BK / 16; ++k)
+                                mma_bf16(tacc + j * ncols, da.at(32 * k), db.at(32 * k), idesc, (dy | dx | c | k) != 0);
+                            if (dx == 2 && (dy == 2 || j == 0)) mma_commit(&aempty[s]);
+                        }
+                        if (!ring.resident) mma_commit(&bempty[rb.s]);
+                    }
+            if (stop) give_up();
+            for (int row = 3; row < R + 2; ++row) first = wrap(first + kpt);
+            mma_commit(&tfull[b]);   // also on the timeout path, so the epilogue warps are released
+        }
+    } else if (warp >= 2 && warp < 6) {
+        const int q = warp & 3;
+        int i = 0;
+        for (int it = blockIdx.x; it < items; it += gridDim.x, ++i) {
+            const int b = i & 1;
+            const bool ok = __all_sync(0xffffffffu, bar_wait(&tfull[b], (uint32_t)((i >> 1) & 1), 1024));
+            tc_after();
+            if (!ok) {
+                if (lane == 0) atomicOr(a.flags, kFlagTimeout);
+                break;
+            }
+            if (__shfl_sync(0xffffffffu, timed_out, 0) == 0) {
+                const int mt = it / ntn, img = mt / per_img, rem = mt % per_img;
+                const int y0 = rem / a.tiles_x * R;
+                for (int j = 0; j < R && y0 + j < a.H; ++j)
+                    conv_epilogue<BK>(a, tmem + (uint32_t)(b * R + j) * ncols, q, lane, img, (rem % a.tiles_x) * 128, y0 + j,
+                                      (it % ntn) * a.BN, stage_out[q]);
+            }
+            tc_before();
+            __syncwarp();
+            if (lane == 0) bar_try_arrive(&tempty[b]);
+        }
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc_after();
+        tmem_dealloc(tmem, 2 * R * ncols);
     }
 }
 
@@ -478,7 +699,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
     __shared__ int timed_out;
     __shared__ float bsum[128];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int ngroups = (a.taps + TPG - 1) / TPG;
     const int tg = blockIdx.y % ngroups, cb = blockIdx.y / ngroups;
     const int cglob = cb * CIB, src = cglob >= a.C0 ? 1 : 0, cs = src ? cglob - a.C0 : cglob;
@@ -504,7 +725,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
     }
     __syncthreads();
     tc_after();
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
 
     if (warp == 0 && lane == 0) {
         tma_prefetch(&maps.x[src]);
@@ -537,10 +758,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
             r.next(a.stages);
         }
         drain(r, full, a.stages, a.flags);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_lane()) {
         const uint32_t idesc = idesc_bf16(128, a.BN, true, true);
         const uint32_t la = swizzle_layout(CIB * 2), lb = swizzle_layout(COB * 2);
-        const uint32_t atom_a = 8 * CIB * 2, atom_b = 8 * COB * 2;
+        constexpr uint32_t atom_a = 8 * CIB * 2, atom_b = 8 * COB * 2;
         Ring r;
         for (int kb = 0; kb < nkb; ++kb, r.next(a.stages)) {
             const int s = r.s;
@@ -549,12 +770,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
                 timed_out = 1;
                 break;
             }
-            tc_after();
             const uint32_t sa = su32(smem + s * stage_bytes), sb = sa + A_BYTES;
+            const Desc da(sa, A_BOX, atom_a, la), db(sb, B_BOX, atom_b, lb);
 #pragma unroll
             for (int k = 0; k < 8; ++k)   // 16 pixel rows (two 8-row groups) per MMA
-                mma_bf16(tmem, smem_desc(sa + 2 * atom_a * k, A_BOX, atom_a, la),
-                         smem_desc(sb + 2 * atom_b * k, B_BOX, atom_b, lb), idesc, (kb | k) != 0);
+                mma_bf16(tmem, da.at(2 * atom_a * k), db.at(2 * atom_b * k), idesc, (kb | k) != 0);
             mma_commit(&empty[s]);
         }
         mma_commit(done);

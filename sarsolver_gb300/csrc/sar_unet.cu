@@ -289,8 +289,10 @@ int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int 
     if (Cout % BN) return fail(SAR_ERR_NOT_SUPPORTED, "wgrad: output channels %d cannot be tiled", Cout);
     WgradMaps maps;
     memset(&maps, 0, sizeof maps);
-    U_CALL(map_nhwc(&maps.x[0], s0.p, s0.C, W, H, images, CIB, bw, bh));
-    if (nsrc > 1) U_CALL(map_nhwc(&maps.x[1], s1.p, s1.C, W, H, images, CIB, bw, bh));
+    const bool rows = taps == 9 && bw == 128;
+    const int box = rows ? kWgradPixels : bw;
+    U_CALL(map_nhwc(&maps.x[0], s0.p, s0.C, W, H, images, CIB, box, bh));
+    if (nsrc > 1) U_CALL(map_nhwc(&maps.x[1], s1.p, s1.C, W, H, images, CIB, box, bh));
     U_CALL(map_nhwc(&maps.dz, dz, Cout, W, H, images, COB, bw, bh));
     WgradArgs a;
     memset(&a, 0, sizeof a);
@@ -308,6 +310,17 @@ int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int 
     a.tiles_y = H / bh;
     a.num_tiles = images * a.tiles_x * a.tiles_y;
     a.BN = BN;
+    a.dw = dw;
+    a.db = db;
+    a.flags = flags;
+    auto launch = [&](auto kern, int splits, int mtiles, size_t smem) -> int {
+        U_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+        kern<<<dim3((unsigned)splits, (unsigned)mtiles, (unsigned)(Cout / BN)), kThreads, smem, st>>>(maps, a);
+        U_CUDA(cudaGetLastError(), "wgrad launch");
+        return SAR_OK;
+    };
+    // K blocks per CTA: three CTAs an SM in conv_wgrad_kernel's division.  No more go into one accumulator with either
+    // kernel: its sums are truncated, so the error grows with their number (1.9e-6 for 14 blocks at 512^2, 2.8e-6 for 21).
     const int tpg = 128 / CIB;
     const int ngroups = (taps + tpg - 1) / tpg;
     const int mtiles = ngroups * (Ctot / CIB), ntiles = Cout / BN;
@@ -315,26 +328,31 @@ int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int 
     int splits = std::max(1, std::min(a.num_tiles, (want + mtiles * ntiles - 1) / (mtiles * ntiles)));
     a.tiles_per_split = (a.num_tiles + splits - 1) / splits;
     splits = (a.num_tiles + a.tiles_per_split - 1) / a.tiles_per_split;
+    if (rows) {
+        // As many CTAs an SM as run these splits in one round, if two stages each fit.  Measured against
+        // conv_wgrad_kernel: 512^2 32 -> 32 channels 18.8 us (30.4), 96 -> 32 40.6 (69.5); 256^2 64 -> 64 12.5 (18.1),
+        // 192 -> 64 19.9 (34.0); 128^2 384 -> 128 18.1 (29.4).
+        const int units = 3 * (Ctot / CIB) * ntiles, acc = (CIB == 64 ? 2 : 1) * (int)tmem_cols(BN);
+        const int stage = ((kWgradPixels * CIB * 2 + 1023) & ~1023) + BN * 128 * 2;
+        const int room = 227 * 1024 - 4096;
+        int per_sm = std::max(1, std::min({3, 512 / acc, room / (2 * stage + 4096), (splits * units + device_sms() - 1) / device_sms()}));
+        a.stages = std::max(2, std::min(8, (room / per_sm - 4096) / stage));
+        const int fit = per_sm * device_sms() / units;   // splits in one round
+        if (fit > splits) {
+            a.tiles_per_split = (a.num_tiles + fit - 1) / fit;
+            splits = (a.num_tiles + a.tiles_per_split - 1) / a.tiles_per_split;
+        }
+        size_t smem = 1024 + (size_t)a.stages * stage + (2 * a.stages + 2) * 8 + 16;
+        smem = std::max(smem, (size_t)room / (per_sm + 1) + 1024);   // no CTA more than TMEM and the stages are meant for
+        const int mt = 3 * (Ctot / CIB);   // filter rows and channel blocks
+        return ci64 ? (co64 ? launch(conv_wgrad_row_kernel<64, 64>, splits, mt, smem) : launch(conv_wgrad_row_kernel<64, 32>, splits, mt, smem))
+                    : (co64 ? launch(conv_wgrad_row_kernel<32, 64>, splits, mt, smem) : launch(conv_wgrad_row_kernel<32, 32>, splits, mt, smem));
+    }
     const int stage = 128 * 128 * 2 + BN * 128 * 2;
     a.stages = std::max(2, std::min(6, (kSmemBudget - 2048) / stage));
-    a.dw = dw;
-    a.db = db;
-    a.flags = flags;
     const size_t smem = 1024 + (size_t)a.stages * stage + (2 * a.stages + 2) * 8 + 16;
-    dim3 grid((unsigned)splits, (unsigned)mtiles, (unsigned)ntiles);
-#define U_WG(CI, CO)                                                                                                 \
-    do {                                                                                                             \
-        U_CUDA(cudaFuncSetAttribute(conv_wgrad_kernel<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), \
-               "smem attr");                                                                                         \
-        conv_wgrad_kernel<CI, CO><<<grid, kThreads, smem, st>>>(maps, a);                                            \
-    } while (0)
-    if (ci64 && co64) U_WG(64, 64);
-    else if (ci64) U_WG(64, 32);
-    else if (co64) U_WG(32, 64);
-    else U_WG(32, 32);
-#undef U_WG
-    U_CUDA(cudaGetLastError(), "wgrad launch");
-    return SAR_OK;
+    return ci64 ? (co64 ? launch(conv_wgrad_kernel<64, 64>, splits, mtiles, smem) : launch(conv_wgrad_kernel<64, 32>, splits, mtiles, smem))
+                : (co64 ? launch(conv_wgrad_kernel<32, 64>, splits, mtiles, smem) : launch(conv_wgrad_kernel<32, 32>, splits, mtiles, smem));
 }
 
 // ------------------------------------------------------------------ elementwise kernels

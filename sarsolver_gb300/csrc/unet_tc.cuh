@@ -808,4 +808,134 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_kernel(const __grid_co
     }
 }
 
+// The weight gradient of 3x3 filters over images at least 128 pixels wide: a K block is 128 pixels of an image row, and
+// a CTA forms the three taps of one filter row from one box of 131 pixels of X (the taps lie a pixel apart in it: the
+// leading offset of the descriptor), where conv_wgrad_kernel loads a box per tap.  An M tile holds four taps of 32
+// channels or two of 64; those past the third are formed and not stored.
+//
+// Bound: L2 to shared memory.  32 -> 32 channels, 512^2: 16 KB of X and dZ a K block and filter row, before 40 KB for
+// four taps.  Measured figures stand at conv_wgrad (sar_unet.cu).
+constexpr int kWgradPixels = 131;
+
+template <int CIB, int COB>
+__global__ void __launch_bounds__(kThreads, 1) conv_wgrad_row_kernel(const __grid_constant__ WgradMaps maps,
+                                                                  const WgradArgs a) {
+    constexpr int ROW = CIB * 2, SLOTS = 128 / CIB;   // bytes of a pixel; taps of a 128-row M tile
+    constexpr int MT = CIB == 64 ? 2 : 1;             // M tiles for the three taps of a filter row
+    constexpr int B_BOX = 128 * COB * 2;
+    constexpr int A_BYTES = (kWgradPixels * ROW + 1023) & ~1023;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int nb = a.BN / COB;
+    const int stage_bytes = A_BYTES + nb * B_BOX;
+    const uint32_t load_bytes = kWgradPixels * ROW + nb * B_BOX;
+    uint64_t* full = (uint64_t*)(smem + a.stages * stage_bytes);
+    uint64_t* empty = full + a.stages;
+    uint64_t* done = empty + a.stages;
+    uint32_t* tslot = (uint32_t*)(done + 1);
+    __shared__ int timed_out;
+    __shared__ float bsum[128];
+
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int dy = blockIdx.y % 3, cb = blockIdx.y / 3;   // filter row, channel block
+    const int cglob = cb * CIB, src = cglob >= a.C0 ? 1 : 0, cs = src ? cglob - a.C0 : cglob;
+    const int n0 = blockIdx.z * a.BN;
+    const int t_begin = blockIdx.x * a.tiles_per_split;
+    const int t_end = min(a.num_tiles, t_begin + a.tiles_per_split);
+    const int nkb = max(0, t_end - t_begin);
+    const uint32_t ncols = tmem_cols(a.BN);
+    const int per_img = a.tiles_x * a.tiles_y;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.stages; ++s) {
+            bar_init(&full[s], 1);
+            bar_init(&empty[s], a.db ? 5 : 1);   // the MMAs, and the four warps that sum dZ
+        }
+        bar_init(done, 1);
+        bar_fence_init();
+        timed_out = 0;
+    }
+    if (warp == 1) {
+        tmem_alloc(tslot, MT * ncols);
+        tmem_relinquish();
+    }
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch(&maps.x[src]);
+        tma_prefetch(&maps.dz);
+        Ring r;
+        for (int kb = 0; kb < nkb; ++kb) {
+            const int s = r.s;
+            if (r.round > 0 && !bar_wait(&empty[s], (r.round - 1) & 1, 256)) {
+                atomicOr(a.flags, kFlagTimeout);
+                timed_out = 1;
+                break;
+            }
+            const int t = t_begin + kb, img = t / per_img, rem = t % per_img;
+            const int x0 = (rem % a.tiles_x) * 128, y0 = rem / a.tiles_x;
+            uint8_t* st = smem + s * stage_bytes;
+            bar_expect_tx(&full[s], load_bytes);
+            tma_4d(st, &maps.x[src], cs, x0 - 1, y0 + dy - 1, img, &full[s]);
+            for (int j = 0; j < nb; ++j) tma_4d(st + A_BYTES + j * B_BOX, &maps.dz, n0 + j * COB, x0, y0, img, &full[s]);
+            r.next(a.stages);
+        }
+        drain(r, full, a.stages, a.flags);
+    } else if (warp == 1 && elect_lane()) {
+        const uint32_t idesc = idesc_bf16(128, a.BN, true, true);
+        const uint32_t la = swizzle_layout(ROW), lb = swizzle_layout(COB * 2);
+        constexpr uint32_t atom_a = 8 * CIB * 2, atom_b = 8 * COB * 2;
+        Ring r;
+        for (int kb = 0; kb < nkb; ++kb, r.next(a.stages)) {
+            const int s = r.s;
+            if (!bar_wait(&full[s], r.round & 1, 64)) {
+                atomicOr(a.flags, kFlagTimeout);
+                timed_out = 1;
+                break;
+            }
+            const uint32_t sa = su32(smem + s * stage_bytes), sb = sa + A_BYTES;
+            const Desc da(sa, ROW, atom_a, la), db(sb, B_BOX, atom_b, lb);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)   // 16 pixels (two 8-pixel groups) per MMA; the taps of an M tile a pixel apart
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+                    mma_bf16(tmem + m * ncols, da.at(m * SLOTS * ROW + 2 * atom_a * k), db.at(2 * atom_b * k), idesc, (kb | k) != 0);
+            mma_commit(&empty[s]);
+        }
+        mma_commit(done);
+    } else if (warp >= 2) {
+        if (a.db) sum_dz<COB>(a, smem + A_BYTES, stage_bytes, full, empty, nkb, n0, bsum);
+        const bool ok = __all_sync(0xffffffffu, bar_wait(done, 0, 1024));
+        const bool go = ok && nkb > 0 && __shfl_sync(0xffffffffu, timed_out, 0) == 0;
+        tc_after();
+        if (!ok) {
+            if (lane == 0) atomicOr(a.flags, kFlagTimeout);
+        } else if (go) {
+            const int q = warp & 3, row = 32 * q + lane, ci = cglob + row % CIB;
+            const size_t ktot = (size_t)9 * a.Ctot;
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const int dx = m * SLOTS + row / CIB;
+                for (int c0 = 0; c0 < a.BN; c0 += 32) {
+                    float v[32];
+                    tmem_ld32(tmem + m * ncols + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, v);
+                    if (dx < 3) {
+                        float* dst = a.dw + (size_t)(n0 + c0) * ktot + (size_t)(3 * dy + dx) * a.Ctot + ci;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) atomicAdd(dst + (size_t)i * ktot, v[i]);
+                    }
+                }
+            }
+        }
+        tc_before();
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc_after();
+        tmem_dealloc(tmem, MT * ncols);
+    }
+}
+
 }  // namespace unet

@@ -528,6 +528,10 @@ struct sar_unet {
     bf16 *wf[kLayers] = {}, *wt[kLayers] = {};
     bf16* wbuf = nullptr;
     unsigned* flags = nullptr;
+    // The weight gradients run beside the chain of data gradients, on a stream of their own that is forked from the
+    // caller's and joined to it again within each backward pass.
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     // activations and gradients of the current (B, H, W)
     int B = 0, H = 0, W = 0;
     std::vector<void*> bufs;
@@ -545,6 +549,9 @@ struct sar_unet {
         release_activations();
         for (void* q : {(void*)params, (void*)grads, (void*)m, (void*)v, (void*)wbuf, (void*)flags})
             if (q) cudaFree(q);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
         if (prev >= 0) cudaSetDevice(prev);
     }
     void release_activations() {
@@ -616,14 +623,17 @@ int layer_forward(sar_unet* n, int i, float* out_f32, cudaStream_t st) {
                         i == 14 ? out_f32 : nullptr, 2, n->flags, st);
 }
 
-// Weight and bias gradients of layer i from dz[i], then (i > 0) the gradient of its input.
+// Weight and bias gradients of layer i from dz[i] (on the side stream: no later kernel of the pass writes what they
+// read, or reads what they write), and (i > 0) the gradient of its input.
 int layer_backward(sar_unet* n, int i, cudaStream_t st) {
     const LayerSpec& l = n->L[i];
     Src s0, s1;
     n->inputs(i, &s0, &s1);
     const int h = n->H >> l.level, w = n->W >> l.level;
+    U_CUDA(cudaEventRecord(n->fork, st), "fork");
+    U_CUDA(cudaStreamWaitEvent(n->side, n->fork, 0), "fork");
     U_CALL(conv_wgrad(s0, s1, n->dz[i], l.cout, n->B, h, w, l.taps, n->grads + n->w_off[i],
-                      n->grads + n->b_off[i], n->flags, st));
+                      n->grads + n->b_off[i], n->flags, n->side));
     if (i == 0) return SAR_OK;
     Dst d0, d1;
     switch (i) {
@@ -668,7 +678,7 @@ int do_forward(sar_unet* n, const float2* in, float scale, float* out, cudaStrea
     return SAR_OK;
 }
 
-int do_backward(sar_unet* n, const float2* gout, cudaStream_t st) {
+int backward_layers(sar_unet* n, const float2* gout, cudaStream_t st) {
     const size_t P0 = n->pixels(0);
     prep_input_kernel<<<ew_grid(P0 * 4), 256, 0, st>>>(gout, 1.f, n->dz[14], P0);
     U_CALL(layer_backward(n, 14, st));   // -> dz[13]
@@ -699,6 +709,16 @@ int do_backward(sar_unet* n, const float2* gout, cudaStream_t st) {
     }
     U_CALL(layer_backward(n, 0, st));
     U_CUDA(cudaGetLastError(), "U-Net backward");
+    return SAR_OK;
+}
+
+int do_backward(sar_unet* n, const float2* gout, cudaStream_t st) {
+    const int rc = backward_layers(n, gout, st);
+    // also after an error: what was forked ends before anything later on the caller's stream
+    const cudaError_t e = cudaEventRecord(n->join, n->side), f = cudaStreamWaitEvent(st, n->join, 0);
+    if (rc) return rc;
+    U_CUDA(e, "join");
+    U_CUDA(f, "join");
     return SAR_OK;
 }
 
@@ -759,6 +779,12 @@ int sar_unet_create(int base_channels, int device, sar_unet** out) {
     get((void**)&n->v, off * 4);
     get((void**)&n->wbuf, woff * 2 * sizeof(bf16));
     get((void**)&n->flags, 16);
+    int least = 0, greatest = 0;   // the data gradients are the longer chain: they go first
+    if (rc == SAR_OK && (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+                         cudaStreamCreateWithPriority(&n->side, cudaStreamNonBlocking, least) != cudaSuccess ||
+                         cudaEventCreateWithFlags(&n->fork, cudaEventDisableTiming) != cudaSuccess ||
+                         cudaEventCreateWithFlags(&n->join, cudaEventDisableTiming) != cudaSuccess))
+        rc = fail(SAR_ERR_CUDA, "U-Net side stream");
     if (rc) {
         delete n;
         return rc;

@@ -1,8 +1,10 @@
 """Convolutions of images at least 128 pixels wide (a tile is part of one image row), with the tolerance of the other
-forward convolution tests, 4e-3 (bf16 outputs)."""
+forward convolution tests, 4e-3 (bf16 outputs); and the backward pass, whose weight gradients run on a stream forked
+from the caller's, on other streams and under graph capture (FP32 sums in another order: 1e-5 of the gradient)."""
 import pytest
 import torch
 
+from sarsolver_gb300.unet import UNet
 from test_gpu_unet import test_conv_forward as conv_forward
 
 pytestmark = pytest.mark.gpu
@@ -32,3 +34,34 @@ ROW_CASES = [
 @pytest.mark.parametrize("case", ROW_CASES)
 def test_wide_conv_forward(case):
     conv_forward(case)
+
+
+@pytest.mark.parametrize("H,W", [(128, 128), (64, 256)])
+def test_backward_on_streams_and_captured(H, W):
+    net = UNet(base_channels=32, seed=7)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    x, go = (torch.complex(torch.randn(1, H, W, device="cuda", generator=g), torch.randn(1, H, W, device="cuda", generator=g))
+             for _ in range(2))
+
+    def step():
+        net.zero_grad()
+        net.forward(x)
+        net.backward(go)
+        return net.grads()
+
+    ref = step().clone()
+    close = lambda t: float((t - ref).norm() / ref.norm()) < 1.0e-5
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert all(close(step()) for _ in range(3))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step()
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        assert close(out)
+    assert net.flags() == 0

@@ -198,6 +198,9 @@ int conv_forward(Src s0, Src s1, int images, int H, int W, int taps, const bf16*
         if (BN % 2 || (BN / 2) % 32) return fail(SAR_ERR_NOT_SUPPORTED, "conv: output channels %d cannot be tiled", Nout);
         BN /= 2;
     }
+    // Tiles for less than half the SMs: split the output channels (256 channels at 64^2: 20 -> 12 us; the sums' order does
+    // not change).  Not with more tiles: at 128^2 halves of 128 channels took 12 us instead of 10, their loads being doubled.
+    while (BN >= 128 && BN % 64 == 0 && 2L * images * (W / bw) * (H / bh) * (Nout / BN) < device_sms()) BN /= 2;
     if (!out_f32 && d0.C + (d1.p ? d1.C : 0) != Nout) return fail(SAR_ERR_INVALID_ARGUMENT, "conv: output split != Nout");
     RowLayout rows;
     if (taps == 9 && bw == 128) rows = row_layout(BK, BN, Ctot / BK, Nout / BN, images, H, W);

@@ -28,12 +28,12 @@
 namespace {
 
 // x += alpha p over P entries and r -= alpha q over NS entries, alpha = sc[ig] / sc[iq]
-// (0 when the denominator is not positive: the caller then stops).
+// (0 when the denominator is not positive: the caller then stops).  Clears sc[iclear] for the next norm.
 __global__ void update_xr_kernel(float2* __restrict__ x, const float2* __restrict__ p, size_t P,
                                  float2* __restrict__ r, const float2* __restrict__ q, size_t NS,
-                                 const double* __restrict__ sc, int ig, int iq) {
-    const double den = sc[iq];
-    const float alpha = den > 0.0 ? (float)(sc[ig] / den) : 0.f;
+                                 double* __restrict__ sc, int ig, int iq, int iclear) {
+    const float alpha = block_ratio(sc + ig, sc + iq);
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc[iclear] = 0.0;
     const size_t total = P + NS;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         if (i < P) {
@@ -53,11 +53,11 @@ __global__ void update_xr_kernel(float2* __restrict__ x, const float2* __restric
     }
 }
 
-// p = s + beta p, beta = sc[inew] / sc[iold].
+// p = s + beta p, beta = sc[inew] / sc[iold].  Clears sc[iclear] for the next norm.
 __global__ void update_p_kernel(float2* __restrict__ p, const float2* __restrict__ s, size_t P,
-                                const double* __restrict__ sc, int inew, int iold) {
-    const double den = sc[iold];
-    const float beta = den > 0.0 ? (float)(sc[inew] / den) : 0.f;
+                                double* __restrict__ sc, int inew, int iold, int iclear) {
+    const float beta = block_ratio(sc + inew, sc + iold);
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc[iclear] = 0.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < P; i += (size_t)gridDim.x * blockDim.x) {
         float2 a = p[i];
         const float2 b = __ldg(s + i);
@@ -91,8 +91,7 @@ __global__ void dot_re_kernel(const float2* __restrict__ a, const float2* __rest
 __global__ void scale_start_kernel(float2* __restrict__ x, size_t P, float2* __restrict__ r,
                                    const float2* __restrict__ y, size_t NS, const double* __restrict__ sc, int inum,
                                    int iden) {
-    const double den = sc[iden];
-    const float c = den > 0.0 ? (float)(sc[inum] / den) : 0.f;
+    const float c = block_ratio(sc + inum, sc + iden);
     const size_t total = P + NS;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         if (i < P) {
@@ -161,7 +160,7 @@ extern "C" int sar_cgls_ex(sar_plan* plan, const void* y_dev, void* x_dev, int s
         CG_CUDA(cudaMemcpyAsync(w.s, ahy_dev, sizeof(float2) * P, cudaMemcpyDeviceToDevice, st), "A^H y");
     else
         CG_CALL(sar_adjoint(plan, y, w.s, st));
-    norm2_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(w.s, P, w.sc + 3);
+    norm2_kernel<<<norm_grid(P, sms), kThreads, 0, st>>>(w.s, P, w.sc + 3);
     if (start == SAR_CGLS_START_ZERO) {
         CG_CUDA(cudaMemsetAsync(x, 0, sizeof(float2) * P, st), "zero x");
         CG_CUDA(cudaMemcpyAsync(w.r, y, sizeof(float2) * NS, cudaMemcpyDeviceToDevice, st), "r = y");
@@ -169,7 +168,7 @@ extern "C" int sar_cgls_ex(sar_plan* plan, const void* y_dev, void* x_dev, int s
         // x0 = c z with c = Re<z, A^H y> / ||A z||^2, the minimiser of ||y - c A z||.
         CG_CALL(sar_forward(plan, x, w.r, st));
         dot_re_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(x, w.s, P, w.sc + 4);
-        norm2_kernel<<<grid_for(NS, sms), kThreads, 0, st>>>(w.r, NS, w.sc + 5);
+        norm2_kernel<<<norm_grid(NS, sms), kThreads, 0, st>>>(w.r, NS, w.sc + 5);
         scale_start_kernel<<<grid_for(P + NS, sms), kThreads, 0, st>>>(x, P, w.r, y, NS, w.sc, 4, 5);
         CG_CALL(sar_adjoint(plan, w.r, w.s, st));
     } else {
@@ -177,7 +176,7 @@ extern "C" int sar_cgls_ex(sar_plan* plan, const void* y_dev, void* x_dev, int s
         residual_kernel<<<grid_for(NS, sms), kThreads, 0, st>>>(w.r, y, NS);
         CG_CALL(sar_adjoint(plan, w.r, w.s, st));
     }
-    norm2_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(w.s, P, w.sc + 0);
+    norm2_kernel<<<norm_grid(P, sms), kThreads, 0, st>>>(w.s, P, w.sc + 0);
     CG_CUDA(cudaMemcpyAsync(w.p, w.s, sizeof(float2) * P, cudaMemcpyDeviceToDevice, st), "p = s");
     CG_CUDA(cudaGetLastError(), "CGLS set-up kernels");
 
@@ -199,12 +198,10 @@ extern "C" int sar_cgls_ex(sar_plan* plan, const void* y_dev, void* x_dev, int s
     for (int it = 1; it <= max_iterations; ++it) {
         const int nxt = cur ^ 1;
         CG_CALL(sar_forward(plan, w.p, w.q, st));
-        CG_CUDA(cudaMemsetAsync(w.sc + 2, 0, sizeof(double), st), "clear |q|^2");
-        norm2_kernel<<<grid_for(NS, sms), kThreads, 0, st>>>(w.q, NS, w.sc + 2);
-        update_xr_kernel<<<grid_for(P + NS, sms), kThreads, 0, st>>>(x, w.p, P, w.r, w.q, NS, w.sc, cur, 2);
+        norm2_kernel<<<norm_grid(NS, sms), kThreads, 0, st>>>(w.q, NS, w.sc + 2);
+        update_xr_kernel<<<grid_for(P + NS, sms), kThreads, 0, st>>>(x, w.p, P, w.r, w.q, NS, w.sc, cur, 2, nxt);
         CG_CALL(sar_adjoint(plan, w.r, w.s, st));
-        CG_CUDA(cudaMemsetAsync(w.sc + nxt, 0, sizeof(double), st), "clear gamma");
-        norm2_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(w.s, P, w.sc + nxt);
+        norm2_kernel<<<norm_grid(P, sms), kThreads, 0, st>>>(w.s, P, w.sc + nxt);
         CG_CUDA(cudaGetLastError(), "CGLS kernels");
         CG_CUDA(cudaMemcpyAsync(host_sc, w.sc, sizeof(double) * 3, cudaMemcpyDeviceToHost, st), "read scalars");
         CG_CUDA(cudaStreamSynchronize(st), "CGLS iteration");
@@ -222,7 +219,7 @@ extern "C" int sar_cgls_ex(sar_plan* plan, const void* y_dev, void* x_dev, int s
             result->converged = 1;
             return SAR_OK;
         }
-        update_p_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(w.p, w.s, P, w.sc, nxt, cur);
+        update_p_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(w.p, w.s, P, w.sc, nxt, cur, 2);
         cur = nxt;
     }
     CG_CUDA(cudaGetLastError(), "CGLS kernels");

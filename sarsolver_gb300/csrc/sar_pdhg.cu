@@ -88,8 +88,10 @@ __global__ void power_start_kernel(float2* __restrict__ v, size_t n) {
 
 // v *= 1 / sqrt(*n2) (left unchanged when the norm is zero).
 __global__ void normalise_kernel(float2* __restrict__ v, size_t n, const double* __restrict__ n2) {
-    const double s2 = *n2;
-    const float k = s2 > 0.0 ? (float)(1.0 / std::sqrt(s2)) : 1.f;
+    __shared__ float scale;   // once per block: FP64 runs at two operations a cycle and SM
+    if (threadIdx.x == 0) scale = *n2 > 0.0 ? (float)(1.0 / std::sqrt(*n2)) : 1.f;
+    __syncthreads();
+    const float k = scale;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float2 a = v[i];
         a.x *= k;
@@ -117,15 +119,15 @@ static int estimate_norm(sar_plan* plan, size_t P, size_t NS, int iterations, fl
                          double* sc, int sms, cudaStream_t st, double* norm_out) {
     power_start_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(v, P);
     CG_CUDA(cudaMemsetAsync(sc, 0, sizeof(double), st), "clear norm");
-    norm2_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(v, P, sc);
+    norm2_kernel<<<norm_grid(P, sms), kThreads, 0, st>>>(v, P, sc);
     normalise_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(v, P, sc);
     double aq = 0.0;
     for (int it = 0; it < iterations; ++it) {
         CG_CALL(sar_forward(plan, v, q, st));
         CG_CUDA(cudaMemsetAsync(sc, 0, 2 * sizeof(double), st), "clear norms");
-        norm2_kernel<<<grid_for(NS, sms), kThreads, 0, st>>>(q, NS, sc);
+        norm2_kernel<<<norm_grid(NS, sms), kThreads, 0, st>>>(q, NS, sc);
         CG_CALL(sar_adjoint(plan, q, s, st));
-        norm2_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(s, P, sc + 1);
+        norm2_kernel<<<norm_grid(P, sms), kThreads, 0, st>>>(s, P, sc + 1);
         CG_CUDA(cudaMemcpyAsync(v, s, sizeof(float2) * P, cudaMemcpyDeviceToDevice, st), "v = A^H A v");
         normalise_kernel<<<grid_for(P, sms), kThreads, 0, st>>>(v, P, sc + 1);
     }

@@ -240,7 +240,7 @@ def run_ours(args):
     k2_ms = stage_ms[1] / max(calls, 1)
     fft_ms = stage_ms[0] / max(calls, 1)
     achieved = P * S / (k2_ms * 1e-3)
-    traffic = read_profile_traffic("bp_grid_ws_pair")
+    traffic = read_profile_traffic("gather")
     result = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
@@ -250,18 +250,18 @@ def run_ours(args):
         "config": {"workload": f"{args.case}: backprojection, {desc}, {args.interp.replace('_ref', '')} interpolation",
                    "pixels": P, "pulses": S, "samples": N, "upsample": upsample,
                    "l2": "inputs larger than L2 (phase history %.0f MB, stored range profiles %.0f MB)"
-                         % (S * N * 8 / 1e6, S * plan.profile_length * (8 if plan.tile_window > 256 else 16) / 1e6),
+                         % (S * N * 8 / 1e6, S * plan.profile_length * 8 / 1e6),
                    "parallelism": "replicas (each GPU runs the whole workload)" if world > 1 else "single GPU"},
         "stages_ms": {"upsample_fft_side": fft_ms, "gather_kernel": k2_ms},
         "forward": {"value": P * S / (fwd_ms * 1e-3), "unit": UNIT, "ms_per_step": fwd_ms,
                     "stages_ms": {"accumulator_clear": fstage[0] / max(fcalls, 1),
                                   "scatter_kernel": fstage[1] / max(fcalls, 1),
                                   "downsample_fft_side": fstage[2] / max(fcalls, 1)},
-                    "note": "y = A x on the same workload (fp_grid_ws_kernel + FFT downsampling), not the headline"},
-        "roofline": {"bound": bound, "kernel": "bp_grid_ws_pair_kernel", "achieved": achieved, "peak": r_roof,
+                    "note": "y = A x on the same workload (scatter_kernel + fir_down_kernel), not the headline"},
+        "roofline": {"bound": bound, "kernel": "gather_kernel", "achieved": achieved, "peak": r_roof,
                      "unit": "px*pulse/s", "frac": achieved / r_roof, "traffic": traffic,
                      "traffic_source": "from profile: ncu dram__bytes_read.sum + dram__bytes_write.sum per "
-                                       "full-size launch, profiles/bp_grid_ws_pair_kernel_config2.md",
+                                       "full-size launch, profiles/gather_kernel_config2.md",
                      "peak_basis": f"{props.multi_processor_count} SMs x {sm_max:.0f} MHz (sm_max_mhz of "
                                    f"MEASURED_PEAKS.json) x min(2 x {rates['ffma_per_clk_sm']:.1f} FFMA/clk/SM / 28 "
                                    f"FP32 flops, {rates['sfu_sincos_per_clk_sm']:.1f} sin+cos/clk/SM / 3 SFU ops) "
@@ -271,10 +271,9 @@ def run_ours(args):
         "e2e": {"value": job_throughput(P * S, world, e2e_ms), "unit": UNIT, "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": S * N * 8, "d2h_bytes_per_step": P * 8,
                 "api": "NumpySimpleSarOperator.backproject(pinned host complex64 tensor) -> pinned host copy"},
-        # our kernels per backprojection: per FFT chunk the fused upsampling kernel, or the packing
-        # and unpacking kernels around cuFFT; then the gather
-        "gpu_launches": args.steps * ((1 if plan.fused_upsampling else 2)
-                                      * ((S + plan_chunk(plan) - 1) // plan_chunk(plan)) + 1),
+        # our kernels per backprojection (upsampling, gather, the sum of its partial images), counted in
+        # one profiled call after the timed ones
+        "gpu_launches": args.steps * launches_per_call(lambda: plan.adjoint(y, out=x)),
         "clocks": clocks,
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -361,9 +360,23 @@ def pipe_rates(dev) -> dict:
             "sms": r.num_sms, "probe_sm_mhz": r.sm_mhz}
 
 
-def plan_chunk(plan) -> int:
-    # one FFT chunk covers all pulses for every configuration here (4 GiB of rows)
-    return plan.num_slow_times
+def launches_per_call(fn) -> int:
+    """Kernels of this library that one call of ``fn`` launches (2, the upsampling and the gather, where
+    the profiler is not available)."""
+    import torch
+    try:
+        from torch.profiler import ProfilerActivity, profile
+        count = 0
+        for _ in range(2):   # a process's first profile holds no kernels
+            with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+                fn()
+                torch.cuda.synchronize()
+            count = sum(1 for e in prof.events()
+                        if e.device_type == torch.autograd.DeviceType.CUDA and "sar::" in e.name)
+        return count if count > 0 else 2
+    except Exception as exc:
+        print(f"launch count not profiled: {exc}", file=sys.stderr)
+        return 2
 
 
 def read_profile_traffic(kernel: str):

@@ -114,19 +114,22 @@ typedef struct sar_plan_info {
     long profile_first_bin;     /* first stored range bin (may be negative) */
     size_t profile_length;      /* stored bins per pulse */
     size_t tile_window;         /* staged bins per (tile, pulse); 0 on the unstructured path */
-    size_t strip_window;        /* forward strip window (bins); 0 on the unstructured path */
+    size_t strip_window;        /* forward window (bins) of a strip or ring, or of a lane of the lattice
+                                   scatter; 0 on the unstructured path */
     size_t device_bytes;        /* device memory held by the plan */
     int grid;                   /* 1 regular-grid path, 0 unstructured path */
     int interp;                 /* SAR_INTERP_* of the plan */
     size_t num_fast_times, num_slow_times, num_scatterers;   /* N, S, P */
     int device;                 /* CUDA device of the plan */
     int fft_callbacks;          /* 1: range-profile FFTs run with cuFFT load/store callbacks */
-    int gather_lanes_y;         /* 1: the grid backprojection runs warp lanes along y (bins change
-                                   more slowly along y than along x), 0: along x */
-    int fused_upsampling;       /* 1: the backprojection's range profiles come from the fused
-                                   upsampling kernel (N = 512 ... 8192, M a multiple of N), 0: cuFFT */
-    int fused_downsampling;     /* 1: the forward projection's FFT side is the fused downsampling
-                                   kernel (N = 512 ... 8192, M a multiple of N), 0: cuFFT */
+    int gather_lanes_y;         /* 1: range bins change more slowly along y than along x, and the tile
+                                   kernel of the backprojection runs warp lanes along y; 0: along x.
+                                   (This and the shears below describe the tile kernels; plans that
+                                   walk a pixel lattice along the iso-range lines do not use them.) */
+    int fused_upsampling;       /* 1: the backprojection's range profiles come from one fused kernel
+                                   (N = 512 ... 8192, M a multiple of N), 0: kernels around cuFFT */
+    int fused_downsampling;     /* 1: the forward projection's FFT side is one fused kernel
+                                   (N = 512 ... 8192, M a multiple of N), 0: kernels around cuFFT */
     int scatter_lanes_y;        /* 1: the grid forward scatter runs warp lanes along y and walks the
                                    tile along x (bins change more slowly along x), 0: lanes along x */
     size_t block_pulses;        /* streamed plan: pulses per block (0: resident plan) */

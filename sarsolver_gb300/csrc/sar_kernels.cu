@@ -1,6 +1,8 @@
-// sar_kernels.cu -- sm_103a kernels of the SAR operator pair.
+// sar_kernels.cu -- sm_103a kernels of the SAR operator pair: tiles, unstructured points, and transforms of
+// any upsampling factor.  The grid plans that fit run on sar_gather.cu and sar_scatter.cu, and even upsampling factors
+// from four on sar_fir.cu.
 //
-//   K1  upsample_pairs (fused, N = 1024, 2048, 4096) or pack_adjoint / cuFFT / unpack_pairs
+//   K1  upsample_pairs (fused, N = 512 ... 8192) or pack_adjoint / cuFFT / unpack_pairs
 //                                      range-profile upsampling (replaces sarsolver_cxx.cpp:331-344)
 //   K2  bp_grid_ws_pair / bp_grid / bp_points
 //                                      backprojection gather (replaces :345-350)
@@ -9,7 +11,7 @@
 //                                      range-profile downsampling around the FFT (:292-307)
 //
 // Nearest-bin sampling (the reference's rule) on the grid kernels uses split bins and decides
-// every bin within 5e-5 of a rounding boundary again in double-float (exact_grid_bin), so the
+// every bin within 5e-5 of a rounding boundary again in double-float (sar_exact.cuh), so the
 // bins equal those of FP64 rounding; the per-pixel kernels compute every bin that way.
 //
 // Layout in HBM: images are complex64 [nz][ny][nx]; phase histories complex64 [S][N] with

@@ -556,7 +556,7 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             const int bins = p->interp == SAR_INTERP_NEAREST_REF ? GATHER_NEAREST
                              : p->gc_fwd.precise_bins            ? GATHER_LINEAR
                                                                  : GATHER_RUNS;
-            p->gather = gather_layout(bins, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+            p->gather = gather_layout(bins, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa);
         }
         if (p->gather.ok) {
             const Lattice& L = p->gather.lattice;
@@ -614,7 +614,7 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         // forward projections are reproducible, which the many small runs of the other scatter are not.
         if (p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins &&
             (p->fwd_transposed ? p->gc_fwd.tiles_y : p->gc_fwd.tiles_x) > 2)
-            p->scatter = scatter_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+            p->scatter = scatter_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa);
         if (p->scatter.ok) {
             const ScatterLayout& L = p->scatter;
             double ea[3], eb[3];
@@ -709,7 +709,15 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             const Lattice plain{1, 0, 0, 1, true};
             const LatticeBounds B = lattice_bounds(plain, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, 16.0, 16.0);
             const double h = B.ok ? B.excursion(16.0, 16.0, s_r) : 0.5 * grid_tile_window(g, s_r);
-            if (h >= 0.0 && h < 1.0e6) {
+            // Rings beyond 2048 slots (by the isotropic or scene-wide bound) only where the tiles' expansions are exact:
+            // else the per-pixel kernels, which such plans ran on before rings of that size fitted, stay.
+            bool take = B.ok && expansion_turns(B.len_a, B.len_b, B.nearest, kappa) < kExpansionTurns;
+            if (!take) {
+                const double hd = tile_halfspan_directional(tx, rx, S, origin, ex, ey, ez, kTile, p->gc_fwd.tiles_x,
+                                                            p->gc_fwd.tiles_y, nz, s_r);
+                take = 2.0 * (std::ceil(hd >= 0.0 ? hd : 0.5 * grid_tile_window(g, s_r)) + 4.0) + 1.0 <= 2048.0;
+            }
+            if (take && h >= 0.0 && h < 1.0e6) {
                 const int H = (int)std::ceil(h) + 4, W = (2 * H + 1 + 31) & ~31;
                 for (size_t budget : {kFpRingTwoBudget, kFpRingSmemBudget}) {
                     if (p->ring_half) break;

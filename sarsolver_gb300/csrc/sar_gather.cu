@@ -592,12 +592,12 @@ int gather_parts(const GatherLayout& L, size_t count, size_t pixels) {
 }
 
 GatherLayout gather_layout(int bins, const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                           const double* ey, const double* ez, int nx, int ny, int nz, double s_r) {
+                           const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa) {
     GatherLayout best;
     const bool split = bins != GATHER_RUNS;
     // split bins: the lanes along the iso-range lines, 16 pixels per thread across them
-    Lattice lattice = split ? choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kGatherWalk, 192, split_cost)
-                            : choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kGatherLines, 64, run_cost);
+    Lattice lattice = split ? choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, kGatherWalk, 192, split_cost)
+                            : choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, kGatherLines, 64, run_cost);
     if (!lattice.ok) return best;
     if (split) {
         std::swap(lattice.vx, lattice.wx);

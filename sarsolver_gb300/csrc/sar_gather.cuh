@@ -54,7 +54,7 @@ struct GatherArgs {
 
 // Layout for the sampling `bins`; not ok where the lattice or the windows do not fit.
 GatherLayout gather_layout(int bins, const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                           const double* ey, const double* ez, int nx, int ny, int nz, double s_r);
+                           const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa);
 // Parts for `count` pulses (at most the layout's).
 int gather_parts(const GatherLayout& L, size_t count, size_t pixels);
 cudaError_t launch_gather(const GatherArgs& a, cudaStream_t st);

@@ -360,9 +360,9 @@ static void scatter_items(size_t S, int nx, int ny, int nz, ScatterLayout* L) {
 }
 
 ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r) {
+                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa) {
     ScatterLayout L;
-    L.lattice = choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, 16, kWalk, run_cost);
+    L.lattice = choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, 16, kWalk, run_cost);
     if (!L.lattice.ok) return L;
     const LatticeBounds B = lattice_bounds(L.lattice, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, 8.0, 8.0);
     if (!B.ok) return L;

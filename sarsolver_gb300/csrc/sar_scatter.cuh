@@ -37,7 +37,7 @@ struct ScatterArgs {
 
 // Host-side choice of lattice, block and segments for linear sampling without split bins (see sar_scatter.cu).
 ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r);
+                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa);
 cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st);
 
 }  // namespace sar

@@ -72,3 +72,23 @@ def test_every_sample_near_a_boundary(along, upsample, step):
     spacing[along] = step * bin_m
     scene = GridSarScene([1, 65, 97], [0.0, spacing[1] * 64, spacing[0] * 96])
     check(Case(scene, ap, upsample, {}), upsample, rng)
+
+
+@pytest.mark.parametrize("interp,upsample,pulses,az,shape,degrees,n", [
+    ("linear", 3.0, 159, 309.0, (1, 241, 184), 28.5, 512), ("linear", 64.0, 53, 22.0, (1, 50, 92), 13.1, 256),
+    ("nearest_ref", 4.0, 45, 124.0, (2, 225, 52), 10.7, 500)])
+def test_coarse_pixels_at_short_range(interp, upsample, pulses, az, shape, degrees, n):
+    """0.8 m pixels at 2 km, where third-order expansions about 16 x 16 pixels leave up to d^4 / (4 R^3) = 1.9e-6 m of
+    range (d = 8 x 1.6 m, R = 1.5 km), 4e-4 rad, a twentieth of it (2e-5) in the mean over a block: lattices with longer
+    steps would leave more, and are not taken there."""
+    rng = np.random.default_rng(pulses)
+    tx = spotlight(pulses, degrees, 2.0e3, 1.0e3, az)
+    rx = spotlight(pulses, 0.5 * degrees, 1.6e3, 0.6e3, az + 20.0)
+    ap = NumpySimpleSarAperture(tx, rx, 0.1 * rng.normal(size=(pulses, 3)), 10.0e9, 200.0e6, num_freqs=n)
+    scene = GridSarScene(list(shape), [2.0 * (shape[0] - 1), 0.8 * (shape[1] - 1), 0.8 * (shape[2] - 1)])
+    plan, general = (SarPlan(scene, ap, upsample_ratio=upsample, interp=interp, path=p) for p in ("grid", "points"))
+    x = torch.from_numpy(crandn(rng, scene.num_scatterers))
+    y = torch.from_numpy(crandn(rng, pulses, n))
+    assert rel_l2(plan.forward(x).cpu().numpy(), general.forward(x).cpu().numpy()) < 2.0e-5
+    assert rel_l2(plan.adjoint(y).cpu().numpy(), general.adjoint(y).cpu().numpy()) < 2.0e-5
+    assert plan.device_flags() == 0

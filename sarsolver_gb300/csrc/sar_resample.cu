@@ -219,32 +219,36 @@ struct DevBuf {
 };
 
 // Batched C2C plans by (device, length, rows), made on first use and kept for the process (plan
-// creation costs milliseconds; resampling jobs repeat the same shapes).  Calls on one plan are
-// serialised by the stream they run on; the cache itself is guarded by a mutex.
+// creation costs milliseconds; resampling jobs repeat the same shapes).  A plan has one work area and one
+// stream, so its uses follow each other: the mutex covers setting the stream and queueing the transform,
+// and a use on another stream waits on the device for the event that the last one left behind.
+struct FftPlan {
+    bool made = false;
+    cufftHandle handle = 0;
+    cudaEvent_t last = nullptr;   // end of the plan's last use
+};
 std::mutex g_plan_mu;
-std::map<std::tuple<int, int, int>, cufftHandle> g_plans;
+std::map<std::tuple<int, int, int>, FftPlan> g_plans;
 
 int fft_rows(void* data, int n, int rows, int direction, cudaStream_t st) {
     int dev = 0;
     cudaGetDevice(&dev);
-    cufftHandle h = 0;
-    {
-        std::lock_guard<std::mutex> lock(g_plan_mu);
-        auto key = std::make_tuple(dev, n, rows);
-        auto it = g_plans.find(key);
-        if (it != g_plans.end()) {
-            h = it->second;
-        } else {
-            int dims[1] = {n};
-            if (cufftPlanMany(&h, 1, dims, nullptr, 1, n, nullptr, 1, n, CUFFT_C2C, rows) != CUFFT_SUCCESS)
-                return err(SAR_ERR_CUFFT, "resampling FFT plan");
-            g_plans[key] = h;
-        }
+    std::lock_guard<std::mutex> lock(g_plan_mu);
+    FftPlan& plan = g_plans[std::make_tuple(dev, n, rows)];
+    if (!plan.last) R_CUDA(cudaEventCreateWithFlags(&plan.last, cudaEventDisableTiming), "resampling FFT event");
+    if (!plan.made) {
+        int dims[1] = {n};
+        if (cufftPlanMany(&plan.handle, 1, dims, nullptr, 1, n, nullptr, 1, n, CUFFT_C2C, rows) != CUFFT_SUCCESS)
+            return err(SAR_ERR_CUFFT, "resampling FFT plan");
+        plan.made = true;
     }
-    cufftResult r = cufftSetStream(h, st);
+    R_CUDA(cudaStreamWaitEvent(st, plan.last, 0), "resampling FFT order");
+    cufftResult r = cufftSetStream(plan.handle, st);
     if (r == CUFFT_SUCCESS)
-        r = cufftExecC2C(h, (cufftComplex*)data, (cufftComplex*)data, direction);
+        r = cufftExecC2C(plan.handle, (cufftComplex*)data, (cufftComplex*)data, direction);
+    const cudaError_t e = cudaEventRecord(plan.last, st);   // also after an error: part of it may be queued
     if (r != CUFFT_SUCCESS) return err(SAR_ERR_CUFFT, "resampling FFT");
+    R_CUDA(e, "resampling FFT order");
     return SAR_OK;
 }
 

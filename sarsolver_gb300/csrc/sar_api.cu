@@ -92,6 +92,7 @@ constexpr size_t kFpSmemBudget = 110 * 1024;
 constexpr size_t kFpRingTwoBudget = 113 * 1024 - 256;   // ring windows: two CTAs per SM (228 KB, 1 KB each reserved)
 constexpr size_t kFpRingSmemBudget = 220 * 1024;   // one CTA per SM
 constexpr size_t kSpecBudget = (size_t)4 << 30;   // bytes of FFT work rows per chunk
+constexpr size_t kChunkRows = 65535;              // rows per chunk: gridDim.y of the kernels around the transforms
 
 }  // namespace
 
@@ -880,7 +881,7 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
     p->fft_len = p->fir ? 2 * (long)N : (long)M;
     p->fft_double = !smooth_length((size_t)p->fft_len);
     const size_t elem = p->fft_double ? sizeof(double2) : sizeof(float2);
-    p->chunk = (int)std::min<size_t>(p->block ? p->block : S, std::max<size_t>(1, kSpecBudget / (p->fft_len * elem)));
+    p->chunk = (int)std::min({p->block ? p->block : S, std::max<size_t>(1, kSpecBudget / (p->fft_len * elem)), kChunkRows});
     if (p->fir) {
         std::vector<float> taps, pair_taps;
         std::vector<double> inv_c;

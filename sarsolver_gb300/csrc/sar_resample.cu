@@ -294,8 +294,11 @@ struct Packed {
     }
 };
 
-// Rows of `N` filtered at a time for cuFFT: about 32 MB, which stay in L2 until they are cropped.
-size_t work_rows(size_t N, size_t T) { return std::min(T, std::max<size_t>(1, ((size_t)32 << 20) / (N * sizeof(float2)))); }
+// Rows of `N` filtered at a time for cuFFT: about 32 MB, which stay in L2 until they are cropped, and at most the
+// 65535 that gridDim.y takes.
+size_t work_rows(size_t N, size_t T) {
+    return std::min({T, std::max<size_t>(1, ((size_t)32 << 20) / (N * sizeof(float2))), (size_t)65535});
+}
 
 size_t packed_bytes(size_t S, size_t N, size_t n, size_t L, size_t T) {
     auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
@@ -367,7 +370,7 @@ int resample(const float2* ph, size_t S, size_t N, const double* delta_range, do
                 filter_rows_kernel<<<grid, 256, 0, st>>>(a, rows, (int)first);
                 R_CUDA(cudaGetLastError(), "slow-time filter");
                 R_CALL(fft_rows(rows, (int)N, count, CUFFT_INVERSE, st));
-                const dim3 crop((unsigned)std::min<size_t>((n + 255) / 256, 1024), (unsigned)std::min(count, 65535));
+                const dim3 crop((unsigned)std::min<size_t>((n + 255) / 256, 1024), (unsigned)count);
                 crop_window_kernel<<<crop, 256, 0, st>>>(rows, out + first * n, a.window, count, (int)N, (int)n);
                 R_CUDA(cudaGetLastError(), "crop");
             }

@@ -137,7 +137,8 @@ def resample_dataset(dataset, fast_downsample_factor: float = 1.0, slow_downsamp
     (metres) and the k-space extent of the aperture at the new SRP, with ``safety_factor`` margin.
     Output pulse t combines old pulses [D t, D t + L) (D = slow factor, L = round(5 D) taps),
     placed at old pulse D t + L // 2; windows touching a pulse with non-finite positions are
-    dropped.  ``keep_on_device`` leaves the phase history as a complex64 CUDA tensor.
+    dropped.  ``keep_on_device`` leaves the phase history as a complex64 CUDA tensor; it is finished when the call
+    returns, so any stream may read it.
     """
     dev = _device(device)
     ap = dataset.aperture
@@ -194,5 +195,7 @@ def resample_dataset(dataset, fast_downsample_factor: float = 1.0, slow_downsamp
     srps = np.repeat(new_srp[None, :], len(starts), axis=0)
     new_ap = NumpySimpleSarAperture(tx, rx, srps, ap.centre_frequency, ap.sample_bandwidth, waveform_fft=wave,
                                     slow_time_weighting=new_wt, sign_multiplier=ap.sign_multiplier, c_eff=ap.c_eff)
+    if keep_on_device:
+        torch.cuda.current_stream(dev).synchronize()
     ph = out if keep_on_device else out.cpu().numpy().astype(np.complex128)
     return NumpySimpleSarDataset(new_ap, ph)

@@ -87,3 +87,15 @@ def test_two_threads():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_result_on_device_is_finished():
+    """The tensor that resample_dataset leaves on the device can be read on any stream once the call has returned."""
+    S = N = 8192   # milliseconds of device work, against some 0.3 ms of host work after its launch
+    tx = np.stack([np.full(S, 9e3), np.linspace(-300, 300, S), np.full(S, 4e3)], axis=-1)
+    ap = NumpySimpleSarAperture(tx, tx.copy(), np.zeros((S, 3)), 10.0e9, 200.0e6, num_freqs=N)
+    ds = NumpySimpleSarDataset(ap, history(S, N, 31))
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for _ in range(3):
+            rs.resample_dataset(ds, 1.0, 1, new_srp=np.array([5.0, 5.0, 0.0]), keep_on_device=True)
+            assert torch.cuda.current_stream().query()

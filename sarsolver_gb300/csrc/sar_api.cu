@@ -148,6 +148,8 @@ struct sar_plan {
     bool fir = false;
     FirLayout fir_layout;
     float2* d_fir_wave = nullptr;   // waveform / c(k)
+    double2* d_fir_wave64 = nullptr;   // the same and the taps below for complex128 rows
+    double *d_taps64 = nullptr, *d_pair_taps64 = nullptr;
     float2* d_half = nullptr;       // e^{2 pi i k / (2 N)} (fused kernels)
     float* d_taps = nullptr;
     float* d_pair_taps = nullptr;
@@ -213,6 +215,9 @@ struct sar_plan {
         cudaFree(d_tw_n);
         cudaFree(d_tw_m);
         cudaFree(d_fir_wave);
+        cudaFree(d_fir_wave64);
+        cudaFree(d_taps64);
+        cudaFree(d_pair_taps64);
         cudaFree(d_half);
         cudaFree(d_taps);
         cudaFree(d_pair_taps);
@@ -879,17 +884,21 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
     const bool want_cb = !p->block && cb_env && cb_env[0] == '1' && smooth_length(M);
     p->fir = !want_cb && fir_plan((long)N, (long)M, p->Lg, p->bg0, &p->fir_layout);
     p->fft_len = p->fir ? 2 * (long)N : (long)M;
-    p->fft_double = !smooth_length((size_t)p->fft_len);
+    // Lengths M with a prime factor above 7 are transformed in complex128 (also where 2 N has none, so that the choice
+    // does not depend on the route), filtered in FP64 and rounded once.  FP32 there: the profiles' error 2.5e-8 -> 8e-8.
+    p->fft_double = !smooth_length(M);
     const size_t elem = p->fft_double ? sizeof(double2) : sizeof(float2);
     p->chunk = (int)std::min({p->block ? p->block : S, std::max<size_t>(1, kSpecBudget / (p->fft_len * elem)), kChunkRows});
     if (p->fir) {
-        std::vector<float> taps, pair_taps;
-        std::vector<double> inv_c;
-        fir_tables(p->fir_layout, &taps, &pair_taps, &inv_c);
+        std::vector<double> taps64, pair_taps64, inv_c;
+        fir_tables(p->fir_layout, &taps64, &pair_taps64, &inv_c);
+        const std::vector<float> taps(taps64.begin(), taps64.end()), pair_taps(pair_taps64.begin(), pair_taps64.end());
+        std::vector<double2> fw64(N);
         std::vector<float2> fw(N), half(N);
         for (size_t f = 0; f < N; ++f) {
             const double wr = g->waveform_fft ? g->waveform_fft[2 * f] : 1.0, wi = g->waveform_fft ? g->waveform_fft[2 * f + 1] : 0.0;
-            fw[f] = make_float2((float)(wr * inv_c[f]), (float)(wi * inv_c[f]));
+            fw64[f] = make_double2(wr * inv_c[f], wi * inv_c[f]);
+            fw[f] = make_float2((float)fw64[f].x, (float)fw64[f].y);
             const double k = f < N - N / 2 ? (double)f : (double)f - (double)N, angle = 3.14159265358979323846 * k / (double)N;
             half[f] = make_float2((float)std::cos(angle), (float)std::sin(angle));
         }
@@ -902,8 +911,17 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         SAR_CUDA(cudaMemcpy(p->d_taps, taps.data(), sizeof(float) * taps.size(), cudaMemcpyHostToDevice), "filter taps");
         SAR_CUDA(cudaMemcpy(p->d_pair_taps, pair_taps.data(), sizeof(float) * pair_taps.size(), cudaMemcpyHostToDevice),
                  "filter taps");
+        if (p->fft_double) {
+            if ((rc = p->alloc(&p->d_fir_wave64, N, "waveform"))) return rc;
+            if ((rc = p->alloc(&p->d_taps64, taps64.size(), "filter taps"))) return rc;
+            if ((rc = p->alloc(&p->d_pair_taps64, pair_taps64.size(), "filter taps"))) return rc;
+            SAR_CUDA(cudaMemcpy(p->d_fir_wave64, fw64.data(), sizeof(double2) * N, cudaMemcpyHostToDevice), "waveform");
+            SAR_CUDA(cudaMemcpy(p->d_taps64, taps64.data(), sizeof(double) * taps64.size(), cudaMemcpyHostToDevice), "filter taps");
+            SAR_CUDA(cudaMemcpy(p->d_pair_taps64, pair_taps64.data(), sizeof(double) * pair_taps64.size(), cudaMemcpyHostToDevice),
+                     "filter taps");
+        }
     }
-    if (!p->fir || !p->fir_layout.fused) {
+    if (!p->fir || !p->fir_layout.fused || p->fft_double) {
         double2* spec = nullptr;
         if ((rc = p->alloc(&spec, ((size_t)p->chunk * p->fft_len * elem + sizeof(double2) - 1) / sizeof(double2), "FFT rows")))
             return rc;
@@ -923,7 +941,10 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
     const bool up_ok = !p->fir && upsample_fused_supported((int)N, (long)M, p->Lg);
     const bool down_ok = !p->fir && downsample_fused_supported((int)N, (long)M, p->Lg);
     p->fused_up = p->fused_down = p->fir && p->fir_layout.fused;
-    if (p->fused_up) {
+    // The fused kernels are FP32: at such lengths M the upsampling takes them only for spans that the U transforms of N
+    // points, FP32 as well, fit.
+    if (p->fft_double) p->fused_up = p->fused_up && upsample_fused_supported((int)N, (long)M, p->Lg);
+    if (p->fused_up || p->fused_down) {
         std::vector<float2> tn(N);
         const double two_pi = 6.283185307179586476925286766559;
         for (size_t q = 0; q < N; ++q)
@@ -1098,6 +1119,8 @@ static FirArgs fir_args(const sar_plan* p, int first) {
     a.tw_n = p->d_tw_n;
     a.taps = p->d_taps;
     a.pair_taps = p->d_pair_taps;
+    a.taps64 = p->d_taps64;
+    a.pair_taps64 = p->d_pair_taps64;
     a.Lg = p->Lg;
     a.first = first;
     return a;
@@ -1118,11 +1141,13 @@ static int upsample_rows(sar_plan* p, const float2* y, size_t begin, size_t end,
             a.wfac = pairs_out ? p->d_wadj : nullptr;
             a.prof = pairs_out ? (void*)pairs_rows : (void*)prof;
             a.format = pairs_out ? prof_format(p) : kProfValues;
-            if (p->fir_layout.fused) {
+            if (p->fused_up && (pairs_out || !dbl)) {
                 SAR_CUDA(launch_fir_fused(a, p->fir_layout, rows, true, st), "fused upsampling");
                 continue;
             }
-            SAR_CUDA(launch_pack_adjoint(y, p->d_fir_wave, p->d_spec, dbl, (int)p->N, p->fft_len, rows, (int)first, st), "pack");
+            SAR_CUDA(dbl ? launch_pack_adjoint(y, p->d_fir_wave64, (double2*)p->d_spec, (int)p->N, p->fft_len, rows, (int)first, st)
+                         : launch_pack_adjoint(y, p->d_fir_wave, p->d_spec, 0, (int)p->N, p->fft_len, rows, (int)first, st),
+                     "pack");
             int rc = run_fft(p, p->d_spec, rows, CUFFT_INVERSE, st);
             if (rc) return rc;
             SAR_CUDA(launch_fir_rows(p->d_spec, dbl, a, p->fir_layout, rows, st), "upsampling filter");
@@ -1363,15 +1388,17 @@ static int downsample_rows(sar_plan* p, const float2* acc_rows, float2* y, size_
             a.acc = acc_rows;
             a.y_out = y;
             a.wfac = p->d_wfwd;
-            if (p->fir_layout.fused) {
+            if (p->fused_down) {
                 SAR_CUDA(launch_fir_fused(a, p->fir_layout, rows, false, st), "fused downsampling");
                 continue;
             }
             SAR_CUDA(launch_fir_fold(p->d_spec, p->fft_double, a, p->fir_layout, rows, st), "downsampling filter");
             int rc = run_fft(p, p->d_spec, rows, CUFFT_FORWARD, st);
             if (rc) return rc;
-            SAR_CUDA(launch_extract_forward(p->d_spec, p->fft_double, p->d_fir_wave, p->d_wfwd, y, (int)p->N, p->fft_len, rows,
-                                            (int)first, st),
+            SAR_CUDA(p->fft_double ? launch_extract_forward((const double2*)p->d_spec, p->d_fir_wave64, p->d_wfwd, y, (int)p->N,
+                                                            p->fft_len, rows, (int)first, st)
+                                   : launch_extract_forward(p->d_spec, 0, p->d_fir_wave, p->d_wfwd, y, (int)p->N, p->fft_len,
+                                                            rows, (int)first, st),
                      "extract");
             continue;
         }

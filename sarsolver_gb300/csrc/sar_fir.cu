@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "sar_fir.cuh"
 #include "sar_kernels.cuh"
@@ -50,6 +51,17 @@ __device__ __forceinline__ void copies_done() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 __device__ __forceinline__ float2 conj_of(float2 a) { return make_float2(a.x, -a.y); }
+// Complex64 rows are filtered in FP32, complex128 rows in FP64.
+template <class R>
+using Cplx = typename std::conditional<std::is_same<R, double>::value, double2, float2>::type;
+__device__ __forceinline__ float2 mad(float h, float2 z, float2 s) { return __ffma2_rn(dup(h), z, s); }
+__device__ __forceinline__ double2 mad(double h, double2 z, double2 s) { return make_double2(fma(h, z.x, s.x), fma(h, z.y, s.y)); }
+__device__ __forceinline__ float2 wide(float2 v, float) { return v; }
+__device__ __forceinline__ double2 wide(float2 v, double) { return make_double2(v.x, v.y); }
+template <class T>
+__device__ __forceinline__ T times(T c, float2 f) {
+    return T{c.x * f.x - c.y * f.y, c.x * f.y + c.y * f.x};
+}
 
 // Transforms of a row side by side: two up to N = 2048, which halves a row's chain of passes; from 4096
 // on one after the other, so that two CTAs share an SM and one's loads overlap the other's passes
@@ -70,8 +82,8 @@ struct FirShape {
 // consecutive groups with the ten (linear pairs: eleven) samples in registers: one shared-memory
 // load and 10 (22) packed FMAs per bin.  Consecutive threads take consecutive phases, so loads are
 // broadcast and the stores of a warp contiguous for H >= 32.
-template <bool PAIRS>
-__device__ __forceinline__ void fir_walk(const float2* z, const float* __restrict__ taps, int H, int gbeg, int gend,
+template <bool PAIRS, class R>
+__device__ __forceinline__ void fir_walk(const Cplx<R>* z, const R* __restrict__ taps, int H, int gbeg, int gend,
                                          int w0, int Lg, int format, float4* dst, float2* vdst, int tid, int nt) {
     constexpr int W = PAIRS ? kFirTaps + 1 : kFirTaps;
     const int ch = max(1, nt / H), len = (gend - gbeg + ch - 1) / ch;
@@ -79,14 +91,14 @@ __device__ __forceinline__ void fir_walk(const float2* z, const float* __restric
         const int q = item % H, c = item / H;
         const int a = gbeg + c * len, b = min(gend, a + len);
         if (a >= b) continue;
-        const float* row = taps + (size_t)q * (PAIRS ? 2 * kFirRow : kFirRow);
-        float h[W], d[W];
+        const R* row = taps + (size_t)q * (PAIRS ? 2 * kFirRow : kFirRow);
+        R h[W], d[W];
 #pragma unroll
         for (int t = 0; t < W; ++t) {
             h[t] = __ldg(row + t);
-            d[t] = PAIRS ? __ldg(row + kFirRow + t) : 0.f;
+            d[t] = PAIRS ? __ldg(row + kFirRow + t) : R(0);
         }
-        float2 zw[W];
+        Cplx<R> zw[W];
 #pragma unroll
         for (int t = 0; t < W - 1; ++t) zw[t] = z[a + t];
         for (int g = a; g < b; g += W) {
@@ -94,39 +106,52 @@ __device__ __forceinline__ void fir_walk(const float2* z, const float* __restric
             for (int j = 0; j < W; ++j) {
                 if (g + j >= b) break;
                 zw[(j + W - 1) % W] = z[g + j + W - 1];
-                float2 s = make_float2(0.f, 0.f), e = s;
+                Cplx<R> s{0, 0}, e{0, 0};
 #pragma unroll
                 for (int t = 0; t < W; ++t) {
-                    s = __ffma2_rn(dup(h[t]), zw[(j + t) % W], s);
-                    if (PAIRS) e = __ffma2_rn(dup(d[t]), zw[(j + t) % W], e);
+                    s = mad(h[t], zw[(j + t) % W], s);
+                    if (PAIRS) e = mad(d[t], zw[(j + t) % W], e);
                 }
                 const int w = (g + j) * H + q - w0;
                 if (w < 0 || w >= Lg) continue;
                 if (PAIRS)
-                    dst[w] = make_float4(s.x, s.y, e.x, e.y);
+                    dst[w] = make_float4((float)s.x, (float)s.y, (float)e.x, (float)e.y);
                 else if (format == kProfValues)
-                    vdst[w] = s;
+                    vdst[w] = make_float2((float)s.x, (float)s.y);
                 else
-                    dst[w] = make_float4(s.x, s.y, 0.f, 0.f);
+                    dst[w] = make_float4((float)s.x, (float)s.y, 0.f, 0.f);
             }
         }
     }
 }
 
-__device__ __forceinline__ void fir_write(const float2* z, const FirArgs& a, int gbeg, int gend, long row, int tid,
-                                          int nt) {
+template <class R>
+__device__ __forceinline__ void fir_write(const Cplx<R>* z, const R* taps, const R* pair_taps, const FirArgs& a, int gbeg,
+                                          int gend, long row, int tid, int nt) {
     float4* dst = reinterpret_cast<float4*>(a.prof) + row * a.Lg;
     float2* vdst = reinterpret_cast<float2*>(a.prof) + row * a.Lg;
     if (a.format == kProfLinearPairs)
-        fir_walk<true>(z, a.pair_taps, a.H, gbeg, gend, a.w0, a.Lg, a.format, dst, vdst, tid, nt);
+        fir_walk<true, R>(z, pair_taps, a.H, gbeg, gend, a.w0, a.Lg, a.format, dst, vdst, tid, nt);
     else
-        fir_walk<false>(z, a.taps, a.H, gbeg, gend, a.w0, a.Lg, a.format, dst, vdst, tid, nt);
+        fir_walk<false, R>(z, taps, a.H, gbeg, gend, a.w0, a.Lg, a.format, dst, vdst, tid, nt);
 }
 
 // Index of fine value e of a staged fold chunk: PS slots of padding per four groups, so that the
 // lanes of a half-warp (16 / PS base samples four groups apart, PS phases each) fall on distinct banks.
 __device__ __forceinline__ int fold_pad(int e, int H, int hshift, int PS) {
     return e + (hshift >= 0 ? e >> (hshift + 2) : e / (4 * H)) * PS;
+}
+
+// The ten taps of a phase: FP32 from shared memory, FP64 (whose sums take far longer than the loads) from the table.
+__device__ __forceinline__ void tap_row(const float4* taps, int p, float (&h)[kFirTaps]) {
+    const float4 *hr = taps + p * (kFirRow / 4), h0 = hr[0], h1 = hr[1], h2 = hr[2];
+    const float v[kFirTaps] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w, h2.x, h2.y};
+#pragma unroll
+    for (int t = 0; t < kFirTaps; ++t) h[t] = v[t];
+}
+__device__ __forceinline__ void tap_row(const double* taps, int p, double (&h)[kFirTaps]) {
+#pragma unroll
+    for (int t = 0; t < kFirTaps; ++t) h[t] = __ldg(taps + (size_t)p * kFirRow + t);
 }
 
 // The tap table into shared memory (the caller's next barrier publishes it).
@@ -137,10 +162,10 @@ __device__ __forceinline__ void load_taps(float4* taps, const FirArgs& a, int ti
 // Base samples i0 .. i0 + gc - 1 (gc a multiple of 4; sample i is base point gb0 - 4 + i) folded from
 // the fine bins of one accumulator row: z(i) = sum_{t, q} h_q(t) acc(group i - t, bin q).  A thread
 // owns four consecutive samples and every PS-th phase: 13 loads feed 40 packed FMAs, and the PS
-// partial sums are added with shuffles.  `buf` holds the chunk's bins, `taps` the tap table (shared
-// memory; eight rows of 48 bytes fall on distinct banks); every thread of the CTA calls.
-template <class STORE>
-__device__ __forceinline__ void fir_fold(const float2* __restrict__ arow, float2* buf, const float4* taps, const FirArgs& a,
+// partial sums are added with shuffles.  `buf` holds the chunk's bins, `taps` the tap table (FP32: shared
+// memory, where eight rows of 48 bytes fall on distinct banks); every thread of the CTA calls.
+template <class R, class TAPS, class STORE>
+__device__ __forceinline__ void fir_fold(const float2* __restrict__ arow, float2* buf, TAPS taps, const FirArgs& a,
                                          int i0, int gc, int tid, int nt, STORE store) {
     const int H = a.H, PS = a.fold_phases;
     const int first = (i0 - (kFirTaps - 1)) * H - a.w0, count = (gc + kFirTaps - 1) * H;
@@ -155,22 +180,21 @@ __device__ __forceinline__ void fir_fold(const float2* __restrict__ arow, float2
     for (int item = tid; item < ((items + 31) & ~31); item += nt) {
         const bool live = item < items;
         const int sb = live ? item / PS : 0, q = item & (PS - 1);
-        float2 o[4];
+        Cplx<R> o[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < 4; ++k) o[k] = Cplx<R>{0, 0};
         if (live)
             for (int p = q; p < H; p += PS) {
-                const float4* hr = taps + p * (kFirRow / 4);
-                const float4 h0 = hr[0], h1 = hr[1], h2 = hr[2];
-                const float h[kFirTaps] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w, h2.x, h2.y};
+                R h[kFirTaps];
+                tap_row(taps, p, h);
                 const float2* b = buf + sb * stride + p;
 #pragma unroll
                 for (int gg = 0; gg < kFirTaps + 3; ++gg) {
-                    const float2 v = b[gg * H + (gg >> 2) * PS];
+                    const Cplx<R> v = wide(b[gg * H + (gg >> 2) * PS], R(0));
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const int t = k + kFirTaps - 1 - gg;
-                        if (t >= 0 && t < kFirTaps) o[k] = __ffma2_rn(dup(h[t]), v, o[k]);
+                        if (t >= 0 && t < kFirTaps) o[k] = mad(h[t], v, o[k]);
                     }
                 }
             }
@@ -230,7 +254,7 @@ __global__ void __launch_bounds__(FirShape<N>::NT, FirShape<N>::CTAS) fir_up_ker
         }
         __syncthreads();
     }
-    fir_write(stage, a, 0, a.groups, s, tid, NT);
+    fir_write<float>(stage, a.taps, a.pair_taps, a, 0, a.groups, s, tid, NT);
 }
 
 // K4, N = 512 ... 8192: accumulator row -> phase-history row, the transpose of fir_up_kernel.
@@ -250,7 +274,7 @@ __global__ void __launch_bounds__(FirShape<N>::NT, FirShape<N>::CTAS) fir_down_k
     load_taps(taps, a, tid, NT);
     for (int i0 = 0; i0 < nb; i0 += a.fold_chunk) {
         const int gc = min(a.fold_chunk, (nb - i0 + 3) & ~3);
-        fir_fold(arow, fsm, taps, a, i0, gc, tid, NT, [&](int i, float2 v) { z[i] = v; });
+        fir_fold<float>(arow, fsm, taps, a, i0, gc, tid, NT, [&](int i, float2 v) { z[i] = v; });
         __syncthreads();
     }
     float2 acc[16];
@@ -297,18 +321,16 @@ __global__ void __launch_bounds__(FirShape<N>::NT, FirShape<N>::CTAS) fir_down_k
     }
 }
 
-__device__ __forceinline__ float2 spec_f2(float2 v) { return v; }
-__device__ __forceinline__ float2 spec_f2(double2 v) { return make_float2((float)v.x, (float)v.y); }
-__device__ __forceinline__ void spec_set(float2* p, float2 v) { *p = v; }
-__device__ __forceinline__ void spec_set(double2* p, float2 v) { *p = make_double2(v.x, v.y); }
-
 constexpr int kFirThreads = 256;
 
 // Any N: the filter from transformed rows spec[row][2 N] (float2, or double2) to the stored span; grid
-// (chunks of fold_chunk groups, rows).
+// (chunks of groups, rows).  The FP64 form, taken where the transform itself is complex128, is bound by the FP64 pipe
+// (two operations a cycle and SM): 1500 x 1999, U = 128, 51860 bins a row: 5.8 ms up and 7.5 ms down with the
+// transforms, of which FP64 filters 2.8 and 4.5; transforms of length M took 293 ms.
 template <class T>
 __global__ void __launch_bounds__(kFirThreads) fir_rows_kernel(const T* __restrict__ spec, const FirArgs a, int chunk) {
-    extern __shared__ __align__(16) float2 fsm[];
+    extern __shared__ __align__(16) unsigned char rsm[];
+    T* zs = reinterpret_cast<T*>(rsm);
     const long s = (long)a.first + blockIdx.y;
     const int g0 = blockIdx.x * chunk, g1 = min(a.groups, g0 + chunk);
     const float2 f = a.wfac ? __ldg(a.wfac + s) : make_float2(1.f, 0.f);
@@ -316,11 +338,13 @@ __global__ void __launch_bounds__(kFirThreads) fir_rows_kernel(const T* __restri
     for (int i = threadIdx.x; i < g1 - g0 + kFirTaps; i += kFirThreads) {
         int n = a.base0 + g0 + i;
         if (n >= a.base_len) n -= a.base_len;
-        const float2 c = spec_f2(row[n]);
-        fsm[i] = make_float2(c.x * f.x - c.y * f.y, c.x * f.y + c.y * f.x);
+        zs[i] = times(row[n], f);
     }
     __syncthreads();
-    fir_write(fsm - g0, a, g0, g1, s, threadIdx.x, kFirThreads);
+    if constexpr (std::is_same<T, double2>::value)
+        fir_write<double>(zs - g0, a.taps64, a.pair_taps64, a, g0, g1, s, threadIdx.x, kFirThreads);
+    else
+        fir_write<float>(zs - g0, a.taps, a.pair_taps, a, g0, g1, s, threadIdx.x, kFirThreads);
 }
 
 // Any N: the fold of an accumulator row onto rows spec[row][2 N], zero outside the span.
@@ -330,19 +354,23 @@ __global__ void __launch_bounds__(kFirThreads) fir_fold_kernel(T* __restrict__ s
     const long s = (long)a.first + blockIdx.y;
     const int nb = a.groups + kFirTaps - 1, i0 = blockIdx.x * a.fold_chunk;
     T* row = spec + (size_t)blockIdx.y * a.base_len;
-    auto put = [&](int i, float2 v) {
+    auto put = [&](int i, T v) {
         if (i >= a.base_len) return;
         int n = a.base0 + i;
         if (n >= a.base_len) n -= a.base_len;
-        spec_set(row + n, v);
+        row[n] = v;
     };
     if (i0 < nb) {
-        float4* taps = reinterpret_cast<float4*>(fsm + a.fold_buf);
-        load_taps(taps, a, threadIdx.x, kFirThreads);
-        fir_fold(a.acc + s * a.Lg, fsm, taps, a, i0, a.fold_chunk, threadIdx.x, kFirThreads, put);
+        if constexpr (std::is_same<T, double2>::value) {
+            fir_fold<double>(a.acc + s * a.Lg, fsm, a.taps64, a, i0, a.fold_chunk, threadIdx.x, kFirThreads, put);
+        } else {
+            float4* taps = reinterpret_cast<float4*>(fsm + a.fold_buf);
+            load_taps(taps, a, threadIdx.x, kFirThreads);
+            fir_fold<float>(a.acc + s * a.Lg, fsm, taps, a, i0, a.fold_chunk, threadIdx.x, kFirThreads, put);
+        }
         return;
     }
-    for (int i = i0 + threadIdx.x; i < i0 + a.fold_chunk; i += kFirThreads) put(i, make_float2(0.f, 0.f));
+    for (int i = i0 + threadIdx.x; i < i0 + a.fold_chunk; i += kFirThreads) put(i, T{0, 0});
 }
 
 // ------------------------------------------------------------------ host side
@@ -423,7 +451,7 @@ bool fir_plan(long N, long M, int Lg, long bg0, FirLayout* L) {
     return true;
 }
 
-void fir_tables(const FirLayout& L, std::vector<float>* taps, std::vector<float>* pair_taps, std::vector<double>* inv_c) {
+void fir_tables(const FirLayout& L, std::vector<double>* taps, std::vector<double>* pair_taps, std::vector<double>* inv_c) {
     const int W = kFirTaps, H = L.H;
     const double pi = 3.14159265358979323846;
     // the usual shape parameter of a Kaiser-Bessel window of width W on a grid oversampled twice
@@ -435,14 +463,14 @@ void fir_tables(const FirLayout& L, std::vector<float>* taps, std::vector<float>
     std::vector<double> h((size_t)(H + 1) * (W + 1), 0.0);   // [q][t]; q = H is phase 0 one sample on
     for (int q = 0; q <= H; ++q)
         for (int t = 0; t <= W; ++t) h[(size_t)q * (W + 1) + t] = psi((double)q / H + 4.0 - t);
-    taps->assign((size_t)H * kFirRow, 0.f);
-    pair_taps->assign((size_t)H * 2 * kFirRow, 0.f);
+    taps->assign((size_t)H * kFirRow, 0.0);
+    pair_taps->assign((size_t)H * 2 * kFirRow, 0.0);
     for (int q = 0; q < H; ++q)
         for (int t = 0; t <= W; ++t) {
             const double a = h[(size_t)q * (W + 1) + t], b = h[(size_t)(q + 1) * (W + 1) + t];
-            if (t < W) (*taps)[(size_t)q * kFirRow + t] = (float)a;
-            (*pair_taps)[(size_t)(2 * q) * kFirRow + t] = (float)(0.5 * (a + b));
-            (*pair_taps)[(size_t)(2 * q + 1) * kFirRow + t] = (float)(b - a);
+            if (t < W) (*taps)[(size_t)q * kFirRow + t] = a;
+            (*pair_taps)[(size_t)(2 * q) * kFirRow + t] = 0.5 * (a + b);
+            (*pair_taps)[(size_t)(2 * q + 1) * kFirRow + t] = b - a;
         }
     // 1 / c(k) at FFT index i of N: the window's Fourier transform at k / (2 N) cycles per base sample
     const int N = L.base_len / 2;
@@ -496,7 +524,7 @@ cudaError_t launch_fir_rows(const void* spec, int dbl, const FirArgs& args, cons
     const FirArgs a = with_layout(args, L);
     const int chunk = std::max(32, 4096 / L.H);   // groups per CTA
     const dim3 grid((unsigned)((L.groups + chunk - 1) / chunk), (unsigned)rows);
-    const size_t smem = (size_t)(chunk + kFirTaps + 1) * sizeof(float2);
+    const size_t smem = (size_t)(chunk + kFirTaps + 1) * (dbl ? sizeof(double2) : sizeof(float2));
     if (dbl)
         fir_rows_kernel<<<grid, kFirThreads, smem, st>>>((const double2*)spec, a, chunk);
     else

@@ -36,6 +36,8 @@ struct FirArgs {
     const float2* wfac = nullptr;   // [S] pulse factors; null: 1 (upsampling)
     const float* taps = nullptr;        // [H][kFirRow]
     const float* pair_taps = nullptr;   // [H][2][kFirRow]: mid-bin value, difference to the next bin
+    const double* taps64 = nullptr;     // the same in 64 bits (complex128 rows)
+    const double* pair_taps64 = nullptr;
     const float2* acc = nullptr;    // [S][Lg] accumulator (downsampling)
     void* prof = nullptr;           // [S][Lg] profiles in `format` (upsampling)
     int Lg = 0, first = 0, format = 0;   // row of the launch's first CTA; kProf... format
@@ -50,10 +52,11 @@ __host__ __device__ constexpr int up_pad_count(int n) { return n + n / 16; }
 // shorter than the grid.
 bool fir_plan(long N, long M, int Lg, long bg0, FirLayout* L);
 // FP64-made tables: taps, pair taps and 1 / c(k) in FFT order.
-void fir_tables(const FirLayout& L, std::vector<float>* taps, std::vector<float>* pair_taps, std::vector<double>* inv_c);
+void fir_tables(const FirLayout& L, std::vector<double>* taps, std::vector<double>* pair_taps, std::vector<double>* inv_c);
 // Fused kernels for `rows` pulses from args.first (rows addressed absolutely, as sar_kernels.cuh's).
 cudaError_t launch_fir_fused(const FirArgs& a, const FirLayout& L, int rows, bool up, cudaStream_t st);
-// The filters alone, between transforms of length 2 N: spec rows [rows][2 N] of complex64 / complex128.
+// The filters alone, between transforms of length 2 N: spec rows [rows][2 N] of complex64, or of complex128, which are
+// filtered in FP64 and rounded once.
 cudaError_t launch_fir_rows(const void* spec, int dbl, const FirArgs& a, const FirLayout& L, int rows, cudaStream_t st);
 cudaError_t launch_fir_fold(void* spec, int dbl, const FirArgs& a, const FirLayout& L, int rows, cudaStream_t st);
 

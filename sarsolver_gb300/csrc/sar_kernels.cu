@@ -1671,8 +1671,8 @@ __device__ __forceinline__ double2 make_spec<double2>(float x, float y) { return
 
 // spec[row][m] = conj(W[i]) y_fft[i] placed at the zero-padded position of FFT index i
 // (sarsolver_cxx.cpp:331-342); y is read from its fftshifted layout.
-template <class T>
-__global__ void pack_adjoint_kernel(const float2* __restrict__ y, const float2* __restrict__ wave,
+template <class T, class W>
+__global__ void pack_adjoint_kernel(const float2* __restrict__ y, const W* __restrict__ wave,
                                     T* __restrict__ spec, int N, long M, int first) {
     const long m = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
@@ -1685,13 +1685,13 @@ __global__ void pack_adjoint_kernel(const float2* __restrict__ y, const float2* 
         i = (int)(N - M + m);
     else if ((N & 1) && m == half)
         i = half;
-    float2 v = make_float2(0.f, 0.f);
+    W v{0, 0};
     if (i >= 0) {
         const float2 yv = y[(size_t)(first + row) * N + (i + half) % N];
-        const float2 w = __ldg(wave + i);
-        v = make_float2(w.x * yv.x + w.y * yv.y, w.x * yv.y - w.y * yv.x);
+        const W w = __ldg(wave + i);
+        v = W{w.x * yv.x + w.y * yv.y, w.x * yv.y - w.y * yv.x};
     }
-    spec[row * M + m] = make_spec<T>(v.x, v.y);
+    spec[row * M + m] = T{v.x, v.y};
 }
 
 // pairs[s][w] for bin b = bg0 + w by `format` (kProfPairs...): linear, (p(b) + 0.5 d, d) with
@@ -1790,8 +1790,8 @@ __global__ void pack_forward_kernel(const float2* __restrict__ acc, T* __restric
 
 // y_fft[i] = W[i] K[i] (low half), W[N-1-i] K[M-1-i] (high half), odd middle
 // (sarsolver_cxx.cpp:295-307), times the pulse factor, written fftshifted (forward.py:44).
-template <class T>
-__global__ void extract_forward_kernel(const T* __restrict__ spec, const float2* __restrict__ wave,
+template <class T, class W>
+__global__ void extract_forward_kernel(const T* __restrict__ spec, const W* __restrict__ wave,
                                        const float2* __restrict__ wfac, float2* __restrict__ y, int N, long M,
                                        int first) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1805,10 +1805,14 @@ __global__ void extract_forward_kernel(const T* __restrict__ spec, const float2*
         m = M - N + i;
     else
         m = half;
-    const float2 k = to_f2(spec[row * M + m]);
-    const float2 w = __ldg(wave + i);
+    W k;   // products in the waveform's precision
+    if constexpr (std::is_same<W, double2>::value)
+        k = spec[row * M + m];
+    else
+        k = to_f2(spec[row * M + m]);
+    const W w = __ldg(wave + i);
     const float2 f = __ldg(wfac + first + row);
-    const float2 a = make_float2(w.x * k.x - w.y * k.y, w.x * k.y + w.y * k.x);
+    const float2 a = make_float2((float)(w.x * k.x - w.y * k.y), (float)(w.x * k.y + w.y * k.x));
     y[(size_t)(first + row) * N + (i + half) % N] = make_float2(a.x * f.x - a.y * f.y, a.x * f.y + a.y * f.x);
 }
 
@@ -1896,9 +1900,16 @@ cudaError_t launch_pack_adjoint(const float2* y, const float2* wave, void* spec,
                                 int first, cudaStream_t st) {
     const dim3 grid((unsigned)((M + 255) / 256), (unsigned)rows);
     if (dbl)
-        pack_adjoint_kernel<double2><<<grid, 256, 0, st>>>(y, wave, (double2*)spec, N, M, first);
+        pack_adjoint_kernel<<<grid, 256, 0, st>>>(y, wave, (double2*)spec, N, M, first);
     else
-        pack_adjoint_kernel<float2><<<grid, 256, 0, st>>>(y, wave, (float2*)spec, N, M, first);
+        pack_adjoint_kernel<<<grid, 256, 0, st>>>(y, wave, (float2*)spec, N, M, first);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pack_adjoint(const float2* y, const double2* wave, double2* spec, int N, long M, int rows, int first,
+                                cudaStream_t st) {
+    const dim3 grid((unsigned)((M + 255) / 256), (unsigned)rows);
+    pack_adjoint_kernel<<<grid, 256, 0, st>>>(y, wave, spec, N, M, first);
     return cudaGetLastError();
 }
 
@@ -2207,9 +2218,16 @@ cudaError_t launch_extract_forward(const void* spec, int dbl, const float2* wave
                                    int N, long M, int rows, int first, cudaStream_t st) {
     const dim3 grid((unsigned)((N + 255) / 256), (unsigned)rows);
     if (dbl)
-        extract_forward_kernel<double2><<<grid, 256, 0, st>>>((const double2*)spec, wave, wfac, y, N, M, first);
+        extract_forward_kernel<<<grid, 256, 0, st>>>((const double2*)spec, wave, wfac, y, N, M, first);
     else
-        extract_forward_kernel<float2><<<grid, 256, 0, st>>>((const float2*)spec, wave, wfac, y, N, M, first);
+        extract_forward_kernel<<<grid, 256, 0, st>>>((const float2*)spec, wave, wfac, y, N, M, first);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_extract_forward(const double2* spec, const double2* wave, const float2* wfac, float2* y, int N, long M,
+                                   int rows, int first, cudaStream_t st) {
+    const dim3 grid((unsigned)((N + 255) / 256), (unsigned)rows);
+    extract_forward_kernel<<<grid, 256, 0, st>>>(spec, wave, wfac, y, N, M, first);
     return cudaGetLastError();
 }
 

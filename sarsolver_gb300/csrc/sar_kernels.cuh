@@ -120,6 +120,9 @@ cudaError_t launch_fp_points(const PointArgs& a, const float2* x, float2* acc, c
 // complex64, or complex128 when dbl != 0.
 cudaError_t launch_pack_adjoint(const float2* y, const float2* wave, void* spec, int dbl, int N, long M, int rows,
                                 int first, cudaStream_t st);
+// The same into complex128 rows with an FP64 waveform.
+cudaError_t launch_pack_adjoint(const float2* y, const double2* wave, double2* spec, int N, long M, int rows, int first,
+                                cudaStream_t st);
 cudaError_t launch_unpack_compact(const float2* compact, int Lc, const float2* wfac, float4* pairs, float2* prof,
                                   long M, int Lg, int rows, int first, int linear, cudaStream_t st);
 // Fused adjoint upsampling for N = 512, 1024, 2048, 4096 or 8192 and M a multiple of N: pairs over the stored span straight
@@ -145,6 +148,8 @@ cudaError_t launch_pack_forward(const float2* acc, void* spec, int dbl, long M, 
                                 cudaStream_t st);
 cudaError_t launch_extract_forward(const void* spec, int dbl, const float2* wave, const float2* wfac, float2* y,
                                    int N, long M, int rows, int first, cudaStream_t st);
+cudaError_t launch_extract_forward(const double2* spec, const double2* wave, const float2* wfac, float2* y, int N, long M,
+                                   int rows, int first, cudaStream_t st);
 cudaError_t launch_phase_grad(const float2* ag, const float2* y, float* g, int S, int N, float scale,
                               cudaStream_t st);
 cudaError_t launch_sharpness(const float2* img, float2* G, double* sum, size_t P, int num_sms, cudaStream_t st);

@@ -113,7 +113,9 @@ typedef struct sar_plan_info {
     size_t working_length;      /* M = (size_t)(upsample_ratio * N), sarsolver_cxx.cpp:223 */
     long profile_first_bin;     /* first stored range bin (may be negative) */
     size_t profile_length;      /* stored bins per pulse */
-    size_t tile_window;         /* staged bins per (tile, pulse); 0 on the unstructured path */
+    size_t tile_window;         /* staged bins per (tile, pulse) of the tile kernel of the backprojection, which
+                                   serves the plans without a gather lattice (sar_plan_get_lattices); 0 on the
+                                   unstructured path */
     size_t strip_window;        /* forward window (bins) of a strip or ring, or of a lane of the lattice
                                    scatter; 0 on the unstructured path */
     size_t device_bytes;        /* device memory held by the plan */
@@ -161,6 +163,14 @@ int sar_plan_create(const sar_geometry *geom, int device, sar_plan **plan_out);
 int sar_plan_create_streamed(const sar_geometry *geom, int device, size_t block_pulses, sar_plan **plan_out);
 int sar_plan_destroy(sar_plan *plan);
 int sar_plan_get_info(const sar_plan *plan, sar_plan_info *info);
+
+/* Pixel lattices of the kernels that walk along iso-range lines: lattice pixel (a, b) is image pixel a v + b w (x, y);
+ * threads walk along w.  window: bins staged per pulse; 0 where the plan runs the tile or unstructured kernels. */
+typedef struct sar_plan_lattice {
+    int v[2], w[2];
+    int window;
+} sar_plan_lattice;
+int sar_plan_get_lattices(const sar_plan *plan, sar_plan_lattice *gather, sar_plan_lattice *scatter);
 
 /* y[S][N] = A x[P].  Device complex64 buffers; asynchronous on `stream`. */
 int sar_forward(sar_plan *plan, const void *x_dev, void *y_dev, void *stream);

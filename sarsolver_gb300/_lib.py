@@ -24,7 +24,7 @@ PATH = {"auto": 0, "grid": 1, "points": 2}
 #: Every function include/sargpu.h declares.
 EXPORTED = (
     "forward_evaluate", "adjoint_evaluate",
-    "sar_plan_create", "sar_plan_destroy", "sar_plan_get_info",
+    "sar_plan_create", "sar_plan_destroy", "sar_plan_get_info", "sar_plan_get_lattices",
     "sar_forward", "sar_adjoint", "sar_profiles",
     "sar_set_slow_time_weighting", "sar_set_slow_time_weighting_device",
     "sar_device_flags", "sar_last_error", "sar_status_string",
@@ -100,6 +100,12 @@ class SarPlanInfo(ctypes.Structure):
     ]
 
 
+class SarPlanLattice(ctypes.Structure):
+    """Mirror of ``sar_plan_lattice``."""
+
+    _fields_ = [("v", c_int * 2), ("w", c_int * 2), ("window", c_int)]
+
+
 class SarCalculationInfo(ctypes.Structure):
     """Byte-for-byte the reference struct (src/sarsolver/cxx_binding/sarsolver_cxx.hpp:28-33,
     mirrored in Python at src/sarsolver/cxx_binding/sarsolver_cxx.py:49-62)."""
@@ -133,6 +139,8 @@ def load() -> ctypes.CDLL:
     lib.sar_plan_create_streamed.restype = c_int
     lib.sar_plan_destroy.argtypes = [c_void_p]
     lib.sar_plan_get_info.argtypes = [c_void_p, POINTER(SarPlanInfo)]
+    lib.sar_plan_get_lattices.argtypes = [c_void_p, POINTER(SarPlanLattice), POINTER(SarPlanLattice)]
+    lib.sar_plan_get_lattices.restype = c_int
     for name in ("sar_forward", "sar_adjoint", "sar_profiles"):
         getattr(lib, name).argtypes = [c_void_p, c_void_p, c_void_p, c_void_p]
     lib.sar_set_slow_time_weighting.argtypes = [c_void_p, c_void_p]

@@ -1106,6 +1106,17 @@ int sar_plan_get_info(const sar_plan* p, sar_plan_info* info) {
     return SAR_OK;
 }
 
+int sar_plan_get_lattices(const sar_plan* p, sar_plan_lattice* gather, sar_plan_lattice* scatter) {
+    if (!p || !gather || !scatter) return fail(SAR_ERR_INVALID_ARGUMENT, "null argument");
+    auto put = [](sar_plan_lattice* out, bool ok, const Lattice& L, int window) {
+        *out = sar_plan_lattice{};
+        if (ok) *out = sar_plan_lattice{{L.vx, L.vy}, {L.wx, L.wy}, window};
+    };
+    put(gather, p->grid && p->gather.ok, p->gather.lattice, p->gather.ww);
+    put(scatter, p->grid && p->scatter.ok, p->scatter.lattice, p->scatter.slots);
+    return SAR_OK;
+}
+
 // Stored profile format of a plan (the upsampling writers' `linear` argument).
 static int prof_format(const sar_plan* p) {
     return p->values ? kProfValues : p->interp == SAR_INTERP_LINEAR ? kProfLinearPairs : kProfNearestPairs;

@@ -133,6 +133,11 @@ class SarPlan:
         self.scatter_shear = int(info.scatter_shear)
         self.gather_shear = int(info.gather_shear)
         self.scatter_ring_half = int(info.scatter_ring_half)
+        gather, scatter = _lib.SarPlanLattice(), _lib.SarPlanLattice()
+        _lib.check(lib.sar_plan_get_lattices(handle, ctypes.byref(gather), ctypes.byref(scatter)), "sar_plan_get_lattices")
+        # Steps (v, w) of the lattice along iso-range lines, or None: the tile or unstructured kernels run instead.
+        self.gather_lattice, self.scatter_lattice = (
+            (tuple(q.v), tuple(q.w)) if q.window else None for q in (gather, scatter))
         # The aperture's own weighting; phase corrections multiply it (autodiff.phase_weights).
         self.base_weights = torch.as_tensor(
             np.asarray(aperture.slow_time_weighting, dtype=np.complex64).reshape(-1)).to(self.device)

@@ -619,8 +619,14 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
         // across stay with them too: two partial sums per bin give the same bits in either order, so their
         // forward projections are reproducible, which the many small runs of the other scatter are not.
         if (p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins &&
-            (p->fwd_transposed ? p->gc_fwd.tiles_y : p->gc_fwd.tiles_x) > 2)
-            p->scatter = scatter_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa);
+            (p->fwd_transposed ? p->gc_fwd.tiles_y : p->gc_fwd.tiles_x) > 2) {
+            ScatterTiles t;
+            t.axes = p->fwd_transposed ? Lattice{0, 1, 1, 0, true} : Lattice{1, 0, shear, 1, true};
+            t.lines = p->fwd_transposed ? p->gc_fwd.tiles_y : p->gc_fwd.tiles_x;
+            t.along = p->fwd_transposed ? p->gc_fwd.tiles_x : p->gc_fwd.tiles_y;
+            t.cover = shear ? (1.0 + 32.0 / nx) * (1.0 + 32.0 / ny) : (double)t.lines * t.along * kTile * kTile / ((double)nx * ny);
+            p->scatter = scatter_layout(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, t);
+        }
         if (p->scatter.ok) {
             const ScatterLayout& L = p->scatter;
             double ea[3], eb[3];

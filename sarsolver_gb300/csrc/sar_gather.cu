@@ -551,11 +551,34 @@ namespace {
 
 constexpr size_t kPartialBytes = (size_t)256 << 20;   // partial images of a plan
 
-// Instructions per pixel-pulse by the bin rate along a line, for the choice of lattice only: by run length, and
-// with split bins by the spread of a half-warp's loads over the banks.
+// Split bins, for the choice of lattice only: instructions per pixel-pulse by the rate along a line, whose half-warps'
+// loads spread over the banks.
 double split_cost(double rate) { return 16.0 + std::min(rate, 8.0); }
-double run_cost(double rate) {
-    return 15.0 * rate < kRunSpan ? 14.0 : 7.0 * rate < kRunSpan ? 16.0 : 3.0 * rate < kRunSpan ? 20.0 : 26.0;
+
+// Bank pairs: the most distinct bins that a half-warp's loads have on one of the sixteen, its lanes `rate` bins apart.
+double bank_degree(double rate) {
+    int hits[16] = {}, last = -1, most = 0;
+    for (int l = 0; l < 16; ++l) {
+        const int bin = (int)std::min(rate * l, 1.0e6);
+        if (bin != last) most = std::max(most, ++hits[bin & 15]);
+        last = bin;
+    }
+    return most;
+}
+
+// Plain bins: seconds per pixel-pulse of a lattice on a full GPU, by run length; where each sample loads two bins, by the
+// bank conflicts of the lanes' loads.  Fitted to 380 geometries with every lattice forced in turn: 0.7 ps with runs of 16,
+// 0.95 without runs up to two bins a bank, then 1.3, 1.6 and 2.4 ps at three, four and five.
+double run_unit(const std::vector<LatticeRate>& rates) {
+    double sum = 0.0;
+    for (const LatticeRate& r : rates) {
+        const double run = 0.66 + 0.02 * std::min(r.v, 8.0);
+        sum += 15.0 * r.w < kRunSpan  ? run
+               : 7.0 * r.w < kRunSpan ? run + 0.06
+               : 3.0 * r.w < kRunSpan ? run + 0.14
+                                      : std::max(0.95, 0.2 + 0.42 * bank_degree(r.v));
+    }
+    return 1.0e-12 * sum / rates.size();
 }
 
 // Estimated seconds of `count` pulses over `tiles` tiles with `parts` CTAs each: whole waves of CTAs at 1.5e12
@@ -584,6 +607,66 @@ int best_parts(const GatherLayout& L, size_t tiles, size_t count, size_t pixels,
     return best;
 }
 
+// The same of a lattice's layout at `unit` seconds per pixel-pulse, plain bins: with fewer CTAs an SM than it holds, each
+// runs faster (one of two: 0.66 of the time).
+double lattice_seconds(const GatherLayout& L, size_t tiles, size_t count, size_t pixels, double unit) {
+    const size_t ctas = tiles * L.parts, slots = (size_t)152 * L.ctas, rest = ctas % slots;
+    const double last = rest ? std::pow((double)((rest + 151) / 152) / L.ctas, 0.6) : 0.0;
+    const double nst = std::ceil((double)count / L.pb), pulse = (double)kGatherLines * kGatherWalk * L.warps * unit;
+    return ((double)(ctas / slots) + last) * (std::ceil(nst / L.parts) + 1.0) * L.pb * pulse * slots +
+           (L.parts > 1 ? 2e-6 + 16.0 * pixels * L.parts / 5e12 : 0.0);
+}
+
+// The layout with the least estimate for a lattice; excursion(lines, walk): bins from a tile's mean to its pixels' (not a
+// number: no layout at all).  `tiles` of the result, and its tile list's shape, are those of `lines` x `walk` pixels.
+struct Shape {
+    GatherLayout layout;
+    int lines = 0, walk = 0;
+    size_t tiles = 0;
+};
+template <class EXCURSION>
+Shape best_shape(int bins, const Lattice& lattice, size_t S, int nx, int ny, int nz, EXCURSION excursion) {
+    const bool split = bins != GATHER_RUNS;
+    const size_t pixels = (size_t)nx * ny * nz;
+    const int most = (int)std::min<size_t>(16, std::max<size_t>(1, kPartialBytes / (pixels * sizeof(float2))));
+    Shape best;
+    double least = INFINITY;
+    for (int shape : {80, 81, 40, 41}) {   // warps, and the warps along the walk: 1 or 2 with split bins, else all
+        const int warps = shape / 10, along = split ? 1 + shape % 10 : warps, across = warps / along;
+        if (!split && shape % 10) continue;
+        const int lines = kGatherLines * across, walk = kGatherWalk * along;
+        // a tap from the excursion of the tile's pixels about its mean bin, plus the base's fraction and rounding
+        const double h = excursion(lines, walk) + 0.1;
+        if (std::isnan(h)) return Shape{};
+        if (!(h < 4096.0)) continue;
+        const int ww = 2 * (int)std::ceil(h + 3.5 + kDip);
+        size_t tiles = 0;
+        for (const LatticeStrip& t : lattice_strips(lattice, lines, nx, ny)) tiles += (size_t)((t.b1 - t.b0) / walk + 1) * nz;
+        for (int pb : {16, 8, 4, 2, 1}) {
+            if (!split && pb < 4) break;
+            const int full = warps == 8 ? 2 : 4;   // CTAs an SM: the registers' limit, and the shared memory's
+            const int ctas = std::min(full, (int)(227 * 1024 / (gather_smem(bins, warps, ww, pb).total + 1024)));
+            if (ctas < (split ? 1 : full)) continue;
+            GatherLayout L;
+            L.lattice = lattice;
+            L.bins = bins;
+            L.warps = warps;
+            L.across = across;
+            L.ctas = ctas;
+            L.ww = ww;
+            L.pb = pb;
+            L.ok = true;
+            double t;
+            L.parts = best_parts(L, tiles, S, pixels, most, &t);
+            if (t < 0.97 * least) {
+                least = t;
+                best = Shape{L, lines, walk, tiles};
+            }
+        }
+    }
+    return best;
+}
+
 }  // namespace
 
 int gather_parts(const GatherLayout& L, size_t count, size_t pixels) {
@@ -593,60 +676,42 @@ int gather_parts(const GatherLayout& L, size_t count, size_t pixels) {
 
 GatherLayout gather_layout(int bins, const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
                            const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa) {
-    GatherLayout best;
     const bool split = bins != GATHER_RUNS;
-    // split bins: the lanes along the iso-range lines, 16 pixels per thread across them
-    Lattice lattice = split ? choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, kGatherWalk, 192, split_cost)
-                            : choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, kGatherLines, 64, run_cost);
-    if (!lattice.ok) return best;
-    if (split) {
+    const size_t pixels = (size_t)nx * ny * nz;
+    auto seconds = [&](const Lattice& L, const std::vector<LatticeRate>& rates) {
+        double v = 0.0, w = 0.0, cost = 0.0;
+        for (const LatticeRate& r : rates) {
+            v = std::max(v, r.v);
+            w = std::max(w, r.w);
+            cost += split_cost(r.w);
+        }
+        if (split) {   // cost, and the share of the tiles (192 x 16) that straddle the image's edges
+            const double bx = 192 * std::abs(L.wx) + kGatherWalk * std::abs(L.vx), by = 192 * std::abs(L.wy) + kGatherWalk * std::abs(L.vy);
+            return cost * (1.0 + 0.5 * bx / nx) * (1.0 + 0.5 * by / ny);
+        }
+        const Shape q = best_shape(bins, L, S, nx, ny, nz, [&](int lines, int walk) { return 0.5 * (lines * v + walk * w); });
+        return q.layout.ok ? lattice_seconds(q.layout, q.tiles, S, pixels, run_unit(rates)) : (double)INFINITY;
+    };
+    Lattice lattice = choose_lattice(scene_rates(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r), ex, ey, kappa, seconds);
+    if (!lattice.ok) return GatherLayout{};
+    if (split) {   // the lanes along the iso-range lines, 16 pixels per thread across them
         std::swap(lattice.vx, lattice.wx);
         std::swap(lattice.vy, lattice.wy);
     }
-    const size_t pixels = (size_t)nx * ny * nz;
-    const int most = (int)std::min<size_t>(16, std::max<size_t>(1, kPartialBytes / (pixels * sizeof(float2))));
-    double least = INFINITY;
-    for (int shape : {80, 81, 40, 41}) {   // warps, and the warps along the walk: 1 or 2 with split bins, else all
-        const int warps = shape / 10, along = split ? 1 + shape % 10 : warps, across = warps / along;
-        if (!split && shape % 10) continue;
-        const int lines = kGatherLines * across, walk = kGatherWalk * along;
+    Shape q = best_shape(bins, lattice, S, nx, ny, nz, [&](int lines, int walk) -> double {
         const LatticeBounds B = lattice_bounds(lattice, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, 0.5 * lines, 0.5 * walk);
-        if (!B.ok) return best;
+        if (!B.ok) return NAN;
         // Split bins are held to the FP64 positions: the expansions' fourth-order terms, at most d^4 / (8 R^3) an
         // antenna, may not use up the margin of kNearEdge.
         const double d = 8.0 * (B.len_a + B.len_b);
-        if (split && !(d * d * d * d / (4.0 * B.nearest * B.nearest * B.nearest) * s_r < 1.0e-5)) return best;
-        // a tap from the excursion of the tile's pixels about its mean bin, plus the base's fraction and rounding
-        const double h = B.excursion(0.5 * lines, 0.5 * walk, s_r) + 0.1;
-        if (!(h < 4096.0)) continue;
-        const int ww = 2 * (int)std::ceil(h + 3.5 + kDip);
-        std::vector<int4> tiles;
+        if (split && !(d * d * d * d / (4.0 * B.nearest * B.nearest * B.nearest) * s_r < 1.0e-5)) return NAN;
+        return B.excursion(0.5 * lines, 0.5 * walk, s_r);
+    });
+    GatherLayout best = q.layout;
+    if (best.ok)
         for (int k = 0; k < nz; ++k)
-            for (const LatticeStrip& t : lattice_strips(lattice, lines, nx, ny))
-                for (long b = t.b0; b <= t.b1; b += walk) tiles.push_back(make_int4(t.a0, (int)b, k, 0));
-        for (int pb : {16, 8, 4, 2, 1}) {
-            if (!split && pb < 4) break;
-            const int full = warps == 8 ? 2 : 4;   // CTAs an SM: the registers' limit, and the shared memory's
-            const int ctas = std::min(full, (int)(227 * 1024 / (gather_smem(bins, warps, ww, pb).total + 1024)));
-            if (ctas < (split ? 1 : full)) continue;
-            GatherLayout L;
-            L.bins = bins;
-            L.warps = warps;
-            L.across = across;
-            L.ctas = ctas;
-            L.ww = ww;
-            L.pb = pb;
-            L.ok = true;
-            double t;
-            L.parts = best_parts(L, tiles.size(), S, pixels, most, &t);
-            if (t < 0.97 * least) {
-                least = t;
-                best = L;
-                best.tiles = tiles;
-            }
-        }
-    }
-    best.lattice = lattice;
+            for (const LatticeStrip& t : lattice_strips(lattice, q.lines, nx, ny))
+                for (long b = t.b0; b <= t.b1; b += q.walk) best.tiles.push_back(make_int4(t.a0, (int)b, k, 0));
     return best;
 }
 

@@ -26,57 +26,80 @@ inline double expansion_turns(double len_a, double len_b, double nearest, double
 }
 constexpr double kExpansionTurns = 1.0e-6;   // taken as exact
 
+// Bins per step along two axes, from one pulse at one point of the scene.
+struct LatticeRate {
+    double v, w;
+};
+
+// The rates along x and y at the centre of the scene and of its four quarters, from up to about 128 of the pulses, and a
+// bound of the nearest antenna's distance from the scene.
+struct SceneRates {
+    std::vector<LatticeRate> xy;
+    double nearest = INFINITY;
+    bool ok = false;
+};
+
+inline double step_length(const double* ex, const double* ey, int a, int b) {
+    double q = 0.0;
+    for (int d = 0; d < 3; ++d) q += (a * ex[d] + b * ey[d]) * (a * ex[d] + b * ey[d]);
+    return std::sqrt(q);
+}
+
+inline SceneRates scene_rates(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
+                              const double* ey, const double* ez, int nx, int ny, int nz, double s_r) {
+    SceneRates R;
+    const double half = 0.5 * (nx * step_length(ex, ey, 1, 0) + ny * step_length(ex, ey, 0, 1) +
+                               nz * std::sqrt(ez[0] * ez[0] + ez[1] * ez[1] + ez[2] * ez[2]));
+    const double points[5][2] = {{0.5, 0.5}, {0.25, 0.25}, {0.25, 0.75}, {0.75, 0.25}, {0.75, 0.75}};
+    const size_t every = std::max<size_t>(1, S / 128);
+    for (size_t s = 0; s < S; ++s)
+        for (int k = 0; k < (s % every ? 1 : 5); ++k) {
+            const double fx = points[k][0] * (nx - 1), fy = points[k][1] * (ny - 1);
+            LatticeRate g{0.0, 0.0};
+            for (int ant = 0; ant < 2; ++ant) {
+                const double* p = (ant ? rx : tx) + 3 * s;
+                double w[3];
+                for (int d = 0; d < 3; ++d) w[d] = origin[d] + fx * ex[d] + fy * ey[d] + 0.5 * (nz - 1) * ez[d] - p[d];
+                const double r = std::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+                if (!(r > 0.0)) return R;
+                if (k == 0) R.nearest = std::min(R.nearest, r - half);
+                g.v += s_r * (w[0] * ex[0] + w[1] * ex[1] + w[2] * ex[2]) / r;
+                g.w += s_r * (w[0] * ey[0] + w[1] * ey[1] + w[2] * ey[2]) / r;
+            }
+            if (!std::isfinite(g.v) || !std::isfinite(g.w)) return R;
+            if (s % every == 0) R.xy.push_back(g);
+        }
+    R.ok = true;
+    return R;
+}
+
+inline std::vector<LatticeRate> lattice_rates(const SceneRates& R, const Lattice& L) {
+    std::vector<LatticeRate> q(R.xy.size());
+    for (size_t i = 0; i < q.size(); ++i)
+        q[i] = LatticeRate{std::fabs(L.vx * R.xy[i].v + L.vy * R.xy[i].w), std::fabs(L.wx * R.xy[i].v + L.wy * R.xy[i].w)};
+    return q;
+}
+
 // Lattices with longer steps than the image's are taken only where their larger blocks still expand exactly (coarse
 // pixels at short range: 0.8 m at 2 km would go from 1.7e-5 to 3e-5 of the result).
-// `cost(rate)`: instructions per pixel-pulse at a bin rate (bins per step along w).  lines x along: the block of
-// lattice pixels the kernel works on, for the share of blocks that straddle the image's edges.
-template <class COST>
-inline Lattice choose_lattice(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                              const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa, int lines,
-                              int along, COST cost) {
+// `seconds(lattice, rates)`: what the kernel is expected to take on a lattice with these rates.
+template <class EST>
+inline Lattice choose_lattice(const SceneRates& R, const double* ex, const double* ey, double kappa, EST seconds) {
     Lattice best;
-    double c0[3];
-    for (int d = 0; d < 3; ++d)
-        c0[d] = origin[d] + 0.5 * ((nx - 1) * ex[d] + (ny - 1) * ey[d] + (nz - 1) * ez[d]);
+    if (!R.ok) return best;
     const int cand[8][4] = {{0, 1, 1, 0}, {1, 0, 0, 1}, {1, 1, 1, 0}, {-1, 1, 1, 0},
                             {2, 1, 1, 0}, {-2, 1, 1, 0}, {1, 2, 0, 1}, {-1, 2, 0, 1}};   // w, v
-    double sum[8] = {}, nearest = INFINITY, half = 0.0;
-    auto len = [&](int a, int b) {
-        double q = 0.0;
-        for (int d = 0; d < 3; ++d) q += (a * ex[d] + b * ey[d]) * (a * ex[d] + b * ey[d]);
-        return std::sqrt(q);
-    };
-    half = 0.5 * (nx * len(1, 0) + ny * len(0, 1) + nz * std::sqrt(ez[0] * ez[0] + ez[1] * ez[1] + ez[2] * ez[2]));
-    for (size_t s = 0; s < S; ++s) {
-        double gx = 0.0, gy = 0.0;   // bin rates along x and y at the scene centre
-        for (int ant = 0; ant < 2; ++ant) {
-            const double* p = (ant ? rx : tx) + 3 * s;
-            const double w[3] = {c0[0] - p[0], c0[1] - p[1], c0[2] - p[2]};
-            const double r = std::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
-            if (!(r > 0.0)) return best;
-            nearest = std::min(nearest, r - half);
-            gx += s_r * (w[0] * ex[0] + w[1] * ex[1] + w[2] * ex[2]) / r;
-            gy += s_r * (w[0] * ey[0] + w[1] * ey[1] + w[2] * ey[2]) / r;
-        }
-        if (!std::isfinite(gx) || !std::isfinite(gy)) return best;
-        for (int c = 0; c < 8; ++c) sum[c] += cost(std::fabs(cand[c][0] * gx + cand[c][1] * gy));
-    }
     double least = INFINITY;
     for (int c = 0; c < 8; ++c) {
-        if (c >= 2 && !(expansion_turns(len(cand[c][0], cand[c][1]), len(cand[c][2], cand[c][3]), nearest, kappa) < kExpansionTurns))
+        const Lattice L{cand[c][2], cand[c][3], cand[c][0], cand[c][1], true};
+        if (c >= 2 && !(expansion_turns(step_length(ex, ey, L.wx, L.wy), step_length(ex, ey, L.vx, L.vy), R.nearest, kappa) < kExpansionTurns))
             continue;
-        const double bx = along * std::abs(cand[c][0]) + lines * std::abs(cand[c][2]);   // a block's extent in pixels
-        const double by = along * std::abs(cand[c][1]) + lines * std::abs(cand[c][3]);
-        const double total = sum[c] * (1.0 + 0.5 * bx / nx) * (1.0 + 0.5 * by / ny);
-        if (total < least) {
-            least = total;
-            best.wx = cand[c][0];
-            best.wy = cand[c][1];
-            best.vx = cand[c][2];
-            best.vy = cand[c][3];
+        const double t = seconds(L, lattice_rates(R, L));
+        if (t < least || !best.ok) {
+            least = t;
+            best = L;
         }
     }
-    best.ok = true;
     return best;
 }
 

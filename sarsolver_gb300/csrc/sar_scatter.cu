@@ -331,23 +331,18 @@ cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ layout
-namespace {
-
-// Instructions per pixel-pulse by run length, for the choice of lattice only.
-double run_cost(double rate) {
-    return 15.0 * rate < kRunSpan ? 16.0 : 7.0 * rate < kRunSpan ? 20.0 : 3.0 * rate < kRunSpan ? 27.0 : 34.0;
-}
-
-}  // namespace
-
 // The CTAs' runs of blocks: each strip of `lines` lattice lines cut into segments so that a launch has about
 // five waves of CTAs.
+static long segment_blocks(long blocks, size_t S, int nz) {
+    const size_t groups = (S + 32 * kScatterWarps - 1) / (32 * kScatterWarps);
+    return std::max<long>(1, (long)((double)blocks * nz * groups / (152.0 * 3 * 5)));
+}
+
 static void scatter_items(size_t S, int nx, int ny, int nz, ScatterLayout* L) {
     const std::vector<LatticeStrip> strips = lattice_strips(L->lattice, L->lines, nx, ny);
     long total = 0;
     for (const LatticeStrip& t : strips) total += (t.b1 - t.b0) / kWalk + 1;
-    const size_t groups = (S + 32 * kScatterWarps - 1) / (32 * kScatterWarps);
-    const long len = std::max<long>(1, (long)((double)total * nz * groups / (152.0 * 3 * 5)));
+    const long len = segment_blocks(total, S, nz);
     L->items.clear();
     for (int k = 0; k < nz; ++k)
         for (const LatticeStrip& t : strips) {
@@ -359,26 +354,79 @@ static void scatter_items(size_t S, int nx, int ny, int nz, ScatterLayout* L) {
         }
 }
 
-ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa) {
+// Lines per block: halved until the windows leave room for three CTAs per SM.  h: bins from a block's anchor to its pixels.
+static bool fit_lines(ScatterLayout* L, int lines, double h) {
+    if (!(h < 4096.0)) return false;
+    L->lines = lines;
+    // taps from half a bin (the anchor's fraction), half a bin of rounding and kDip below to two bins above
+    L->half = (int)std::ceil(h + 1.0 + kDip);
+    L->slots = L->half + (int)std::ceil(h + 4.0);
+    return scatter_smem(L->slots, lines).total <= 75 * 1024;
+}
+
+// Estimated seconds on a lattice, from the rates alone: the blocks' pixel-pulses by run length (0.4 ps with runs of 16, 0.9
+// with two taps a pixel), what a block costs by itself (spread over its lines), and the slots it flushes: those the anchor
+// leaves behind, and a whole window at the end of a segment.  Fitted to 840 launches, every lattice of 380 geometries
+// forced in turn: 9 % rms.  Lines count most: with large rates along them 16 lines a block take 1.4 ps, two lines 10 ps.
+static double scatter_seconds(const Lattice& lattice, const std::vector<LatticeRate>& rates, size_t S, int nx, int ny, int nz) {
+    double v = 0.0, w = 0.0, mean = 0.0, unit = 0.0;
+    for (const LatticeRate& r : rates) {
+        v = std::max(v, r.v);
+        w = std::max(w, r.w);
+        mean += r.w / rates.size();
+        unit += (15.0 * r.w < kRunSpan ? 0.42 : 7.0 * r.w < kRunSpan ? 0.6 : 3.0 * r.w < kRunSpan ? 0.64 : 0.93) / rates.size();
+    }
     ScatterLayout L;
-    L.lattice = choose_lattice(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r, kappa, 16, kWalk, run_cost);
+    int lines = 16;
+    while (lines >= 2 && !fit_lines(&L, lines, 0.5 * lines * v + 8.0 * w + 0.1)) lines /= 2;
+    if (lines < 2) return INFINITY;
+    long blocks = 0;
+    for (const LatticeStrip& t : lattice_strips(lattice, lines, nx, ny)) blocks += (t.b1 - t.b0) / kWalk + 1;
+    const double groups = (double)((S + 32 * kScatterWarps - 1) / (32 * kScatterWarps)), len = (double)segment_blocks(blocks, S, nz);
+    const double flushed = (L.slots / len + kWalk * mean) / (kWalk * lines);   // slots per pixel-pulse
+    const double pulses = groups * 32 * kScatterWarps, work = (double)blocks * nz * kWalk * lines * pulses;
+    const double per_sm = (double)std::min<size_t>(4, 227 * 1024 / (scatter_smem(L.slots, lines).total + 1024));
+    const double waves = std::ceil(blocks * nz / len) * groups / (152.0 * per_sm);
+    // few waves: a partly filled GPU, and the last wave's share
+    const double fill = waves < 1.0 ? 0.6 + 0.5 / waves : waves < 1.6 ? 1.3 : waves < 3.0 ? 1.07 : 1.0;
+    return 1.0e-12 * work * (unit + 2.0 * flushed + 4.1 / lines) * fill;
+}
+
+// The same for the tile kernel: 1.05, 1.2 and 1.4 ps a pixel-pulse with run windows of 16, 8 and 4 pixels along its walk,
+// else 2.4 ps, or 4.8 where neighbouring lanes fall on one bin (atomics).  Strips are cut where their window, of some 480
+// bins, ends.
+static double tile_seconds(const ScatterTiles& t, const std::vector<LatticeRate>& rates, size_t S, size_t pixels) {
+    double v = 0.0, v_mean = 0.0, w = 0.0, unit = 0.0;
+    for (const LatticeRate& r : rates) {
+        v = std::max(v, r.v);
+        w = std::max(w, r.w);
+        v_mean += r.v / rates.size();
+        unit += (15.0 * r.w < kRunSpan ? 1.05 : 7.0 * r.w < kRunSpan ? 1.2 : 3.0 * r.w < kRunSpan ? 1.4 : 2.4) / rates.size();
+    }
+    if (unit > 1.4 && v_mean < 1.1) unit = 4.8;
+    const double seg = std::max(1.0, std::floor((440.0 - 32.0 * v) / (32.0 * std::max(w, 1.0e-3))));
+    const double waves = std::ceil(t.along / std::min(seg, (double)t.along)) * t.lines * std::ceil(S / 16.0) / 304.0;
+    return 5.0e-6 + 1.0e-12 * S * pixels * t.cover * unit * (waves < 1.0 ? 0.75 + 0.25 / waves : 1.0);
+}
+
+// The tile kernel is taken where it is estimated at less than 0.9 of the lattice's time: mostly small images with four and
+// more bins a pixel, whose blocks of few lines, a segment each, are all flush (192 x 192 x 400 pulses, 0.3 m, U = 16, 78
+// degrees off an axis: 45 against 72 us), and looks along an axis with run windows.  Of 336 geometries it is a seventh;
+// with the line at 1 the errors of both estimates cost what they gain.
+ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
+                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa,
+                             const ScatterTiles& tiles) {
+    ScatterLayout L;
+    const SceneRates rates = scene_rates(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r);
+    auto seconds = [&](const Lattice& l, const std::vector<LatticeRate>& r) { return scatter_seconds(l, r, S, nx, ny, nz); };
+    L.lattice = choose_lattice(rates, ex, ey, kappa, seconds);
     if (!L.lattice.ok) return L;
+    const double lattice = seconds(L.lattice, lattice_rates(rates, L.lattice));
+    if (tile_seconds(tiles, lattice_rates(rates, tiles.axes), S, (size_t)nx * ny * nz) < 0.9 * lattice) return L;
     const LatticeBounds B = lattice_bounds(L.lattice, tx, rx, S, origin, ex, ey, ez, nx, ny, nz, 8.0, 8.0);
     if (!B.ok) return L;
-    // lines are halved until the windows leave room for three CTAs per SM
-    for (L.lines = 16; L.lines >= 2; L.lines /= 2) {
-        const double h = B.excursion(0.5 * L.lines, 8.0, s_r) + 0.1;
-        if (!(h < 4096.0)) continue;
-        // taps from half a bin (the anchor's fraction), half a bin of rounding and kDip below to two bins above
-        L.half = (int)std::ceil(h + 1.0 + kDip);
-        L.slots = L.half + (int)std::ceil(h + 4.0);
-        if (scatter_smem(L.slots, L.lines).total <= 75 * 1024) {
-            L.ok = true;
-            scatter_items(S, nx, ny, nz, &L);
-            break;
-        }
-    }
+    for (int lines = 16; lines >= 2 && !L.ok; lines /= 2) L.ok = fit_lines(&L, lines, B.excursion(0.5 * lines, 8.0, s_r) + 0.1);
+    if (L.ok) scatter_items(S, nx, ny, nz, &L);
     return L;
 }
 

@@ -35,9 +35,19 @@ struct ScatterArgs {
     int vx, vy, wx, wy, lines, half, slots;
 };
 
-// Host-side choice of lattice, block and segments for linear sampling without split bins (see sar_scatter.cu).
+// How the tile kernel would scatter the same: image steps along its lanes (v) and its walk (w), lines of 32 x 32 tiles, the
+// tiles of a line, and pixels of tiles per image pixel.
+struct ScatterTiles {
+    Lattice axes;
+    int lines = 1, along = 1;
+    double cover = 1.0;
+};
+
+// Host-side choice of lattice, block and segments for linear sampling without split bins (see sar_scatter.cu); not ok
+// where the tile kernel is expected to be clearly faster.
 ScatterLayout scatter_layout(const double* tx, const double* rx, size_t S, const double* origin, const double* ex,
-                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa);
+                             const double* ey, const double* ez, int nx, int ny, int nz, double s_r, double kappa,
+                             const ScatterTiles& tiles);
 cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st);
 
 }  // namespace sar

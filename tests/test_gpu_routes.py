@@ -49,3 +49,17 @@ def test_tile_kernels(shape, spacing, upsample, interp, gather):
     assert rel_l2(plan.forward(x).cpu().numpy(), general.forward(x).cpu().numpy()) < 1.0e-5
     assert rel_l2(plan.adjoint(y).cpu().numpy(), general.adjoint(y).cpu().numpy()) < 1.0e-5
     assert plan.device_flags() == 0
+
+
+@pytest.mark.parametrize("side,pulses,spacing,upsample,az,gather,scatter", [
+    # (v, w): no runs along any line, so short windows of many lines, and lanes whose loads fall on few bins, come first
+    (512, 1024, 0.5, 8.0, 50.0, ((0, 1), (1, 0)), ((1, 0), (-1, 1))),
+    (512, 1024, 0.25, 8.0, 18.0, ((0, 1), (1, 0)), ((1, 0), (0, 1))),
+    (512, 1024, 0.3, 16.0, 22.0, ((0, 1), (1, 0)), ((0, 1), (-1, 2))),
+    (192, 400, 0.5, 8.0, 42.0, ((1, 0), (-1, 1)), ...),   # (forward: within 5 % on either kernel)
+    (192, 400, 0.3, 16.0, 14.0, ((1, 0), (0, 1)), None)])   # the tile kernel: 46 us against 70
+def test_lattices_of_oblique_looks(side, pulses, spacing, upsample, az, gather, scatter):
+    """Measured with every lattice forced: with others the first forward projection took 2083 us for 429, the second
+    backprojection 387 us for 286, the third 706 us for 334, the fourth 74 us for 48."""
+    plan = make(pulses, (side, side), spacing, upsample, "linear", az=az, samples=1024)
+    assert plan.gather_lattice == gather and scatter in (plan.scatter_lattice, ...)

@@ -113,6 +113,7 @@ struct sar_plan {
     bool fwd_transposed = false;   // forward scatter: lanes along y, rows walked along x
     int gather_shear = 0;          // backprojection on a sheared lattice (gc_adj), lanes along ey + m ex
     int ring_half = 0;             // forward scatter on ring windows (FpGridArgs.ring_half), 0: strips
+    int ring_pad = 1;
     long tiles_valid = 0;          // its tiles that hold image pixels (0: all tiles of the grid)
     bool staged = true;
     bool values = false;   // stored profiles are plain values (kProfValues), not pairs
@@ -695,7 +696,7 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
                             }
                         }
                 const int ws = (need + 31) & ~31;
-                if (fp_grid_ws_smem_bytes(ws, pbf, p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins, 0,
+                if (fp_grid_ws_smem_bytes(ws, pbf, p->interp == SAR_INTERP_LINEAR && !p->gc_fwd.precise_bins, 1,
                                           p->interp == SAR_INTERP_NEAREST_REF) <= kFpSmemBudget) {
                     p->seg_tiles = seg;
                     p->segs_per_column = segs;
@@ -731,20 +732,37 @@ int build_plan(const sar_geometry* g_in, sar_plan* p) {
             }
             if (take && h >= 0.0 && h < 1.0e6) {
                 const int H = (int)std::ceil(h) + 4, W = (2 * H + 1 + 31) & ~31;
-                for (size_t budget : {kFpRingTwoBudget, kFpRingSmemBudget}) {
-                    if (p->ring_half) break;
-                    for (int pbf : {16, 8})
-                        if (fp_grid_ws_smem_bytes(W, pbf, 0, 1, p->interp == SAR_INTERP_NEAREST_REF) <= budget) {
+                const int nearest = p->interp == SAR_INTERP_NEAREST_REF;
+                // Padding every 16 bins spreads lanes 8 or 16 bins apart over the banks and brings lanes 15 apart together: by
+                // the expected conflicts of the lanes' bins (512^2 x 1024, 0.3 m, U = 24, linear: at 22 degrees 0.78 ms with it
+                // and 1.63 without, at 30 degrees 1.47 and 0.84; without conflicts it costs 3 to 6 %).
+                const Lattice lanes = p->fwd_transposed ? Lattice{0, 1, 1, 0, true} : plain;
+                double with = 0.0, without = 0.0;
+                for (const LatticeRate& r : lattice_rates(scene_rates(tx, rx, S, origin, ex, ey, ez, nx, ny, nz, s_r), lanes)) {
+                    with += bank_degree(r.v, true);
+                    without += bank_degree(r.v, false);
+                }
+                const int first = with < 0.95 * without;
+                // Pulses per CTA.  The kernel holds two CTAs an SM for nearest bins, one for linear.  8 take 0.62 of the time
+                // of 16: what fills the waves better, of what fits.
+                const size_t count = p->block ? p->block : S, strips = (size_t)nz * lines, slots = nearest ? 304 : 152;
+                auto waves = [&](int pbf) { return (double)((strips * ((count + pbf - 1) / pbf) + slots - 1) / slots); };
+                const bool eight = 0.62 * waves(8) < waves(16);
+                for (size_t budget : {nearest ? kFpRingTwoBudget : kFpRingSmemBudget, kFpRingSmemBudget})
+                    for (int pbf : {eight ? 8 : 16, 16, 8})
+                        for (int pad : {first, 1 - first}) {
+                            if (p->ring_half || fp_grid_ws_smem_bytes(W, pbf, 0, pad, nearest) > budget) continue;
                             p->ring_half = H;
+                            p->ring_pad = pad;
                             p->ws = W;
                             p->pbf = pbf;
-                            p->seg_tiles = along;
-                            p->segs_per_column = 1;
-                            p->n_strips = (size_t)nz * lines;
-                            strip_start.assign(p->n_strips * S, 0);   // not read with ring windows
-                            p->forward_points = false;
-                            break;
                         }
+                if (p->ring_half) {
+                    p->seg_tiles = along;
+                    p->segs_per_column = 1;
+                    p->n_strips = strips;
+                    strip_start.assign(p->n_strips * S, 0);   // not read with ring windows
+                    p->forward_points = false;
                 }
             }
         }
@@ -1383,6 +1401,7 @@ static int scatter_pulses(sar_plan* p, const float2* x, float2* acc, size_t firs
     a.segs_per_column = p->segs_per_column;
     a.ws = p->ws;
     a.ring_half = p->ring_half;
+    a.pad = p->ring_pad;
     a.pbf = p->pbf;
     a.linear = p->interp == SAR_INTERP_LINEAR;
     // the scatter walks the axis along which bins change slowly: the transpose of the gather's

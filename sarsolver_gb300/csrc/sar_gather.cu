@@ -555,17 +555,6 @@ constexpr size_t kPartialBytes = (size_t)256 << 20;   // partial images of a pla
 // loads spread over the banks.
 double split_cost(double rate) { return 16.0 + std::min(rate, 8.0); }
 
-// Bank pairs: the most distinct bins that a half-warp's loads have on one of the sixteen, its lanes `rate` bins apart.
-double bank_degree(double rate) {
-    int hits[16] = {}, last = -1, most = 0;
-    for (int l = 0; l < 16; ++l) {
-        const int bin = (int)std::min(rate * l, 1.0e6);
-        if (bin != last) most = std::max(most, ++hits[bin & 15]);
-        last = bin;
-    }
-    return most;
-}
-
 // Plain bins: seconds per pixel-pulse of a lattice on a full GPU, by run length; where each sample loads two bins, by the
 // bank conflicts of the lanes' loads.  Fitted to 380 geometries with every lattice forced in turn: 0.7 ps with runs of 16,
 // 0.95 without runs up to two bins a bank, then 1.3, 1.6 and 2.4 ps at three, four and five.
@@ -576,7 +565,7 @@ double run_unit(const std::vector<LatticeRate>& rates) {
         sum += 15.0 * r.w < kRunSpan  ? run
                : 7.0 * r.w < kRunSpan ? run + 0.06
                : 3.0 * r.w < kRunSpan ? run + 0.14
-                                      : std::max(0.95, 0.2 + 0.42 * bank_degree(r.v));
+                                      : std::max(0.95, 0.2 + 0.42 * bank_degree(r.v, false));
     }
     return 1.0e-12 * sum / rates.size();
 }

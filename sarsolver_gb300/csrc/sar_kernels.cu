@@ -828,19 +828,17 @@ constexpr int kXtStride = kTile + 1;   // staged image tile: 32 lines of 33 valu
 
 __device__ __forceinline__ size_t align_up(size_t n, size_t a) { return (n + a - 1) & ~(a - 1); }
 
-// Ring windows are not padded: they hold wide tiles, whose lanes' bins spread over the banks by themselves, and
-// without the padding two CTAs fit an SM at upsample 128.
-__host__ __device__ inline int window_slots(int ws, int ring) { return ring ? ws : ws + (ws >> 4) + 1; }
+__host__ __device__ inline int window_slots(int ws, int pad) { return pad ? ws + (ws >> 4) + 1 : ws; }
 
 struct FpWsLayout {
     size_t win, coef, xt, base, fast, wst, bars, anchors, queue, total;
 };
 
 // wide_x: image values staged as (re, re, im, im) (the linear run-window kernels), else (re, im).
-__host__ __device__ inline FpWsLayout fp_ws_layout(int ws, int pbf, int wide_x, int ring, int nearest) {
+__host__ __device__ inline FpWsLayout fp_ws_layout(int ws, int pbf, int wide_x, int pad, int nearest) {
     FpWsLayout L;
     L.win = 0;
-    L.coef = L.win + (size_t)pbf * window_slots(ws, ring) * sizeof(float2);
+    L.coef = L.win + (size_t)pbf * window_slots(ws, pad) * sizeof(float2);
     L.coef = (L.coef + 15) & ~(size_t)15;
     L.xt = L.coef + (size_t)2 * pbf * 4 * kSetF4 * sizeof(float4);
     L.base = L.xt + (size_t)2 * kTile * kXtStride * (wide_x ? sizeof(float4) : sizeof(float2));
@@ -853,14 +851,14 @@ __host__ __device__ inline FpWsLayout fp_ws_layout(int ws, int pbf, int wide_x, 
     return L;
 }
 
-size_t fp_grid_ws_smem_bytes(int ws, int pbf, int wide_x, int ring, int nearest) {
-    return fp_ws_layout(ws, pbf, wide_x, ring, nearest).total;
+size_t fp_grid_ws_smem_bytes(int ws, int pbf, int wide_x, int pad, int nearest) {
+    return fp_ws_layout(ws, pbf, wide_x, pad, nearest).total;
 }
 
 // Window slot of bin w: one padding slot every 16 bins, so lanes whose bins differ by a
-// multiple of 16 do not share a shared-memory bank pair.
-template <bool RING>
-__device__ __forceinline__ int wslot(int w) { return RING ? w : w + (w >> 4); }
+// multiple of 16 do not share a shared-memory bank pair.  Ring windows have them or not (FpGridArgs.pad).
+template <bool PAD>
+__device__ __forceinline__ int wslot(int w) { return PAD ? w + (w >> 4) : w; }
 // Ring slot of x in [0, 2 ws).
 __device__ __forceinline__ int ring_wrap(int x, int ws) { return (int)min((unsigned)x, (unsigned)(x - ws)); }
 
@@ -885,9 +883,9 @@ __device__ __forceinline__ RowEval<PRECISE> scatter_eval(const ColumnTerms& ct, 
     return e;
 }
 
-template <bool RING = false>
+template <bool PAD>
 __device__ __forceinline__ void rmw_add(float2* wp, int idx, float w, float cr, float ci) {
-    float2* q = wp + wslot<RING>(idx);
+    float2* q = wp + wslot<PAD>(idx);
     float2 u = *q;
     u.x = fmaf(w, cr, u.x);
     u.y = fmaf(w, ci, u.y);
@@ -902,7 +900,7 @@ __device__ __forceinline__ float2 staged_value(const float4 v) { return make_flo
 // disjoint (one phase per row); MODE 1: bins n distinct (two phases); MODE 0: atomics.
 // RING: ring windows (off_p / off_q + bin is a slot before wrapping, in [0, 2 ws)), else strip windows
 // (off = base - window start).
-template <bool LINEAR, bool PRECISE, int MODE, bool TWO, typename XT, bool RING = false>
+template <bool LINEAR, bool PRECISE, int MODE, bool TWO, typename XT, bool RING, bool PAD>
 __device__ __forceinline__ void scatter_rows(const ColumnTerms& ctp, float c9p, float w9p, float ibp,
                                              const ColumnTerms& ctq, float c9q, float w9q, float ibq,
                                              const XT* xrow, float2* wp, float2* wq, int off_p, int off_q,
@@ -932,42 +930,42 @@ __device__ __forceinline__ void scatter_rows(const ColumnTerms& ctp, float c9p, 
             const float w0p = 0.5f - ep.bp.s, w1p = 0.5f + ep.bp.s;
             const float w0q = TWO ? 0.5f - eq.bp.s : 0.f, w1q = TWO ? 0.5f + eq.bp.s : 0.f;
             if (MODE == 2) {
-                rmw_add<RING>(wp, ip, w0p, ep.cr, ep.ci);
-                rmw_add<RING>(wp, next(ip), w1p, ep.cr, ep.ci);
+                rmw_add<PAD>(wp, ip, w0p, ep.cr, ep.ci);
+                rmw_add<PAD>(wp, next(ip), w1p, ep.cr, ep.ci);
                 if (TWO) {
-                    rmw_add<RING>(wq, iq, w0q, eq.cr, eq.ci);
-                    rmw_add<RING>(wq, next(iq), w1q, eq.cr, eq.ci);
+                    rmw_add<PAD>(wq, iq, w0q, eq.cr, eq.ci);
+                    rmw_add<PAD>(wq, next(iq), w1q, eq.cr, eq.ci);
                 }
                 __syncwarp();
             } else if (MODE == 1) {
-                rmw_add<RING>(wp, ip, w0p, ep.cr, ep.ci);
-                if (TWO) rmw_add<RING>(wq, iq, w0q, eq.cr, eq.ci);
+                rmw_add<PAD>(wp, ip, w0p, ep.cr, ep.ci);
+                if (TWO) rmw_add<PAD>(wq, iq, w0q, eq.cr, eq.ci);
                 __syncwarp();
-                rmw_add<RING>(wp, next(ip), w1p, ep.cr, ep.ci);
-                if (TWO) rmw_add<RING>(wq, next(iq), w1q, eq.cr, eq.ci);
+                rmw_add<PAD>(wp, next(ip), w1p, ep.cr, ep.ci);
+                if (TWO) rmw_add<PAD>(wq, next(iq), w1q, eq.cr, eq.ci);
                 __syncwarp();
             } else {
-                float2* a0 = wp + wslot<RING>(ip);
-                float2* a1 = wp + wslot<RING>(next(ip));
+                float2* a0 = wp + wslot<PAD>(ip);
+                float2* a1 = wp + wslot<PAD>(next(ip));
                 atomicAdd(&a0->x, w0p * ep.cr); atomicAdd(&a0->y, w0p * ep.ci);
                 atomicAdd(&a1->x, w1p * ep.cr); atomicAdd(&a1->y, w1p * ep.ci);
                 if (TWO) {
-                    float2* b0 = wq + wslot<RING>(iq);
-                    float2* b1 = wq + wslot<RING>(next(iq));
+                    float2* b0 = wq + wslot<PAD>(iq);
+                    float2* b1 = wq + wslot<PAD>(next(iq));
                     atomicAdd(&b0->x, w0q * eq.cr); atomicAdd(&b0->y, w0q * eq.ci);
                     atomicAdd(&b1->x, w1q * eq.cr); atomicAdd(&b1->y, w1q * eq.ci);
                 }
             }
         } else {
             if (MODE >= 1) {
-                rmw_add<RING>(wp, ip, 1.0f, ep.cr, ep.ci);
-                if (TWO) rmw_add<RING>(wq, iq, 1.0f, eq.cr, eq.ci);
+                rmw_add<PAD>(wp, ip, 1.0f, ep.cr, ep.ci);
+                if (TWO) rmw_add<PAD>(wq, iq, 1.0f, eq.cr, eq.ci);
                 __syncwarp();
             } else {
-                float2* a0 = wp + wslot<RING>(ip);
+                float2* a0 = wp + wslot<PAD>(ip);
                 atomicAdd(&a0->x, ep.cr); atomicAdd(&a0->y, ep.ci);
                 if (TWO) {
-                    float2* b0 = wq + wslot<RING>(iq);
+                    float2* b0 = wq + wslot<PAD>(iq);
                     atomicAdd(&b0->x, eq.cr); atomicAdd(&b0->y, eq.ci);
                 }
             }
@@ -1005,10 +1003,10 @@ __device__ __forceinline__ float2 near_bins(const NearTerms& t, float2 d, float2
 }
 
 // Returns a mask of the contributions near a rounding boundary: bit 2 row + h for pulse h of the pair.
-template <int MODE, bool TWO, bool RING>
+template <int MODE, bool TWO, bool RING, bool PAD>
 __device__ __forceinline__ unsigned scatter_rows_near(const NearTerms& t, const float2* xrow, float2* wp, float2* wq,
                                                       int off_p, int off_q, int ws, int lane) {
-    auto slot = [&](int i) { return wslot<RING>(RING ? ring_wrap(i, ws) : (int)min((unsigned)i, (unsigned)(ws - 2))); };
+    auto slot = [&](int i) { return wslot<PAD>(RING ? ring_wrap(i, ws) : (int)min((unsigned)i, (unsigned)(ws - 2))); };
     unsigned edge = 0;
 #pragma unroll 4
     for (int rr = 0; rr < 16; ++rr) {
@@ -1115,14 +1113,14 @@ __device__ __forceinline__ void scatter_rows_runs(const ColumnTerms& ctp, float 
         const float2 s0r = mul2(add2(Er, mul2(Dr, M1)), f2(0.5f, 0.5f)), s0i = mul2(add2(Ei, mul2(Di, M1)), f2(0.5f, 0.5f));
         const float2 s1r = add2(Cr, mul2(Er, M1)), s1i = add2(Ci, mul2(Ei, M1));
         const float2 s2r = mul2(add2(Er, Dr), f2(0.5f, 0.5f)), s2i = mul2(add2(Ei, Di), f2(0.5f, 0.5f));
-        rmw_add(wp, n0p, 1.0f, s0r.x, s0i.x);
-        if (TWO) rmw_add(wq, n0q, 1.0f, s0r.y, s0i.y);
+        rmw_add<true>(wp, n0p, 1.0f, s0r.x, s0i.x);
+        if (TWO) rmw_add<true>(wq, n0q, 1.0f, s0r.y, s0i.y);
         __syncwarp();
-        rmw_add(wp, n0p + 1, 1.0f, s1r.x, s1i.x);
-        if (TWO) rmw_add(wq, n0q + 1, 1.0f, s1r.y, s1i.y);
+        rmw_add<true>(wp, n0p + 1, 1.0f, s1r.x, s1i.x);
+        if (TWO) rmw_add<true>(wq, n0q + 1, 1.0f, s1r.y, s1i.y);
         __syncwarp();
-        rmw_add(wp, n0p + 2, 1.0f, s2r.x, s2i.x);
-        if (TWO) rmw_add(wq, n0q + 2, 1.0f, s2r.y, s2i.y);
+        rmw_add<true>(wp, n0p + 2, 1.0f, s2r.x, s2i.x);
+        if (TWO) rmw_add<true>(wq, n0q + 2, 1.0f, s2r.y, s2i.y);
         __syncwarp();
     }
   }
@@ -1139,15 +1137,15 @@ __device__ __forceinline__ int pair_mode(int a, int b) {
 }
 
 // Returns the mask of scatter_rows_near (nearest bins), else 0.
-template <bool LINEAR, bool PRECISE, bool TWO, typename XT, bool RING = false>
+template <bool LINEAR, bool PRECISE, bool TWO, typename XT, bool RING, bool PAD>
 __device__ __forceinline__ unsigned scatter_half(int mode, const ColumnTerms& ctp, float c9p, float w9p, float ibp,
                                                  const ColumnTerms& ctq, float c9q, float w9q, float ibq,
                                                  const XT* xrow, float2* wp, float2* wq, int off_p, int off_q,
                                                  int ws, int lane) {
     if constexpr (!LINEAR && PRECISE) {
         const NearTerms t = near_terms(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq);
-        return mode >= 1 ? scatter_rows_near<1, TWO, RING>(t, xrow, wp, wq, off_p, off_q, ws, lane)
-                         : scatter_rows_near<0, TWO, RING>(t, xrow, wp, wq, off_p, off_q, ws, lane);
+        return mode >= 1 ? scatter_rows_near<1, TWO, RING, PAD>(t, xrow, wp, wq, off_p, off_q, ws, lane)
+                         : scatter_rows_near<0, TWO, RING, PAD>(t, xrow, wp, wq, off_p, off_q, ws, lane);
     }
     if constexpr (LINEAR && !PRECISE && !RING) {
         if (mode >= 3) {
@@ -1162,13 +1160,13 @@ __device__ __forceinline__ unsigned scatter_half(int mode, const ColumnTerms& ct
     }
     if constexpr (LINEAR || !PRECISE) {
         if (mode >= 2)
-            scatter_rows<LINEAR, PRECISE, 2, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
+            scatter_rows<LINEAR, PRECISE, 2, TWO, XT, RING, PAD>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
                                                             ws, lane);
         else if (mode == 1)
-            scatter_rows<LINEAR, PRECISE, 1, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
+            scatter_rows<LINEAR, PRECISE, 1, TWO, XT, RING, PAD>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
                                                             ws, lane);
         else
-            scatter_rows<LINEAR, PRECISE, 0, TWO, XT, RING>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
+            scatter_rows<LINEAR, PRECISE, 0, TWO, XT, RING, PAD>(ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow, wp, wq, off_p, off_q,
                                                             ws, lane);
     }
     return 0u;
@@ -1177,10 +1175,11 @@ __device__ __forceinline__ unsigned scatter_half(int mode, const ColumnTerms& ct
 // Adds the window slots of bins [lo, hi] (absolute) of one pulse into its accumulator row and clears
 // them (ring windows: the bins a tile step leaves behind, and the last tile's at the end).  The ring holds bins from
 // `first` on, bin `first` in slot `rot`.
+template <bool PAD>
 __device__ __forceinline__ void ring_flush(float2* wp, int lo, int hi, int first, int rot, const FpGridArgs& a, int s,
                                            int lane) {
     for (int bin = lo + lane; bin <= hi; bin += 32) {
-        float2* q = wp + ring_wrap(bin - first + rot, a.ws);
+        float2* q = wp + wslot<PAD>(ring_wrap(bin - first + rot, a.ws));
         const float2 v = *q;
         if (v.x == 0.f && v.y == 0.f) continue;
         *q = make_float2(0.f, 0.f);
@@ -1196,13 +1195,13 @@ __device__ __forceinline__ void ring_flush(float2* wp, int lo, int hi, int first
 // RING (split bins only): ring windows instead of strip windows (FpGridArgs.ring_half): a CTA walks
 // its whole line of tiles and, between tiles, each warp adds and clears the bins its pulses leave
 // behind, so windows no longer bound the length of a strip (1-tile strips at upsample 128 otherwise).
-template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false>
+template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false, bool PAD = true>
 __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws_kernel(const FpGridArgs a) {
     extern __shared__ __align__(16) unsigned char fsm[];
-    const int pbf = a.pbf, ws = a.ws, wslots = window_slots(ws, RING);
+    const int pbf = a.pbf, ws = a.ws, wslots = window_slots(ws, PAD);
     constexpr bool WIDE_X = LINEAR && !PRECISE;
     using XT = typename std::conditional<WIDE_X, float4, float2>::type;
-    const FpWsLayout L = fp_ws_layout(ws, pbf, WIDE_X, RING, !LINEAR);
+    const FpWsLayout L = fp_ws_layout(ws, pbf, WIDE_X, PAD, !LINEAR);
     float2* win = reinterpret_cast<float2*>(fsm + L.win);
     float4* coef0 = reinterpret_cast<float4*>(fsm + L.coef);
     XT* xt0 = reinterpret_cast<XT*>(fsm + L.xt);
@@ -1386,9 +1385,9 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
                 if (t > 0 && nb != prev_base[k]) {
                     const int ob = prev_base[k], rot = wst[p];
                     if (nb > ob)
-                        ring_flush(win + p * wslots, ob - rh, min(ob + rh, nb - rh - 1), ob - rh, rot, a, s0 + p, lane);
+                        ring_flush<PAD>(win + p * wslots, ob - rh, min(ob + rh, nb - rh - 1), ob - rh, rot, a, s0 + p, lane);
                     else
-                        ring_flush(win + p * wslots, max(ob - rh, nb + rh + 1), ob + rh, ob - rh, rot, a, s0 + p, lane);
+                        ring_flush<PAD>(win + p * wslots, max(ob - rh, nb + rh + 1), ob + rh, ob - rh, rot, a, s0 + p, lane);
                     __syncwarp();
                     if (lane == 0) {
                         const int moved = (rot + (nb - ob)) % ws;
@@ -1424,9 +1423,9 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
                         load_column<PRECISE, TRANSPOSED>(coef + (pq * 4 + qs) * kSetF4, tt, c9q, w9q, ibq);
                     const XT* xrow = xt + 16 * half * kXtStride;
                     const unsigned edge =
-                        two ? scatter_half<LINEAR, PRECISE, true, XT, RING>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow,
+                        two ? scatter_half<LINEAR, PRECISE, true, XT, RING, PAD>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq, xrow,
                                                                             wp, wq, off_p, off_q, ws, lane)
-                            : scatter_half<LINEAR, PRECISE, false, XT, RING>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq,
+                            : scatter_half<LINEAR, PRECISE, false, XT, RING, PAD>(mode, ctp, c9p, w9p, ibp, ctq, c9q, w9q, ibq,
                                                                              xrow, wp, wq, off_p, off_q, ws, lane);
                     if constexpr (!LINEAR && PRECISE) {
                         unsigned left = edge;
@@ -1463,14 +1462,14 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
         for (int k = 0; k < kMaxStagePulses / (kWsConsumers / 32); ++k) {
             const int p = warp + k * (kWsConsumers / 32);
             if (p >= npb) break;
-            ring_flush(win + p * wslots, prev_base[k] - rh, prev_base[k] + rh, prev_base[k] - rh, wst[p], a, s0 + p, lane);
+            ring_flush<PAD>(win + p * wslots, prev_base[k] - rh, prev_base[k] + rh, prev_base[k] - rh, wst[p], a, s0 + p, lane);
         }
     } else {
         // merge this warp's windows into the global accumulator
         for (int p = warp; p < npb; p += kWsConsumers / 32) {
             const float2* wp = win + p * wslots;
             for (int w = lane; w < ws; w += 32) {
-                const float2 v = wp[wslot<false>(w)];
+                const float2 v = wp[wslot<true>(w)];
                 if (v.x == 0.f && v.y == 0.f) continue;
                 const long gi = (long)wst[p] + w - a.bg0;
                 if (gi < 0 || gi >= a.Lg) {
@@ -1484,23 +1483,25 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
     }
 }
 
-template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false>
+template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false, bool PAD = true>
 static cudaError_t launch_fp_grid_ws_t(const FpGridArgs& a, cudaStream_t st) {
-    const size_t smem = fp_grid_ws_smem_bytes(a.ws, a.pbf, LINEAR && !PRECISE, RING, !LINEAR);
+    const size_t smem = fp_grid_ws_smem_bytes(a.ws, a.pbf, LINEAR && !PRECISE, PAD, !LINEAR);
     const int lines = TRANSPOSED ? a.g.tiles_y : a.g.tiles_x;
     const dim3 grid((unsigned)(a.segs_per_column * lines * a.g.nz), (unsigned)((a.S + a.pbf - 1) / a.pbf));
-    cudaError_t e = cudaFuncSetAttribute(fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING>,
+    cudaError_t e = cudaFuncSetAttribute(fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING, PAD>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING><<<grid, kWsThreads, smem, st>>>(a);
+    fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING, PAD><<<grid, kWsThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
 template <bool TRANSPOSED>
 static cudaError_t launch_fp_grid_ws_o(const FpGridArgs& a, cudaStream_t st) {
     if (a.ring_half > 0)   // ring windows: split bins only
-        return a.linear ? launch_fp_grid_ws_t<true, true, TRANSPOSED, true>(a, st)
-                        : launch_fp_grid_ws_t<false, true, TRANSPOSED, true>(a, st);
+        return a.linear ? (a.pad ? launch_fp_grid_ws_t<true, true, TRANSPOSED, true>(a, st)
+                                 : launch_fp_grid_ws_t<true, true, TRANSPOSED, true, false>(a, st))
+                        : (a.pad ? launch_fp_grid_ws_t<false, true, TRANSPOSED, true>(a, st)
+                                 : launch_fp_grid_ws_t<false, true, TRANSPOSED, true, false>(a, st));
     if (a.linear)
         return a.g.precise_bins ? launch_fp_grid_ws_t<true, true, TRANSPOSED>(a, st)
                                 : launch_fp_grid_ws_t<true, false, TRANSPOSED>(a, st);

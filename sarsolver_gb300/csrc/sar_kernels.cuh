@@ -88,11 +88,12 @@ struct FpGridArgs {
     int ring_half = 0;         // > 0 (split bins only): ring windows -- a pulse's ws slots hold the bins
                                //    from its tile's base bin - ring_half on, and a tile touches bins
                                //    within ring_half of its base bin; 0: strip windows from strip_start
+    int pad = 1;               // ring windows: a padding slot every 16 bins, as the other windows have, or none
 };
 // Warp-specialised variant: producer warps stage image tiles and coefficient sets; each
 // gathering warp owns whole pulses, so its windows need no atomics when bins along a row of
 // the tile are provably distinct (pbf <= 32, multiple of 8).
-size_t fp_grid_ws_smem_bytes(int ws, int pbf, int wide_x, int ring, int nearest);   // wide_x: linear, not precise bins
+size_t fp_grid_ws_smem_bytes(int ws, int pbf, int wide_x, int pad, int nearest);   // wide_x: linear, not precise bins
 cudaError_t launch_fp_grid_ws(const FpGridArgs& a, cudaStream_t st);
 
 // Unstructured positions (K2/K3 point variants).

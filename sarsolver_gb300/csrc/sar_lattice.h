@@ -80,6 +80,18 @@ inline std::vector<LatticeRate> lattice_rates(const SceneRates& R, const Lattice
     return q;
 }
 
+// Shared-memory bank pairs: the most distinct bins that a half-warp's accesses have on one of the sixteen, its lanes `rate`
+// bins apart; windows with a padding slot every 16 bins, or without.
+inline double bank_degree(double rate, bool pad) {
+    int hits[16] = {}, last = -1, most = 0;
+    for (int l = 0; l < 16; ++l) {
+        const int bin = (int)std::min(rate * l, 1.0e6);
+        if (bin != last) most = std::max(most, ++hits[(pad ? bin + (bin >> 4) : bin) & 15]);
+        last = bin;
+    }
+    return most;
+}
+
 // Lattices with longer steps than the image's are taken only where their larger blocks still expand exactly (coarse
 // pixels at short range: 0.8 m at 2 km would go from 1.7e-5 to 3e-5 of the result).
 // `seconds(lattice, rates)`: what the kernel is expected to take on a lattice with these rates.

@@ -63,3 +63,17 @@ def test_lattices_of_oblique_looks(side, pulses, spacing, upsample, az, gather, 
     backprojection 387 us for 286, the third 706 us for 334, the fourth 74 us for 48."""
     plan = make(pulses, (side, side), spacing, upsample, "linear", az=az, samples=1024)
     assert plan.gather_lattice == gather and scatter in (plan.scatter_lattice, ...)
+
+
+@pytest.mark.parametrize("interp", ["linear", "nearest_ref"])
+@pytest.mark.parametrize("az,pulses", [(22.0, 33), (30.0, 33), (22.0, 1030), (30.0, 1030), (0.0, 1030)])
+def test_ring_windows(interp, az, pulses):
+    """Ring windows with padding and without (22 and 30 degrees, where either spares most bank conflicts), 8 and 16 pulses
+    a CTA (few pulses and many)."""
+    rng = np.random.default_rng(pulses + int(az))
+    plan = make(pulses, (100, 130), 0.3, 24.0 if az else 128.0, interp, az=az)
+    general = make(pulses, (100, 130), 0.3, 24.0 if az else 128.0, interp, az=az, path="points")
+    assert plan.scatter_ring_half > 0 and plan.scatter_lattice is None
+    x = torch.from_numpy(crandn(rng, 13000))
+    assert rel_l2(plan.forward(x).cpu().numpy(), general.forward(x).cpu().numpy()) < 1.0e-5
+    assert plan.device_flags() == 0

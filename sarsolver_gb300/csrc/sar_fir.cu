@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(FirShape<N>::NT, FirShape<N>::CTAS) fir_up_ker
         for (int e = 0; e < 16; ++e) v[e] = r ? cmulf(X[e], __ldg(a.half + t + T * e)) : X[e];
         up_first_pass<N>(v, A, t);
         __syncthreads();
-        const float2* F = up_passes<N>(A, B, a.tw_n, t);
+        const float2* F = up_passes<N, false>(A, B, a.tw_n, t);
         for (int i = ((r ^ a.base0) & 1) + 2 * t; i < a.stage_len; i += 2 * T) {
             const float2 c = F[up_pad(((a.base0 + i) & (2 * N - 1)) >> 1)];
             stage[i] = make_float2(c.x * f.x - c.y * f.y, c.x * f.y + c.y * f.x);
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(FirShape<N>::NT, FirShape<N>::CTAS) fir_down_k
         }
         up_first_pass<N>(v, B, t);
         __syncthreads();
-        float2* F = up_passes<N>(B, A, a.tw_n, t);
+        float2* F = up_passes<N, true>(B, A, a.tw_n, t);
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
             const float2 c = F[up_pad(t + T * e)];

@@ -1991,7 +1991,7 @@ __global__ void __launch_bounds__(N / 16, 8192 / N) upsample_pairs_kernel(
         for (int e = 0; e < 16; ++e) v[e] = cmulf(X[e], v[e]);
         up_first_pass<N>(v, A, t);
         __syncthreads();
-        const float2* F = up_passes<N>(A, B, tw_n, t);   // F[j] = p(U j + r)
+        const float2* F = up_passes<N, false>(A, B, tw_n, t);   // F[j] = p(U j + r)
         if (DIRECT) {
             // the span's bins w = q + U i, at j = j0 + i (mod N)
             for (int i = t; q + U * i <= Lg; i += T) {
@@ -2100,7 +2100,7 @@ __global__ void __launch_bounds__(N / 16, 8192 / N) downsample_forward_kernel(
         for (int e = 0; e < 16; ++e) v[e] = A[up_pad(t + T * e)];
         up_first_pass<N>(v, B, t);
         __syncthreads();
-        const float2* F = up_passes<N>(B, A, tw_n, t);
+        const float2* F = up_passes<N, true>(B, A, tw_n, t);
         // Y += e^{2 pi i k r / M} F[k]  (conjugate domain)
         float2 w[16];
         residue_twiddles<N>(tw_m, M, t, r, w);

@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(N / 16, 8192 / N) filter_crop_kernel(const Fil
     for (int e = 0; e < 16; ++e) x[e] = make_float2(z[(e + 8) & 15].x * a.scale, z[(e + 8) & 15].y * a.scale);   // ifftshift
     sar::up_first_pass<N>(x, A, t);
     __syncthreads();
-    const float2* F = sar::up_passes<N>(A, B, tw_n, t);
+    const float2* F = sar::up_passes<N, true>(A, B, tw_n, t);
     const int lo = a.n / 2;
     for (int j = t; j < a.n; j += T)
         a.out[(size_t)blockIdx.x * a.n + j] = sar::cmulf(__ldg(a.window + j), F[sar::up_pad(j < lo ? j : N - (a.n - j))]);

@@ -112,9 +112,10 @@ __device__ __forceinline__ void up_first_pass(const float2 (&x)[16], float2* out
     }
 }
 
-// v[r] *= w^r for r = 1..15 from w, w^2, w^4 and w^8, each rounded by itself.  Built from w alone, w^r has r times w's
-// rounding error, which was most of a transform's: range profiles of N = 512 ... 8192, 2-norm, 2.7e-7 to 3.7e-7 then and
-// 1.4e-7 to 1.7e-7 so, at the same speed.
+// v[r] *= w^r for r = 1..15.  Built from w alone, w^r has r times w's rounding error, which was most of a transform's:
+// range profiles of N = 512 ... 8192, 2-norm, 2.7e-7 to 3.7e-7.  From the table's w and w^4 (upsampling): 1.5e-7 to 2.0e-7;
+// from w, w^2, w^4 and w^8 (FOUR; downsampling, whose few values leave the twiddles most of the error): 1.4e-7 to 1.7e-7,
+// and 8e-8 for 9.5e-8 downsampled at U = 128.  4096 rows of 4096: upsampling 133, 138 and 148 us, downsampling 174, 180 and 182.
 __device__ __forceinline__ void apply_powers(float2 (&v)[16], float2 w, float2 w2, float2 w4, float2 w8) {
     const float2 w3 = cmulf(w2, w), w5 = cmulf(w4, w), w6 = cmulf(w4, w2), w7 = cmulf(w4, w3);
     v[1] = cmulf(v[1], w);
@@ -148,7 +149,7 @@ __device__ __forceinline__ void residue_twiddles(const float2* __restrict__ tw_m
 
 // Radix-16 Stockham pass over N points (sub-transform length ns = N / 256 or N / 16 before it) by the
 // N / 16 threads j of one transform.
-template <int N>
+template <int N, bool FOUR>
 __device__ __forceinline__ void up_pass(const float2* in, float2* out, int ns, const float2* __restrict__ tw_n,
                                         int j) {
     float2 v[16];
@@ -156,7 +157,12 @@ __device__ __forceinline__ void up_pass(const float2* in, float2* out, int ns, c
     for (int r = 0; r < 16; ++r) v[r] = in[up_pad(j + r * (N / 16))];
     const int k = j & (ns - 1);
     const int q = k * (N / (ns * 16));   // w = e^{2 pi i k / (16 ns)}; 8 q < N / 2
-    apply_powers(v, __ldg(tw_n + q), __ldg(tw_n + 2 * q), __ldg(tw_n + 4 * q), __ldg(tw_n + 8 * q));
+    if constexpr (FOUR) {
+        apply_powers(v, __ldg(tw_n + q), __ldg(tw_n + 2 * q), __ldg(tw_n + 4 * q), __ldg(tw_n + 8 * q));
+    } else {
+        const float2 w = __ldg(tw_n + q), w4 = __ldg(tw_n + 4 * q);
+        apply_powers(v, w, cmulf(w, w), w4, cmulf(w4, w4));
+    }
     dft16_inv(v);
     const int base = (j / ns) * ns * 16 + k;
 #pragma unroll
@@ -165,15 +171,15 @@ __device__ __forceinline__ void up_pass(const float2* in, float2* out, int ns, c
 
 // The radix-16 passes after the first (from `in`, ping-ponging with `tmp`): returns the buffer that
 // holds the transform.  The caller synchronises before; each pass ends with a barrier.
-template <int N>
+template <int N, bool FOUR>
 __device__ __forceinline__ float2* up_passes(float2* in, float2* tmp, const float2* __restrict__ tw_n, int j) {
     constexpr int R0 = UpShape<N>::R0;
-    up_pass<N>(in, tmp, R0, tw_n, j);
+    up_pass<N, FOUR>(in, tmp, R0, tw_n, j);
     __syncthreads();
-    up_pass<N>(tmp, in, 16 * R0, tw_n, j);
+    up_pass<N, FOUR>(tmp, in, 16 * R0, tw_n, j);
     __syncthreads();
     if constexpr (UpShape<N>::P == 3) {
-        up_pass<N>(in, tmp, 256 * R0, tw_n, j);
+        up_pass<N, FOUR>(in, tmp, 256 * R0, tw_n, j);
         __syncthreads();
         return tmp;
     }

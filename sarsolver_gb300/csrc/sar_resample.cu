@@ -59,7 +59,7 @@ unsigned blocks_for(size_t n) { return (unsigned)std::min<size_t>((n + 255) / 25
 
 // out[s][j] = in[s][(j + shift_in) % N] * exp(2 pi i phase(s, f)) * scale, where f is the natural
 // (fftshifted) frequency index of the value read and phase = b_s + a_s f in turns.  coef[s] =
-// (b_s, a_hi_s, a_lo_s, unused); a_hi * f is formed with its exact FMA remainder.
+// (b_s, a_hi_s, a_lo_s, the tail of b_s); a_hi * f is formed with its exact FMA remainder.
 __global__ void rephase_kernel(const float2* __restrict__ in, float2* __restrict__ out, const float4* __restrict__ coef,
                                int S, int N, int shift_in, float scale) {
     const size_t total = (size_t)S * N;
@@ -109,9 +109,13 @@ struct FilterArgs {
     float scale;
 };
 
-__device__ __forceinline__ float2 unit(float hi, float lo, float f, float b) {   // exp(2 pi i ((hi + lo) f + b))
+// exp(2 pi i ((hi + lo) f + b + b_lo)).  The large terms are added without error and reduced to half a turn before the small
+// ones join them, so that the phase is rounded once (to 1.5e-8 turns at most): the factors of a sample are two of these,
+// multiplied, and held to the accuracy of one phase formed in plain FP32 sums.
+__device__ __forceinline__ float2 unit(float hi, float lo, float f, float b, float b_lo) {
     const float p = hi * f, pe = fmaf(hi, f, -p);   // exact remainder of the product
-    float t = (p - rintf(p)) + pe + lo * f + b;
+    const float r = p - rintf(p), s = r + b, bb = s - r, e = (r - (s - bb)) + (b - bb);   // s + e = r + b
+    float t = (s - rintf(s)) + (e + (pe + fmaf(lo, f, b_lo)));
     t -= rintf(t);
     float2 v;
     sincospif(2.0f * t, &v.y, &v.x);
@@ -130,7 +134,7 @@ __device__ __forceinline__ void filtered_bins(const FilterArgs& a, int first, in
             __syncthreads();   // the previous batch's readers
             for (int i = threadIdx.x; i < nk * 16; i += blockDim.x) {
                 const float4 c = __ldg(a.coef + first + kb + i / 16);
-                steps[i / 16][i % 16] = unit(c.y, c.z, (float)(T * (i % 16)), 0.f);
+                steps[i / 16][i % 16] = unit(c.y, c.z, (float)(T * (i % 16)), 0.f, 0.f);
             }
             __syncthreads();
         }
@@ -140,7 +144,7 @@ __device__ __forceinline__ void filtered_bins(const FilterArgs& a, int first, in
             float2 w = __ldg(a.kern + kb + k);
             if (a.coef) {
                 const float4 c = __ldg(a.coef + s);
-                w = sar::cmulf(w, unit(c.y, c.z, (float)t, c.x));
+                w = sar::cmulf(w, unit(c.y, c.z, (float)t, c.x, c.w));
             }
             float2 v[16];
 #pragma unroll
@@ -205,7 +209,7 @@ std::vector<float4> phase_coefficients(const double* dr, size_t S, size_t N, dou
         b -= std::nearbyint(b);
         const float a_hi = (float)a;
         const float a_lo = (float)(a - (double)a_hi);
-        co[s] = make_float4((float)b, a_hi, a_lo, 0.f);
+        co[s] = make_float4((float)b, a_hi, a_lo, (float)(b - (double)(float)b));
     }
     return co;
 }

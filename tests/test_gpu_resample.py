@@ -125,3 +125,26 @@ def test_resampling_matches_oracle(S, N, fast, slow, move):
     want = np.stack([(taps[:, None] * down[slow * t:slow * t + L]).sum(axis=0) for t in range(T)])
     assert rel(out.phase_history(), want) < 2e-6
     assert rel(out.aperture.waveform_fft, ora.fast_freq_downsample(wave[None], n, 1.2)[0]) < 1e-6
+
+
+@pytest.mark.parametrize("S,N,fast,slow", [(300, 1999, 1.9, 2), (300, 3000, 1.0, 2), (400, 1024, 1.9, 1), (200, 512, 1.3, 1),
+                                           (300, 700, 2.0, 3), (300, 4096, 1.9, 2)])
+def test_fused_rephasing_is_as_accurate_as_each_sample_rephased(S, N, fast, slow):
+    """The filter's phase factors, products of two, against move_srps, which forms each sample's phase by itself, followed by
+    the same resampling without a move: the error to the FP64 restatement may be no larger."""
+    from oracle import resample as ora
+    rng = np.random.default_rng(N)
+    az = np.deg2rad(np.linspace(-2, 2, S))
+    tx = np.stack([10e3 * np.cos(az), 10e3 * np.sin(az), np.full(S, 5e3)], axis=-1)
+    old, new = 3.0 * rng.standard_normal((S, 3)), np.array([40.0, -25.0, 0.0])
+    ph = ((rng.standard_normal((S, N)) + 1j * rng.standard_normal((S, N))) / np.sqrt(2)).astype(np.complex64)
+    make = lambda srps, p: NumpySimpleSarDataset(NumpySimpleSarAperture(tx, tx.copy(), srps, 10e9, 200e6, num_freqs=N), p)
+    news = np.repeat(new[None], S, axis=0)
+    fused = rs.resample_dataset(make(old, ph), fast, slow, new_srp=new).phase_history()
+    moved = rs.move_srps(torch.from_numpy(ph).cuda(), old, new, tx, tx, 10e9, 200e6)
+    apart = rs.resample_dataset(make(news, moved), fast, slow, new_srp=new).phase_history()
+    n, taps = min(int(1.0 + N / fast), N), ora.downsample_kernel(slow)
+    down = ora.fast_freq_downsample(ora.move_srps(ph.astype(np.complex128), old, new, tx, tx, 10e9, 200e6), n, 1.2)
+    T = (S - len(taps)) // slow - 1
+    want = np.stack([(taps[:, None] * down[slow * t:slow * t + len(taps)]).sum(axis=0) for t in range(T)])
+    assert rel(fused, want) <= rel(apart, want)

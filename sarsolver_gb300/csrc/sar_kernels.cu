@@ -1195,7 +1195,7 @@ __device__ __forceinline__ void ring_flush(float2* wp, int lo, int hi, int first
 // RING (split bins only): ring windows instead of strip windows (FpGridArgs.ring_half): a CTA walks
 // its whole line of tiles and, between tiles, each warp adds and clears the bins its pulses leave
 // behind, so windows no longer bound the length of a strip (1-tile strips at upsample 128 otherwise).
-template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false, bool PAD = true>
+template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false, bool PAD = true, bool BY_TILE = false>
 __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws_kernel(const FpGridArgs a) {
     extern __shared__ __align__(16) unsigned char fsm[];
     const int pbf = a.pbf, ws = a.ws, wslots = window_slots(ws, PAD);
@@ -1348,11 +1348,10 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
     int2* queue = reinterpret_cast<int2*>(fsm + L.queue) + warp * kNearQueue;
     int notes = 0;
     // Moves go to this warp's windows, in the notes' order, where these still hold the bins: always with strip windows,
-    // and with rings where every tile settles its own notes.  That is for images of at most two lines of tiles: a bin
+    // and with rings where every tile settles its own notes (BY_TILE).  That is for images of at most two lines of tiles: a bin
     // then gets two sums, whose order does not matter, and the same bits every time.  (Settled tile by tile, few notes at
     // a time, 1024^2 x 1024 at upsample 128 would take 2.63 ms instead of 2.34.)
-    const int lines_all = TRANSPOSED ? g.tiles_y : g.tiles_x;
-    const bool by_tile = RING && lines_all <= 2, in_window = !RING || by_tile;
+    constexpr bool in_window = !RING || BY_TILE;
     auto settle = [&](int keep) {
         while (notes > keep) {
             const int n = min(32, notes);
@@ -1473,7 +1472,7 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
                 }
             }
         }
-        if (!LINEAR && PRECISE && by_tile && ok) settle(0);
+        if (BY_TILE && ok) settle(0);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[2 + b]);
     }
@@ -1509,20 +1508,23 @@ __global__ void __launch_bounds__(kWsThreads, RING && LINEAR ? 1 : 2) fp_grid_ws
     }
 }
 
-template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false, bool PAD = true>
+template <bool LINEAR, bool PRECISE, bool TRANSPOSED, bool RING = false, bool PAD = true, bool BY_TILE = false>
 static cudaError_t launch_fp_grid_ws_t(const FpGridArgs& a, cudaStream_t st) {
     const size_t smem = fp_grid_ws_smem_bytes(a.ws, a.pbf, LINEAR && !PRECISE, PAD, !LINEAR);
     const int lines = TRANSPOSED ? a.g.tiles_y : a.g.tiles_x;
     const dim3 grid((unsigned)(a.segs_per_column * lines * a.g.nz), (unsigned)((a.S + a.pbf - 1) / a.pbf));
-    cudaError_t e = cudaFuncSetAttribute(fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING, PAD>,
+    cudaError_t e = cudaFuncSetAttribute(fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING, PAD, BY_TILE>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING, PAD><<<grid, kWsThreads, smem, st>>>(a);
+    fp_grid_ws_kernel<LINEAR, PRECISE, TRANSPOSED, RING, PAD, BY_TILE><<<grid, kWsThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
 template <bool TRANSPOSED>
 static cudaError_t launch_fp_grid_ws_o(const FpGridArgs& a, cudaStream_t st) {
+    if (a.ring_half > 0 && !a.linear && (TRANSPOSED ? a.g.tiles_y : a.g.tiles_x) <= 2)
+        return a.pad ? launch_fp_grid_ws_t<false, true, TRANSPOSED, true, true, true>(a, st)
+                     : launch_fp_grid_ws_t<false, true, TRANSPOSED, true, false, true>(a, st);
     if (a.ring_half > 0)   // ring windows: split bins only
         return a.linear ? (a.pad ? launch_fp_grid_ws_t<true, true, TRANSPOSED, true>(a, st)
                                  : launch_fp_grid_ws_t<true, true, TRANSPOSED, true, false>(a, st))

@@ -5,7 +5,7 @@
 
 One step = one backprojection x = A^H y of the 2048^2-pixel x 4096-pulse x 4096-sample workload
 (upsample 8, linear interpolation): the fused range-profile upsampling kernel followed by the
-tiled gather kernel, with y resident in HBM.  The metric is pixel-pulses per second.  The roofline
+gather kernel along iso-range lines, with y resident in HBM.  The metric is pixel-pulses per second.  The roofline
 denominator comes from the arithmetic-pipe rates measured on the same GPU in the same run
 (sar_measure_pipe_rates); the CPU-baseline leg also checks the GPU image against the FP64 oracle
 on a 256^2 patch over all pulses.
@@ -225,15 +225,16 @@ def run_ours(args):
     barrier()
     e2e_ms = reduce_max(e0.elapsed_time(e1) / args.steps, world, dev)
 
-    # ---- roofline of the gather kernel: 28 FP32 flops + 3 special-function ops per pixel-pulse
-    # (canonical work: range 10 + 1 sqrt, bin 3, interpolation 6, phase 1 + sin + cos, MAC 8), on the
-    # FP32 and SFU rates measured on this GPU now
+    # ---- roofline of the gather kernel: 28 FP32 flops + 2 special-function ops per pixel-pulse
+    # (canonical work: range 10, bin 3, interpolation 6, phase 1 + sin + cos, MAC 8; the range is a
+    # polynomial about a block's centre, without a square root per pixel), on the FP32 and SFU rates
+    # measured on this GPU now
     props = torch.cuda.get_device_properties(dev)
     peaks = measured_peaks()
     sm_max = float(peaks.get("sm_max_mhz", 0.0)) or float((clocks or {}).get("sm_max_mhz", 0.0)) or 2070.0
     rates = pipe_rates(dev)
     fp32_units = 2.0 * rates["ffma_per_clk_sm"] / 28.0
-    sfu_units = rates["sfu_sincos_per_clk_sm"] / 3.0
+    sfu_units = rates["sfu_sincos_per_clk_sm"] / 2.0
     units_per_clk = min(fp32_units, sfu_units)
     bound = "fp32" if fp32_units <= sfu_units else "sfu"
     r_roof = props.multi_processor_count * sm_max * 1e6 * units_per_clk
@@ -264,7 +265,7 @@ def run_ours(args):
                                        "full-size launch, profiles/gather_kernel_config2.md",
                      "peak_basis": f"{props.multi_processor_count} SMs x {sm_max:.0f} MHz (sm_max_mhz of "
                                    f"MEASURED_PEAKS.json) x min(2 x {rates['ffma_per_clk_sm']:.1f} FFMA/clk/SM / 28 "
-                                   f"FP32 flops, {rates['sfu_sincos_per_clk_sm']:.1f} sin+cos/clk/SM / 3 SFU ops) "
+                                   f"FP32 flops, {rates['sfu_sincos_per_clk_sm']:.1f} sin+cos/clk/SM / 2 SFU ops) "
                                    "per px*pulse; pipe rates measured in this run (sar_measure_pipe_rates)",
                      "pipe_rates": rates},
         "device_flags": flags,

@@ -454,7 +454,8 @@ bool fir_plan(long N, long M, int Lg, long bg0, FirLayout* L) {
 void fir_tables(const FirLayout& L, std::vector<double>* taps, std::vector<double>* pair_taps, std::vector<double>* inv_c) {
     const int W = kFirTaps, H = L.H;
     const double pi = 3.14159265358979323846;
-    // the usual shape parameter of a Kaiser-Bessel window of width W on a grid oversampled twice
+    // Kaiser-Bessel window of width W on a grid oversampled twice: Jackson et al., IEEE Trans. Med. Imaging 10 (1991), its
+    // shape parameter by Beatty, Nishimura and Pauly, ibid. 24 (2005), beta = pi sqrt((W / a)^2 (a - 1/2)^2 - 0.8), a = 2
     const double beta = pi * std::sqrt(0.5625 * W * W - 0.8), i0b = bessel_i0(beta);
     auto psi = [&](double x) {
         const double u = 2.0 * x / W;

@@ -173,7 +173,7 @@ RowLayout row_layout(int bk, int bn, int kpt, int ntn, int images, int H, int W)
             L.ring = unet::RowRing{R, na, nb, resident};
             L.per_sm = per_sm;
             L.smem = 1024 + (size_t)na * slot + (size_t)nb * block + (2 * (na + nb) + 4) * 8 + 16;
-            // no more CTAs than TMEM has room for share an SM (one beyond would wait in tcgen05.alloc)
+            // no more CTAs of this kernel than TMEM has room for share an SM (see conv_forward's grid)
             L.smem = std::max(L.smem, (size_t)227 * 1024 / (per_sm + 1) + 1024);
             return L;
         }
@@ -256,7 +256,10 @@ int conv_forward(Src s0, Src s1, int images, int H, int W, int taps, const bf16*
     size_t smem = 1024 + (size_t)a.stages * stage + (2 * a.stages + 4) * 8 + 16;
     // Persistent grid: as many CTAs as fit on the SMs, by shared memory and by TMEM (two
     // accumulators each).  When TMEM is the tighter limit the shared-memory request is raised so
-    // that no more CTAs than that share an SM (a CTA beyond it would wait in tcgen05.alloc).
+    // that no more CTAs of this kernel than that share an SM (a CTA beyond it would wait in
+    // tcgen05.alloc).  The limit counts one kernel: in a backward pass a weight gradient's CTA, on its
+    // own stream, may hold columns too, and a CTA then waits for them in tcgen05.alloc before it has
+    // begun.  The holder needs nothing of the waiter's, so such a wait ends with the holder's work.
     const int items = images * a.tiles_x * a.tiles_y * (Nout / BN);
     const size_t sm_smem = 227u * 1024u;
     const int by_smem = std::max(1, (int)(sm_smem / (smem + 9216)));   // with the static and reserved shared memory
@@ -346,7 +349,7 @@ int conv_wgrad(Src s0, Src s1, const bf16* dz, int Cout, int images, int H, int 
             splits = (a.num_tiles + a.tiles_per_split - 1) / a.tiles_per_split;
         }
         size_t smem = 1024 + (size_t)a.stages * stage + (2 * a.stages + 2) * 8 + 16;
-        smem = std::max(smem, (size_t)room / (per_sm + 1) + 1024);   // no CTA more than TMEM and the stages are meant for
+        smem = std::max(smem, (size_t)room / (per_sm + 1) + 1024);   // of this kernel, no CTA more than TMEM and the stages are meant for
         const int mt = 3 * (Ctot / CIB);   // filter rows and channel blocks
         return ci64 ? (co64 ? launch(conv_wgrad_row_kernel<64, 64>, splits, mt, smem) : launch(conv_wgrad_row_kernel<64, 32>, splits, mt, smem))
                     : (co64 ? launch(conv_wgrad_row_kernel<32, 64>, splits, mt, smem) : launch(conv_wgrad_row_kernel<32, 32>, splits, mt, smem));

@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(32 * (NW + NW / 4), NW == 8 ? 2 : 4) gather_ke
                     sum = df_add(sum, df_make(__shfl_xor_sync(0xffffffffu, sum.hi, o), __shfl_xor_sync(0xffffffffu, sum.lo, o)));
                 const int base = __shfl_sync(0xffffffffu, base_bin_of(sum, (float)NS), lane - q);
                 bin_coeffs(ae, vb, base, a.lat, co);
-                // every tap (n0 .. n0 + 2) inside the staged window [-ww / 2, ww / 2]
+                // every tap inside the staged window [-ww / 2, ww / 2]: n0 .. n0 + 2, nearest n0 alone (its bins lie a bin
+                // higher than linear ones, whose offset is -1/2, so the window's two further taps are not all left over)
                 float lo, hi;
                 if (SPLIT) {
                     bin_extent(co, &lo, &hi);
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(32 * (NW + NW / 4), NW == 8 ? 2 : 4) gather_ke
                     lo = co.v[0] - ext;
                     hi = co.v[0] + ext;
                 }
-                if (!(lo - 0.5f - kDip >= -(float)(ww / 2) && hi + 2.5f <= (float)(ww / 2))) {
+                if (!(lo - 0.5f - kDip >= -(float)(ww / 2) && hi + (BINS == GATHER_NEAREST ? 1.5f : 2.5f) <= (float)(ww / 2))) {
                     if (valid) raise_flag(a.flags, FLAG_GATHER_WINDOW);
                     co = Coeffs{};   // invalid result (flagged); every index is then the window's middle
                 }

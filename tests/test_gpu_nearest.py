@@ -92,3 +92,16 @@ def test_coarse_pixels_at_short_range(interp, upsample, pulses, az, shape, degre
     assert rel_l2(plan.forward(x).cpu().numpy(), general.forward(x).cpu().numpy()) < 2.0e-5
     assert rel_l2(plan.adjoint(y).cpu().numpy(), general.adjoint(y).cpu().numpy()) < 2.0e-5
     assert plan.device_flags() == 0
+
+
+@pytest.mark.parametrize("spacing", [0.1, 0.107, 0.114, 0.121, 0.128, 0.135, 0.142, 0.149])
+@pytest.mark.parametrize("shape,az", [((1, 241, 53), 355.0), ((2, 127, 38), 44.0)])
+def test_narrow_windows(shape, az, spacing):
+    """Fine pixels seen from afar, where the host's bound of a tile's bins is tight: windows that end wherever the
+    spacing has it, at up to a whole bin from the bound, hold every nearest bin of pulses with any range offset."""
+    rng = np.random.default_rng(round(1000 * spacing))
+    tx = spotlight(200, 17.0, 5.0e4, 2.5e4, az)
+    rx = spotlight(200, 8.5, 4.0e4, 1.5e4, az + 20.0)
+    ap = NumpySimpleSarAperture(tx, rx, rng.normal(size=(200, 3)), 10.0e9, 200.0e6, num_freqs=256)
+    scene = GridSarScene(list(shape), [2.0 * (shape[0] - 1), spacing * (shape[1] - 1), spacing * (shape[2] - 1)])
+    check(Case(scene, ap, 1.0, {}), 1.0, rng)

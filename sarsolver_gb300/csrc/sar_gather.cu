@@ -60,8 +60,9 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __constant__ float2 kOffsets[8] = {{-8.f, -7.f}, {-6.f, -5.f}, {-4.f, -3.f}, {-2.f, -1.f}, {0.f, 1.f}, {2.f, 3.f}, {4.f, 5.f}, {6.f, 7.f}};
 
 // One pulse onto a thread's 16 pixels (pairs ar[k], ai[k]: offsets 2 k - 8, 2 k - 7).  cs: the sub-tile's set
-// [c0 .. c9 v0 .. v5 h], all phase coefficients but c0, c1, c3, c6 in radians; u: the line's offset; w: the pulse's
-// window at its base bin.  G: pixels per run, 0: two loads per pixel.
+// [c0 .. c9 v0 .. v5 h n], all phase coefficients but c0, c1, c3, c6 in radians; u: the line's offset; w: the pulse's
+// window at its base bin, n (an integer) the sub-tile's distance from it: FP32 then rounds bins of the sub-tile's own
+// excursion, not of its tile's up to 128 pixels.  G: pixels per run, 0: two loads per pixel.
 //
 // c2 is reduced to half turns: c2 = c2' + w2 with |c2'| <= 1/4 and w2 a multiple of 1/2, whose part w2 d is a whole
 // number of turns at even offsets and h = w2 mod 1 at odd ones, the two halves of a pair.  A line's phases stay
@@ -70,7 +71,9 @@ __constant__ float2 kOffsets[8] = {{-8.f, -7.f}, {-6.f, -5.f}, {-4.f, -3.f}, {-2
 template <int G>
 __device__ __forceinline__ void gather_line(const float4* cs, float u, const float2* w, float2 (&ar)[8], float2 (&ai)[8]) {
     const float4 A = cs[0], B = cs[1], C = cs[2], D = cs[3];
-    const float h = reinterpret_cast<const float*>(cs)[16];
+    const float2 E = reinterpret_cast<const float2*>(cs)[8];
+    const float h = E.x;
+    w += __float_as_int(E.y);
     float p0 = fmaf(fmaf(fmaf(B.z, u, A.w), u, A.y), u, A.x);
     p0 -= rintf(p0);
     const float2 P0 = mul2(mk(p0, p0 + h), dup(GA_TWO_PI));
@@ -300,9 +303,12 @@ __global__ void __launch_bounds__(32 * (NW + NW / 4), NW == 8 ? 2 : 4) gather_ke
                 if (SPLIT) {
                     bin_extent(co, &lo, &hi);
                 } else {
+                    const df rel = df_sub(vb, df_make((float)base, 0.f));
+                    co.i0 = round_shift(rel.hi);
+                    co.v[0] = ((rel.hi - co.i0) + rel.lo) + a.lat.bin_offset;
                     const float ext = 8.f * (fabsf(co.v[1]) + fabsf(co.v[2])) + 64.f * (fabsf(co.v[3]) + fabsf(co.v[4]) + fabsf(co.v[5]));
-                    lo = co.v[0] - ext;
-                    hi = co.v[0] + ext;
+                    lo = co.i0 + co.v[0] - ext;
+                    hi = co.i0 + co.v[0] + ext;
                 }
                 if (!(lo - 0.5f - kDip >= -(float)(ww / 2) && hi + (BINS == GATHER_NEAREST ? 1.5f : 2.5f) <= (float)(ww / 2))) {
                     if (valid) raise_flag(a.flags, FLAG_GATHER_WINDOW);
@@ -324,7 +330,7 @@ __global__ void __launch_bounds__(32 * (NW + NW / 4), NW == 8 ? 2 : 4) gather_ke
                         dst[4] = make_float4(w2 - rintf(w2), co.i0, co.ia, co.ib);
                         dst[5] = make_float4(co.w[0], co.w[1], co.w[2], co.w[3]);
                     } else {
-                        reinterpret_cast<float*>(dst)[16] = w2 - rintf(w2);
+                        reinterpret_cast<float2*>(dst)[8] = mk(w2 - rintf(w2), __int_as_float((int)co.i0));
                     }
                     dst[0] = make_float4(co.c[0], co.c[1], (co.c[2] - w2) * K, co.c[3]);
                     dst[1] = make_float4(co.c[4] * K, co.c[5] * K, co.c[6], co.c[7] * K);

@@ -48,3 +48,22 @@ def test_gather_matches_oracle(az, shape, spacing, pulses, degrees, bistatic, ra
     assert rel_l2(blocks.cpu().numpy(), got.cpu().numpy()) < 5.0e-6
     assert torch.equal(plan.adjoint_streamed(yd.cpu().pin_memory(), block=max(1, pulses // 3)), blocks)
     assert plan.device_flags() == 0
+
+
+@pytest.mark.parametrize("az,shape,spacing,pulses,degrees,bistatic,radius,n,upsample", [
+    (62.0, (2, 200, 23), 0.8, 192, 20.0, False, 10.0e3, 1000, 3.0), (34.0, (1, 153, 248), 0.8, 165, 19.0, True, 50.0e3, 256, 1.0)])
+def test_coarse_bins(az, shape, spacing, pulses, degrees, bistatic, radius, n, upsample):
+    """Tiles of 128 pixels that span 140 bins and more, at an upsample where neighbouring bins differ by their own size: a
+    bin's rounding counts in full.  Held in FP32 to the sub-tile's 16 bins at most it is 1e-6 (half a unit of 2^-20) at
+    worst and half of that in the mean, as much as phases of up to two and a half turns (0.6e-6); to the tile's, four
+    times as much.  Bound: 1.3e-6."""
+    rng = np.random.default_rng(pulses)
+    tx = spotlight(pulses, degrees, radius, 0.5 * radius, az)
+    rx = spotlight(pulses, 0.5 * degrees, 0.8 * radius, 0.3 * radius, az + 20.0) if bistatic else tx.copy()
+    ap = NumpySimpleSarAperture(tx, rx, 0.1 * rng.normal(size=(pulses, 3)), 10.0e9, 200.0e6, num_freqs=n)
+    case = Case(GridSarScene(list(shape), [2.0 * (shape[0] - 1), spacing * (shape[1] - 1), spacing * (shape[2] - 1)]), ap, upsample, {})
+    plan = SarPlan(case.scene, ap, upsample_ratio=upsample, interp="linear", path="grid")
+    y = crandn(rng, pulses, n)
+    got = plan.adjoint(torch.from_numpy(y)).cpu().numpy()
+    assert rel_l2(got, oracle.adjoint(case.problem(), y, "linear", threads=8)) < 1.3e-6
+    assert plan.device_flags() == 0

@@ -43,3 +43,26 @@ def test_scatter_matches_oracle(az, shape, spacing, pulses, degrees, bistatic, r
     got = plan.forward(torch.from_numpy(x)).cpu().numpy()
     assert rel_l2(got, oracle.forward(case.problem(), x, "linear", threads=8)) < 1.0e-5
     assert plan.device_flags() == 0
+
+
+@pytest.mark.parametrize("interp", ["linear", "nearest_ref"])
+@pytest.mark.parametrize("spacing,az", [(0.5, 0.0), (0.4, 20.0), (0.3, 45.0)])
+def test_wide_tiles_forward(spacing, az, interp):
+    """Tiles of more than 2048 bins at upsample 128: the forward projection runs per pixel, with phases in double-float
+    that are rounded once (1e-7 rad of at most 2 pi: 1.8e-7 in the mean over random phases with the fold's and the
+    transform's 1.5e-7 and the sums' 2e-7: 3e-7).  Bound: twice that; block expansions in FP32 leave 8e-7 and more."""
+    rng = np.random.default_rng(int(az))
+    tx = spotlight(60, 3.0, 1.0e4, 5.0e3, az)
+    ap = NumpySimpleSarAperture(tx, tx.copy(), 0.1 * rng.normal(size=(60, 3)), 10.0e9, 200.0e6, num_freqs=1024)
+    scene = GridSarScene([1, 110, 150], [0.0, spacing * 109, spacing * 149])
+    case = Case(scene, ap, 128.0, {})
+    plan = SarPlan(scene, ap, upsample_ratio=128.0, interp=interp, path="grid")
+    x = crandn(rng, scene.num_scatterers)
+    got = plan.forward(torch.from_numpy(x)).cpu().numpy()
+    assert rel_l2(got, oracle.forward(case.problem(), x, interp, threads=8)) < 6.0e-7
+    assert plan.device_flags() == 0
+    streamed = SarPlan(scene, ap, upsample_ratio=128.0, interp=interp, path="grid", block_pulses=25)   # ring windows
+    assert streamed.scatter_ring_half > 0 == plan.scatter_ring_half
+    xd = torch.from_numpy(x).to(torch.complex64).cuda()
+    assert rel_l2(streamed.forward(xd).cpu().numpy(), got) < 1.0e-5
+    assert streamed.device_flags() == 0

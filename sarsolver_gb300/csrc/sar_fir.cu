@@ -24,9 +24,9 @@
 // filters alone (fir_rows_kernel / fir_fold_kernel).
 //
 // Measured (GB300, pulses x samples, up / down, against the U-transform kernels or cuFFT of length M
-// before): 4096 x 4096, U = 8: 144 / 172 us (462 / 536); 1024 x 2048, U = 128: down 146 us (1059);
-// 1024 x 1024, U = 128: 61 / 74 us (409 / 569); 128 x 512, U = 8: down 7.2 us (30); 1500 x 2000 (cuFFT),
-// U = 128: up 175 us in three kernels (3800 with transforms of length 256000).
+// before): 4096 x 4096, U = 8: 136 / 182 us (462 / 536); 2048 x 2048, U = 8: 43 / 53 us; 1024 x 2048, U = 128:
+// 78 / 153 us (down 1059); 1024 x 1024, U = 128: 42 / 84 us (409 / 569); 1500 x 2000 (cuFFT), U = 128: 164 / 238 us in
+// three kernels (up 3800 with transforms of length 256000).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -65,7 +65,7 @@ __device__ __forceinline__ T times(T c, float2 f) {
 
 // Transforms of a row side by side: two up to N = 2048, which halves a row's chain of passes; from 4096
 // on one after the other, so that two CTAs share an SM and one's loads overlap the other's passes
-// (4096 rows of 4096, U = 8: upsampling 144 against 189 us, downsampling 172 against 340 us).
+// (4096 rows of 4096, U = 8, when chosen: upsampling 144 against 189 us, downsampling 172 against 340 us).
 constexpr int fir_groups(int N) { return N <= 2048 ? 2 : 1; }
 
 template <int N>

@@ -522,8 +522,8 @@ cudaError_t launch_sum_parts(const float2* partial, float2* x, size_t pixels, in
     return cudaGetLastError();
 }
 
-// Measured (GB300, this kernel alone, against the tile gather before): 2048^2 x 4096 pulses 12.2 ms (14.3);
-// 1024^2 x 2048 1.52 ms (1.88); 512^2 x 1024 0.22 ms (0.28).  19.6 instructions per pixel-pulse, of which the
+// Measured (GB300, this kernel alone, against the tile gather before): 2048^2 x 4096 pulses 12.1 ms (14.3);
+// 1024^2 x 2048 1.50 ms (1.88); 512^2 x 1024 0.22 ms (0.28).  About 19 instructions per pixel-pulse, of which the
 // producers' about 2; issue 64 %, FMA pipe 62 %, special functions 57 % of their cycles.  Tried: sign and
 // magnitude on the integer pipe, 3 % slower; without the phase's cubic term along the line 2 % faster (not kept: a
 // second copy of the body); totals in shared memory instead of the image every 512 pulses, 13.7 ms (registers).
